@@ -74,8 +74,10 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   extern __shared__ unsigned char smem_raw[];
   // full_bar: operand bytes landed (pair: counted on the leader, except a follower's tail block,
   // which is counted on the follower's tail_full of that stage); tail_bar (leader): the follower
-  // has patched its half of a tail block
-  __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], tail_full[MAX_STAGES], acc_full[2], acc_empty[2], tail_bar;
+  // has patched its half of the tail block in that stage. One barrier per stage: with experts of
+  // fewer blocks than the ring has stages several tails are in the ring at once, and a follower
+  // that arrived twice on a single barrier would move it two phases on, past the leader's wait
+  __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], tail_full[MAX_STAGES], acc_full[2], acc_empty[2], tail_bar[MAX_STAGES];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   __shared__ int s_row_off[kMaxLocalExperts + 1];
@@ -92,9 +94,8 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   const int gm = max(1, BAND_M_TILES_ROWS / TM);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); mbar_init(&tail_full[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); mbar_init(&tail_full[s], 1); mbar_init(&tail_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4 * CG); }
-    mbar_init(&tail_bar, 1);
     s_abort = 0;
     fence_barrier_init();
     for (int e = 0; e <= p.El; ++e) {
@@ -172,7 +173,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     // ---------------- MMA warp: all lanes patch tail blocks, one elected lane of the leader issues ----------------
     const bool issuer = elect_one() && leader;
     const uint32_t idesc = instr_desc_bf16(TM, BN, true, true);
-    uint32_t it = 0, tile_n = 0, tails = 0, tail_par = 0;
+    uint32_t it = 0, tile_n = 0, tail_par = 0;               // tail_par: one phase bit per stage (tail_full / tail_bar)
     Tile tl;
     for (int t = unit; decode(t, p.El, m_tiles, n_tiles, gm, s_row_off, tl) && !*abort; t += n_units, ++tile_n) {
       const int k_blocks = (tl.rows + BK - 1) / BK;
@@ -207,11 +208,11 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
           __syncwarp();
           if (CG == 2) {
             if (!leader) {
-              if (lane == 0) mbar_arrive_cluster(&tail_bar, 0);
+              if (lane == 0) mbar_arrive_cluster(&tail_bar[s], 0);
               continue;
             }
-            if (!mbar_wait(&tail_bar, tails & 1, p.status, abort)) { ok = false; break; }
-            ++tails;
+            if (!mbar_wait(&tail_bar[s], (tail_par >> s) & 1, p.status, abort)) { ok = false; break; }
+            tail_par ^= 1u << s;
           }
         }
         fence_after_sync();

@@ -90,6 +90,24 @@ def test_grouped_wgrad(counts, M, N, pair):
         r += c
 
 
+@pytest.mark.parametrize("counts", [[70] * 12, [1, 65, 130, 3, 0, 200, 64, 129] * 2, [320 + 17] * 5])
+def test_grouped_wgrad_many_short_ragged_experts(counts):
+    """Several ragged last blocks in the operand ring at once: more output tiles than CTA pairs and
+    experts of fewer 64-row blocks than the ring has stages."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    torch.manual_seed(7)
+    rows, M, N = sum(counts), 2560, 2048
+    g = torch.randn(rows, M, device="cuda").to(torch.bfloat16)
+    x = torch.randn(rows, N, device="cuda").to(torch.bfloat16)
+    dw = G.grouped_wgrad(g, x, G.offsets_from_counts(counts, "cuda"), pair=True)
+    torch.cuda.synchronize()
+    r = 0
+    for e, c in enumerate(counts):
+        ref = g[r:r + c].float().t() @ x[r:r + c].float()
+        torch.testing.assert_close(dw[e].float(), ref, atol=0.05 * max(c, 1) ** 0.5, rtol=2e-2)
+        r += c
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_grouped_gemm_swiglu_also_stores_pre_activation(pair):
     from gpu_data_transfer_profile_b200.ops import gemm as G
