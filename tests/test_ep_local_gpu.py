@@ -455,3 +455,45 @@ def test_buffer_without_combine_slots_pulls_and_refuses_to_push():
         buf.check_status()
     finally:
         buf.destroy()
+
+
+# few tokens with long rows (a row is cut into parts, one warp each), expert counts that are no multiple of
+# a warp, one rank (no flags) and two
+@pytest.mark.parametrize("R,T,H,E,K,dtype,fp8", [(1, 1, 7168, 160, 8, torch.bfloat16, False), (1, 37, 7168, 33, 4, torch.bfloat16, True),
+                                                 (2, 5, 4096 + 8, 96, 6, torch.float32, False), (2, 300, 3200, 8, 2, torch.bfloat16, True),
+                                                 (1, 1100, 2176, 64, 3, torch.float16, False)])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_dispatch_rows_cut_into_parts_and_receive_tables(R, T, H, E, K, dtype, fp8, grouped):
+    xs, idxs, ws = _mk(R, T, H, E, K, dtype=dtype, seed=11, zipf=0.7)
+    g = _group(R, 768 << 20)
+    El = E // R
+    try:
+        cx, ci, cw = [x.cuda() for x in xs], [i.cuda() for i in idxs], [w.cuda() for w in ws]
+        lays = None if grouped else g.get_dispatch_layout(ci, E)
+        outs = g.dispatch(cx, layouts=lays, topk_idx=ci, topk_weights=cw, use_fp8=fp8, group_by_expert=grouped, num_experts=E)
+        ref = (O.dispatch_expert_mode_ref if grouped else O.dispatch_rank_mode_ref)(xs, idxs, ws, E)
+        for d in range(R):
+            h, cnt = outs[d][4], ref[d][5]
+            n = ref[d][0].shape[0]
+            meta = h.meta.cpu().tolist()
+            assert meta[0] == n == h.n_recv and meta[2:2 + El] == list(cnt) == list(outs[d][3])
+            off = h.meta[2 + El:2 + El + El + 1].cpu().tolist()
+            assert off == [sum(cnt[:q]) for q in range(El + 1)]
+            if fp8:
+                q, sc = outs[d][0]
+                torch.testing.assert_close(sc.cpu(), O.fp8_block_quant_ref(ref[d][0])[1], rtol=1e-6, atol=0)
+                torch.testing.assert_close(O.fp8_block_dequant_ref(q.cpu(), sc.cpu()), ref[d][0].float(), atol=0.3, rtol=0.07)
+            else:
+                assert torch.equal(outs[d][0].cpu(), ref[d][0])
+            if grouped:
+                assert torch.equal(h.recv_prob.cpu(), ref[d][1])
+            else:
+                assert torch.equal(outs[d][1].cpu(), ref[d][1]) and torch.equal(outs[d][2].cpu(), ref[d][2])
+        again = g.dispatch(cx, handles=[o[4] for o in outs], use_fp8=fp8)     # the cached form writes the same rows
+        for d in range(R):
+            a, b = again[d][0], outs[d][0]
+            assert torch.equal(a[0].view(torch.uint8), b[0].view(torch.uint8)) if fp8 else torch.equal(a, b)
+        g.check_status()
+        g.check_canaries()
+    finally:
+        g.destroy()
