@@ -56,6 +56,11 @@ struct CombineArgs {
   const float* weights;      // optional [T][J]
   char* out;                 // [T][H]
   float* out_topk_w;         // optional [T][K]
+  // With send_row (both roles; [T][J] row of (token, item) at its destination) rows whose source is this rank take
+  // no slot: the send role skips them, the reduce role reads them from x / topk_w. Null: every row has a slot.
+  const int* send_row;
+  const long long* topk_idx; // [T][K] (expert mode, with send_row: which rank holds item k)
+  int parts;                 // filled by the launcher
 };
 
 // Number of SMs: the largest useful grid (CTAs have 1024 threads, one per SM).
@@ -81,6 +86,7 @@ struct CombinePullArgs {
   const float* weights;      // optional [T][J]
   char* out;                 // [T][H]
   float* out_topk_w;         // optional [T][K]
+  int parts;                 // filled by the launcher
 };
 void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                          const CombinePullArgs& a, int dtype_code, int* status, int blocks, cudaStream_t st);

@@ -8,8 +8,9 @@
 //   one pass, no slot region, nothing left to do when the last row has arrived.
 // PUSH (rows anywhere): every received row is stored into its slot on the source rank with LSU
 //   peer stores; when its own rows are out a CTA waits (bounded) for the peers' flags and reduces
-//   the slots of this rank's tokens. The fc2 GEMM epilogue of csrc/gemm stores its tiles into the
-//   same slots and is followed by the reduce role alone.
+//   the slots of this rank's tokens. Rows whose source is this rank itself take no slot: they are
+//   read where they lie, so a group of one neither sends nor waits. The fc2 GEMM epilogue of
+//   csrc/gemm stores its tiles into the same slots and is followed by the reduce role alone.
 //
 // What was measured and dropped: cutting the push into token chunks with one flag per chunk, so
 // that the reduction of chunk c overlaps the arrival of chunk c+1. Any release fence on an SM
@@ -18,7 +19,11 @@
 // one fence per CTA and chunk and to 654 us with the reduction running beside it, against 519 us
 // for send-then-reduce. The pull form gets the overlap without any fence.
 //
-// One CTA of 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
+// Bound: memory (or NVLink) bandwidth; every reduction asks for the indices of a warp's next item
+// before it loads the rows of the current one, and few tokens are cut into more parts per row on
+// smaller CTAs. Measured on one B200, before and after: push of 2047 tokens x 8 rows of 14 KiB
+// 133 -> 57 us (the slot round trip is gone), push of 96 rows of 2 KiB 14.7 -> 3.7 us, pull of 4096
+// rows of 14 KiB 27.3 -> 22.8 us. One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
 // peers are launched after the halves they wait for (all announcements / sends first).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -97,6 +102,7 @@ __device__ __forceinline__ void combine_copy_row(const CombineArgs& a, const EpG
                                                  const PeerPtrs& peers, int row, int lane, int* status) {
   const int2 meta = a.recv_meta[row];
   const int slot = meta.x, s = meta.y;
+  if (a.send_row != nullptr && s == g.rank) return;      // the reduce role reads it in place
   if (s < 0 || s >= g.R || slot < 0 || slot >= g.slot_cap) {
     if (lane == 0) set_status(status, kOverflowSlots);
     return;
@@ -143,15 +149,95 @@ __device__ void combine_send_role(const CombineArgs& a, const EpGeom& g, const E
   }
 }
 
+// ---- reduction --------------------------------------------------------------------------------
+// Work item = (token, part of the row): out[t] = sum_j w[t][j] * row_j(t), j in ascending order.
+// Lane j < J looks after contributor j: Index holds what it reads for an item, `fetch(t)` issues
+// those loads and `resolve(t, index, &side)` turns them into the address of the row (null: none)
+// and of its side values. fetch runs one item ahead.
+struct Index { int row, slot; long long expert; float w; };
+
+__device__ __forceinline__ int reduce_first(int parts, int warp) { return (warp / parts) * gridDim.x + blockIdx.x; }
+
+template <typename T, typename Fetch, typename Resolve>
+__device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* out, float* out_topk_w,
+                                             Fetch fetch, Resolve resolve) {
+  __shared__ const char* s_row[kCombWarps][kMaxItemsPerToken];
+  __shared__ const float* s_side[kCombWarps][kMaxItemsPerToken];
+  __shared__ float s_w[kCombWarps][kMaxItemsPerToken];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int J = g.J;
+  const int row_bytes = g.H * (int)sizeof(T);
+  const int nvec = row_bytes >> 4;
+  const int part = warp % parts;
+  const int part_vec = (nvec + parts - 1) / parts;
+  const int v_end = min(nvec, (part + 1) * part_vec);
+  // neighbouring items land on different CTAs, so every SM reads from a mix of peers
+  const int per_round = gridDim.x * (nwarps / parts);
+  int t = reduce_first(parts, warp);
+  Index ix = fetch(t);
+  for (; t < g.T; t += per_round) {
+    const float* side = nullptr;
+    const char* mine = nullptr;
+    if (lane < J) {
+      mine = resolve(t, ix, &side);
+      s_row[warp][lane] = mine;
+      s_side[warp][lane] = side;
+      s_w[warp][lane] = ix.w;
+    }
+    const unsigned vmask = __ballot_sync(0xffffffffu, mine != nullptr);
+    __syncwarp();
+    ix = fetch(t + per_round);
+    // kRUnroll vectors per lane and contributor are loaded together (independent loads in flight),
+    // then accumulated in fp32; contributors are visited one after the other.
+    for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kRUnroll) {
+      float acc[kRUnroll][Vec16<T>::N];
+#pragma unroll
+      for (int u = 0; u < kRUnroll; ++u)
+#pragma unroll
+        for (int q = 0; q < Vec16<T>::N; ++q) acc[u][q] = 0.f;
+      for (unsigned mm = vmask; mm; mm &= mm - 1) {
+        const int j = __ffs(mm) - 1;
+        const char* rowp = s_row[warp][j];
+        const float wj = s_w[warp][j];
+        uint4 val[kRUnroll];
+#pragma unroll
+        for (int u = 0; u < kRUnroll; ++u) {
+          const int v = v0 + u * 32;
+          if (v < v_end) val[u] = ld_global_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU may have written it
+        }
+#pragma unroll
+        for (int u = 0; u < kRUnroll; ++u)
+          if (v0 + u * 32 < v_end) Vec16<T>::acc(acc[u], val[u], wj);
+      }
+#pragma unroll
+      for (int u = 0; u < kRUnroll; ++u) {
+        const int v = v0 + u * 32;
+        if (v < v_end) st_global_v4(out + (size_t)t * row_bytes + ((size_t)v << 4), Vec16<T>::pack(acc[u]));
+      }
+    }
+    if (out_topk_w != nullptr && part == 0) {
+      if (g.mode == 0) {
+        // rank mode: [T,K] = sum over destination ranks of the K side values of each row
+        if (lane < g.K) {
+          float s = 0.f;
+          for (unsigned mm = vmask; mm; mm &= mm - 1) s += s_side[warp][__ffs(mm) - 1][lane];
+          out_topk_w[(size_t)t * g.K + lane] = s;
+        }
+      } else if (lane < J) {
+        // expert mode: [T,K], entry k is the single side value returned for item (t,k)
+        out_topk_w[(size_t)t * J + lane] = mine != nullptr ? *side : 0.f;
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // ---- push form: reduce role ----------------------------------------------------------------
-// Work item = (token, part of the row): out[t] = sum_j w[t][j] * comb_x[slot[t][j]]  (w = 1 when absent).
 template <typename T>
 __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const EpRegions& rg,
                                     char* self_base, int* status) {
-  __shared__ int s_slot[kCombWarps][kMaxItemsPerToken];
-  __shared__ float s_w[kCombWarps][kMaxItemsPerToken];
   __shared__ int s_ok;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   if (a.wait) {
     if (threadIdx.x == 0) s_ok = 1;
     __syncthreads();
@@ -164,78 +250,40 @@ __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const
   }
   const int J = g.J;
   const int row_bytes = g.H * (int)sizeof(T);
-  const int nvec = row_bytes >> 4;
-  // a row is cut into up to 4 parts of at least 128 vectors, one warp each (shorter dependent chains)
-  int parts = nvec / 128;
-  parts = parts < 1 ? 1 : (parts > 4 ? 4 : parts);
-  if (parts == 3) parts = 2;
-  if (nwarps % parts) parts = 1;
-  const int part_vec = (nvec + parts - 1) / parts;
-  const int tok_per_round = nwarps / parts;
-  const int part = warp % parts, tok_in_cta = warp / parts;
+  const int wk = g.mode == 0 ? g.K : 1;              // side values per row
   const char* comb = self_base + rg.comb_x;
   const float* comb_w = reinterpret_cast<const float*>(self_base + rg.comb_w);
-  const int per_round = gridDim.x * tok_per_round;
-  for (int t = blockIdx.x * tok_per_round + tok_in_cta; t < g.T; t += per_round) {
-    int slot = -1;
-    if (lane < J) {
-      slot = a.send_slot[(size_t)t * J + lane];
-      if (slot >= g.slot_cap) slot = -1;
-      s_slot[warp][lane] = slot;
-      s_w[warp][lane] = a.weights ? a.weights[(size_t)t * J + lane] : 1.f;
-    }
-    const unsigned vmask = __ballot_sync(0xffffffffu, slot >= 0);
-    __syncwarp();
-    const int v_end = min(nvec, (part + 1) * part_vec);
-    // kRUnroll vectors per lane and contributor are loaded together (independent loads in flight),
-    // then accumulated in fp32; contributors are visited one after the other.
-    for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kRUnroll) {
-      float acc[kRUnroll][Vec16<T>::N];
-#pragma unroll
-      for (int u = 0; u < kRUnroll; ++u)
-#pragma unroll
-        for (int q = 0; q < Vec16<T>::N; ++q) acc[u][q] = 0.f;
-      for (unsigned mm = vmask; mm; mm &= mm - 1) {
-        const int j = __ffs(mm) - 1;
-        const char* rowp = comb + (size_t)s_slot[warp][j] * row_bytes;
-        const float wj = s_w[warp][j];
-        uint4 val[kRUnroll];
-#pragma unroll
-        for (int u = 0; u < kRUnroll; ++u) {
-          const int v = v0 + u * 32;
-          if (v < v_end) val[u] = ld_global_v4(rowp + ((size_t)v << 4));
-        }
-#pragma unroll
-        for (int u = 0; u < kRUnroll; ++u)
-          if (v0 + u * 32 < v_end) Vec16<T>::acc(acc[u], val[u], wj);
+  const bool in_place = a.send_row != nullptr;
+  const int n_rows = in_place ? min(*a.n_recv_ptr, g.cap) : 0;
+  auto fetch = [&](int t) {
+    Index ix{-1, -1, -1, 1.f};
+    if (t < g.T && lane < J) {
+      const size_t at = (size_t)t * J + lane;
+      ix.slot = a.send_slot[at];
+      if (in_place) {
+        ix.row = a.send_row[at];
+        ix.expert = g.mode == 0 ? (long long)lane * g.El : a.topk_idx[at];
       }
-#pragma unroll
-      for (int u = 0; u < kRUnroll; ++u) {
-        const int v = v0 + u * 32;
-        if (v < v_end) st_global_v4(a.out + (size_t)t * row_bytes + ((size_t)v << 4), Vec16<T>::pack(acc[u]));
-      }
+      if (a.weights) ix.w = a.weights[at];
     }
-    if (a.out_topk_w != nullptr && part == 0) {
-      if (g.mode == 0) {
-        // rank mode: [T,K] = sum over destination ranks of the K side values of each row
-        if (lane < g.K) {
-          float s = 0.f;
-          for (unsigned mm = vmask; mm; mm &= mm - 1)
-            s += comb_w[(size_t)s_slot[warp][__ffs(mm) - 1] * g.K + lane];
-          a.out_topk_w[(size_t)t * g.K + lane] = s;
-        }
-      } else if (lane < J) {
-        // expert mode: [T,K], entry k is the single side value returned for item (t,k)
-        a.out_topk_w[(size_t)t * J + lane] = slot >= 0 ? comb_w[slot] : 0.f;
-      }
+    return ix;
+  };
+  auto resolve = [&](int t, const Index& ix, const float** side) -> const char* {
+    if (ix.slot < 0 || ix.slot >= g.slot_cap) return nullptr;
+    if (in_place && ix.expert >= 0 && ix.expert < g.E && (int)ix.expert / g.El == g.rank) {
+      if (ix.row < 0 || ix.row >= n_rows) return nullptr;
+      *side = a.topk_w + (size_t)ix.row * wk;
+      return a.x + (size_t)ix.row * row_bytes;
     }
-    __syncwarp();
-  }
+    *side = comb_w + (size_t)ix.slot * wk;
+    return comb + (size_t)ix.slot * row_bytes;
+  };
+  reduce_items<T>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
-combine_kernel(EpGeom g, EpRegions rg, PeerPtrs peers, CombineArgs a, int* status) {
+combine_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombineArgs a, int* status) {
   if (a.role != kCombineReduceOnly) combine_send_role(a, g, rg, peers, status);
   if (a.role != kCombineSendOnly) combine_reduce_role<T>(a, g, rg, peers.base[g.rank], status);
 }
@@ -247,27 +295,45 @@ int combine_max_ctas() {
   return sms;
 }
 
-void launch_combine(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers, const CombineArgs& a,
+// How a reduction of T tokens is cut: parts per row (a power of two, at least 2 KiB each; more, down to 512 bytes,
+// while the grid has warps to spare), warps per CTA and CTAs no more than the items need.
+struct ReduceShape { int parts, warps, blocks; };
+static ReduceShape reduce_shape(long long T, int row_bytes, int blocks, bool may_shrink) {
+  const int nvec = row_bytes >> 4;
+  ReduceShape s{1, kCombWarps, blocks};
+  while (s.parts < 4 && nvec / (s.parts * 2) >= 128) s.parts *= 2;
+  while (s.parts < 16 && nvec / (s.parts * 2) >= 32 && T * s.parts * 2 <= (long long)blocks * kCombWarps) s.parts *= 2;
+  if (!may_shrink) return s;
+  const long long items = (T > 0 ? T : 1) * s.parts;
+  while (s.warps > 4 && s.warps / 2 >= s.parts && (long long)blocks * (s.warps / 2) >= items) s.warps /= 2;
+  const long long need = (items + s.warps - 1) / s.warps;
+  if (need < s.blocks) s.blocks = (int)need;
+  return s;
+}
+
+void launch_combine(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers, const CombineArgs& args,
                     int dtype_code, int* status, int blocks, cudaStream_t st) {
   if (blocks < 1) blocks = 1;
+  CombineArgs a = args;
+  // A group of one with its rows at hand has nothing to send and nobody to wait for.
+  if (g.R == 1 && a.send_row != nullptr && a.role == kCombineBoth) { a.role = kCombineReduceOnly; a.wait = 0; }
+  const ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, a.role == kCombineReduceOnly);
+  a.parts = rs.parts;
   if (dtype_code == 0)
-    combine_kernel<__nv_bfloat16><<<blocks, kCombWarps * 32, 0, st>>>(g, rg, peers, a, status);
+    combine_kernel<__nv_bfloat16><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
   else if (dtype_code == 1)
-    combine_kernel<__half><<<blocks, kCombWarps * 32, 0, st>>>(g, rg, peers, a, status);
+    combine_kernel<__half><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
   else
-    combine_kernel<float><<<blocks, kCombWarps * 32, 0, st>>>(g, rg, peers, a, status);
+    combine_kernel<float><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
 }
 
 // ---- pull form -----------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
-combine_pull_kernel(EpGeom g, EpRegions rg, PeerPtrs peers, CombinePullArgs a, int* status) {
-  __shared__ int s_row[kCombWarps][kMaxItemsPerToken];
-  __shared__ int s_src[kCombWarps][kMaxItemsPerToken];
-  __shared__ float s_w[kCombWarps][kMaxItemsPerToken];
+combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombinePullArgs a, int* status) {
   __shared__ long long s_info[kMaxRanks][4];
   __shared__ int s_ok;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   char* self_base = peers.base[g.rank];
   if (a.publish && blockIdx.x == 0 && (int)threadIdx.x < g.R) {
     // rows were written by earlier kernels of this stream: complete and visible at this point
@@ -282,108 +348,56 @@ combine_pull_kernel(EpGeom g, EpRegions rg, PeerPtrs peers, CombinePullArgs a, i
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
   if ((int)threadIdx.x < g.R) {
-    const int* flags = reinterpret_cast<const int*>(self_base + rg.flags) + kChCombine * kMaxRanks;
-    if (a.wait && !wait_flag_ge(flags + threadIdx.x, g.epoch, g.timeout_ns, status, kTimeoutCombine)) s_ok = 0;
-    const long long* info = reinterpret_cast<const long long*>(self_base + rg.pull_info) + threadIdx.x * 4;
-    for (int q = 0; q < 3; ++q) s_info[threadIdx.x][q] = __ldcg(&info[q]);
+    if (g.R == 1 && a.publish) {             // a group of one: what it announces is at hand
+      s_info[0][0] = a.x_off; s_info[0][1] = a.w_off; s_info[0][2] = a.n_rows;
+    } else {
+      const int* flags = reinterpret_cast<const int*>(self_base + rg.flags) + kChCombine * kMaxRanks;
+      if (a.wait && !wait_flag_ge(flags + threadIdx.x, g.epoch, g.timeout_ns, status, kTimeoutCombine)) s_ok = 0;
+      const long long* info = reinterpret_cast<const long long*>(self_base + rg.pull_info) + threadIdx.x * 4;
+      for (int q = 0; q < 3; ++q) s_info[threadIdx.x][q] = __ldcg(&info[q]);
+    }
   }
   __syncthreads();
   if (!s_ok) return;
   const int J = g.J;
   const int row_bytes = g.H * (int)sizeof(T);
-  const int nvec = row_bytes >> 4;
-  int parts = nvec / 128;
-  parts = parts < 1 ? 1 : (parts > 4 ? 4 : parts);
-  if (parts == 3) parts = 2;
-  if (nwarps % parts) parts = 1;
-  const int part_vec = (nvec + parts - 1) / parts;
-  const int tok_per_round = nwarps / parts;
-  const int part = warp % parts, tok_in_cta = warp / parts;
-  // consecutive (token, part) items land on different CTAs: every SM reads from a mix of peers
-  const int per_round = gridDim.x * tok_per_round;
-  for (int t = tok_in_cta * gridDim.x + blockIdx.x; t < g.T; t += per_round) {
-    int row = -1;
-    if (lane < J) {
-      row = a.send_row[(size_t)t * J + lane];
-      int d = lane;
-      if (g.mode == 1) {
-        const long long e = a.topk_idx[(size_t)t * g.K + lane];
-        d = (e >= 0 && e < g.E) ? (int)(e / g.El) : -1;
-      }
-      if (row >= 0 && (d < 0 || (long long)row >= s_info[d][2] || s_info[d][0] < 0)) {
-        set_status(status, kOverflowSlots);       // the peer did not announce that many rows
-        row = -1;
-      }
-      s_row[warp][lane] = row;
-      s_src[warp][lane] = d;
-      s_w[warp][lane] = a.weights ? a.weights[(size_t)t * J + lane] : 1.f;
+  const int wk = g.mode == 0 ? g.K : 1;
+  auto fetch = [&](int t) {
+    Index ix{-1, -1, -1, 1.f};
+    if (t < g.T && lane < J) {
+      const size_t at = (size_t)t * J + lane;
+      ix.row = a.send_row[at];
+      ix.expert = g.mode == 0 ? (long long)lane * g.El : a.topk_idx[at];
+      if (a.weights) ix.w = a.weights[at];
     }
-    const unsigned vmask = __ballot_sync(0xffffffffu, row >= 0);
-    __syncwarp();
-    const int v_end = min(nvec, (part + 1) * part_vec);
-    for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kRUnroll) {
-      float acc[kRUnroll][Vec16<T>::N];
-#pragma unroll
-      for (int u = 0; u < kRUnroll; ++u)
-#pragma unroll
-        for (int q = 0; q < Vec16<T>::N; ++q) acc[u][q] = 0.f;
-      for (unsigned mm = vmask; mm; mm &= mm - 1) {
-        const int j = __ffs(mm) - 1;
-        const int d = s_src[warp][j];
-        const char* rowp = peers.base[d] + s_info[d][0] + (size_t)s_row[warp][j] * row_bytes;
-        const float wj = s_w[warp][j];
-        uint4 val[kRUnroll];
-#pragma unroll
-        for (int u = 0; u < kRUnroll; ++u) {
-          const int v = v0 + u * 32;
-          if (v < v_end) val[u] = ld_global_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU wrote these rows
-        }
-#pragma unroll
-        for (int u = 0; u < kRUnroll; ++u)
-          if (v0 + u * 32 < v_end) Vec16<T>::acc(acc[u], val[u], wj);
-      }
-#pragma unroll
-      for (int u = 0; u < kRUnroll; ++u) {
-        const int v = v0 + u * 32;
-        if (v < v_end) st_global_v4(a.out + (size_t)t * row_bytes + ((size_t)v << 4), Vec16<T>::pack(acc[u]));
-      }
+    return ix;
+  };
+  auto resolve = [&](int t, const Index& ix, const float** side) -> const char* {
+    if (ix.row < 0) return nullptr;
+    const int d = (ix.expert >= 0 && ix.expert < g.E) ? (int)ix.expert / g.El : -1;
+    if (d < 0 || (long long)ix.row >= s_info[d][2] || s_info[d][0] < 0) {
+      set_status(status, kOverflowSlots);       // the peer did not announce that many rows
+      return nullptr;
     }
-    if (a.out_topk_w != nullptr && part == 0) {
-      // side values: K floats per row in rank mode (summed over the destinations), one in expert mode
-      if (g.mode == 0) {
-        if (lane < g.K) {
-          float s = 0.f;
-          for (unsigned mm = vmask; mm; mm &= mm - 1) {
-            const int j = __ffs(mm) - 1, d = s_src[warp][j];
-            const float* wp = reinterpret_cast<const float*>(peers.base[d] + s_info[d][1]);
-            s += wp[(size_t)s_row[warp][j] * g.K + lane];
-          }
-          a.out_topk_w[(size_t)t * g.K + lane] = s;
-        }
-      } else if (lane < J) {
-        float v = 0.f;
-        if (row >= 0) {
-          const int d = s_src[warp][lane];
-          v = reinterpret_cast<const float*>(peers.base[d] + s_info[d][1])[row];
-        }
-        a.out_topk_w[(size_t)t * J + lane] = v;
-      }
-    }
-    __syncwarp();
-  }
+    *side = reinterpret_cast<const float*>(peers.base[d] + s_info[d][1]) + (size_t)ix.row * wk;
+    return peers.base[d] + s_info[d][0] + (size_t)ix.row * row_bytes;
+  };
+  reduce_items<T>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
 void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
-                         const CombinePullArgs& a, int dtype_code, int* status, int blocks, cudaStream_t st) {
+                         const CombinePullArgs& args, int dtype_code, int* status, int blocks, cudaStream_t st) {
   if (blocks < 1) blocks = 1;
-  const int threads = a.pull ? kCombWarps * 32 : 32;
-  if (!a.pull) blocks = 1;
+  CombinePullArgs a = args;
+  ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, true);
+  if (!a.pull) rs = ReduceShape{1, 1, 1};
+  a.parts = rs.parts;
   if (dtype_code == 0)
-    combine_pull_kernel<__nv_bfloat16><<<blocks, threads, 0, st>>>(g, rg, peers, a, status);
+    combine_pull_kernel<__nv_bfloat16><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
   else if (dtype_code == 1)
-    combine_pull_kernel<__half><<<blocks, threads, 0, st>>>(g, rg, peers, a, status);
+    combine_pull_kernel<__half><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
   else
-    combine_pull_kernel<float><<<blocks, threads, 0, st>>>(g, rg, peers, a, status);
+    combine_pull_kernel<float><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
 }
 
 // Signal only (used when a fused GEMM epilogue has already stored the rows).

@@ -669,27 +669,33 @@ class Buffer:
     def _combine_p1(self, x, handle: DispatchHandle, topk_weights):
         """Push form, send half as its own launch (several virtual ranks on one GPU)."""
         st = self._combine_prepare(x, handle, topk_weights)
+        st["in_place"] = True
         self.C.combine(st["geom"], st["regions"], self.peers, 1, max(1, Buffer.num_sms), False,
                        handle.n_recv_dev, handle.recv_meta, x, st["topk_w"], self._ctr[2],
-                       None, None, None, None, self.status_ptr)
+                       None, None, None, None, self.status_ptr, handle.send_row, handle.topk_idx)
         return st
 
     def _combine_p2(self, st, handle: DispatchHandle, weights=None):
         """Push form, reduce half as its own launch (waits for every rank's combine flag first)."""
         out, out_w = self._combine_outputs(st, handle)
+        # rows of this rank's own tokens are still where `_combine_p1` found them; the fused fc2 has put
+        # every row into its slot
+        here = st.get("in_place", False)
         self.C.combine(st["geom"], st["regions"], self.peers, 2, max(1, Buffer.num_sms), True,
-                       None, None, None, None, self._ctr[2],
-                       handle.send_slot, weights, out, out_w, self.status_ptr)
+                       handle.n_recv_dev if here else None, handle.recv_meta if here else None,
+                       st["x"] if here else None, st["topk_w"] if here else None, self._ctr[2],
+                       handle.send_slot, weights, out, out_w, self.status_ptr,
+                       handle.send_row if here else None, handle.topk_idx if here else None)
         return out, out_w
 
     def _combine_fused(self, x, handle: DispatchHandle, topk_weights, weights=None):
         """Push form in ONE launch: every CTA sends its share of the rows, then waits for the peers'
-        flags and reduces its share of the tokens."""
+        flags and reduces its share of the tokens (this rank's own rows are reduced where they lie)."""
         st = self._combine_prepare(x, handle, topk_weights)
         out, out_w = self._combine_outputs(st, handle)
         self.C.combine(st["geom"], st["regions"], self.peers, 0, max(1, Buffer.num_sms), True,
                        handle.n_recv_dev, handle.recv_meta, x, st["topk_w"], self._ctr[2],
-                       handle.send_slot, weights, out, out_w, self.status_ptr)
+                       handle.send_slot, weights, out, out_w, self.status_ptr, handle.send_row, handle.topk_idx)
         return out, out_w
 
     def _region_offset(self, t: Optional[torch.Tensor]) -> int:

@@ -497,3 +497,43 @@ def test_dispatch_rows_cut_into_parts_and_receive_tables(R, T, H, E, K, dtype, f
         g.check_canaries()
     finally:
         g.destroy()
+
+
+# own rows are reduced where they lie, peers' rows from their slots; few tokens: rows cut into up to 16 parts
+@pytest.mark.parametrize("R,T,H,E,K,dtype", [(1, 3, 7168, 16, 8, torch.bfloat16), (2, 9, 7168, 16, 4, torch.bfloat16),
+                                             (4, 2, 4104, 8, 2, torch.float32), (2, 700, 520, 8, 8, torch.float16)])
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_push_combine_reads_own_rows_in_place(R, T, H, E, K, dtype, grouped, weighted):
+    xs, idxs, ws = _mk(R, T, H, E, K, dtype=dtype, seed=21)
+    idxs[0][0, 0] = -1                                    # an empty choice contributes nothing
+    g = _group(R, 512 << 20)
+    try:
+        cx, ci, cw = [x.cuda() for x in xs], [i.cuda() for i in idxs], [w.cuda() for w in ws]
+        for rep in range(3):
+            lays = None if grouped else g.get_dispatch_layout(ci, E)
+            outs = g.dispatch(cx, layouts=lays, topk_idx=ci, topk_weights=cw, group_by_expert=grouped, num_experts=E)
+            ys = [(o[0].float() * (rep + 1 + d)).to(dtype) for d, o in enumerate(outs)]       # tensors of their own: push
+            side = [o[4].recv_prob if grouped else o[2] for o in outs]
+            J = K if grouped else R
+            iw = [torch.rand(T, J, device="cuda", generator=torch.Generator("cuda").manual_seed(r)) for r in range(R)] if weighted else None
+            comb = g.combine(ys, [o[4] for o in outs], topk_weights=side, item_weights=iw)
+            for r in range(R):
+                valid = idxs[r] >= 0
+                dest = torch.where(valid, idxs[r] // (E // R), torch.zeros_like(idxs[r]))
+                if grouped:
+                    factor = torch.where(valid, rep + 1.0 + dest, torch.zeros(()))
+                else:
+                    hit = torch.zeros(T, R, dtype=torch.bool)
+                    hit[torch.arange(T)[:, None].expand_as(dest)[valid], dest[valid]] = True
+                    factor = hit * (rep + 1.0 + torch.arange(R))
+                if weighted:
+                    factor = factor * iw[r].cpu()
+                got, got_w = comb[r]
+                tol = dict(atol=1e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=0.08, rtol=2e-2)
+                torch.testing.assert_close(got.cpu().float(), xs[r].float() * factor.sum(1, keepdim=True), **tol)
+                torch.testing.assert_close(got_w.cpu(), torch.where(valid, ws[r], torch.zeros(())), atol=1e-6, rtol=1e-6)
+        g.check_status()
+        g.check_canaries()
+    finally:
+        g.destroy()
