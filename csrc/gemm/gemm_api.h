@@ -32,8 +32,8 @@ struct GemmParams {
 };
 
 // a: bf16 [a_rows, K] on this GPU; w: bf16 [El * w_rows, K] on this GPU. Returns 0 on success.
-// pair: run CTA pairs (clusters of two SMs, `cta_group::2`) on 256 x 256 tiles instead of single
-// CTAs on 128 x 256 tiles; `ctas` then counts CTAs as well (pairs = ctas / 2, capped by residency).
+// pair: run CTA pairs (clusters of two SMs, `cta_group::2`) on 256 weight rows x up to 256 tokens instead of
+// single CTAs on 128 weight rows; `ctas` then counts CTAs as well (pairs = ctas / 2, capped by residency).
 int launch_grouped_gemm(const void* a, long long a_rows, const void* w, int epi, GemmParams p,
                         const PeerPtrs& peers, int ctas, bool pair, cudaStream_t st);
 

@@ -186,6 +186,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr) : "memory");
 }
+// 32 lanes x 16 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Compiler-level dependency only (emits nothing): values loaded by an EARLIER tmem_ld32 whose
 // tmem_ld_wait() was separated from the load by other code must not be consumed by instructions
@@ -197,6 +206,24 @@ __device__ __forceinline__ void tmem_ld_pin(uint32_t* r) {
         "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
         "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
       :: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld_pin16(uint32_t* r) {
+  asm volatile(""
+      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+        "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+      :: "memory");
+}
+
+// ---- named barriers of a 128-thread group -----------------------------------------------------
+__device__ __forceinline__ void group_sync(int id) { __syncwarp(); asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(id) : "memory"); }
+// true for every thread of the group if `ok` is true in all of them
+__device__ __forceinline__ bool group_all(int id, bool ok) {
+  uint32_t all;
+  __syncwarp();
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbarrier.cta.red.and.aligned.pred p, %2, 128, q;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(all) : "r"((uint32_t)ok), "r"(id) : "memory");
+  return all != 0;
 }
 
 }  // namespace tc

@@ -49,6 +49,39 @@ def test_grouped_gemm_weights_stored_k_by_n(counts, N, K, pair):
     torch.testing.assert_close(out.float(), ref, atol=0.05 * (K ** 0.5) * 0.1, rtol=2e-2)
 
 
+# edges of the token tiles (one row, a unit of 16 / 32 rows more or less, 256 and beyond, more than 32 experts, most of
+# them empty) and of the weight tiles (fewer output columns than a CTA holds, a ragged last tile), short reductions.
+# Tolerance: one bf16 rounding of the result (2^-8 of it covers a value at the boundary) plus f32 accumulation noise.
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("counts", [[1], [15, 16, 17, 31, 32, 33], [255, 256, 257], [511, 513, 800], [5] * 40,
+                                    [0] * 10 + [300] + [0] * 30 + [2]])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 72), (264, 200), (640, 328)])
+def test_grouped_gemm_token_and_weight_tile_edges(counts, N, K, pair):
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    torch.manual_seed(8)
+    rows, E = sum(counts), len(counts)
+    a = torch.randn(rows + 3, K, device="cuda").to(torch.bfloat16)
+    a[rows:] = float("nan")                                # rows after the last expert must not leak
+    w = (torch.randn(E, N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    off = G.offsets_from_counts(counts, "cuda")
+    tol = dict(rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)
+    for kn in (False, True):
+        out = torch.full((rows + 3, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        G.grouped_gemm(a, w.transpose(1, 2).contiguous() if kn else w, off, out=out, pair=pair, w_kn=kn)
+        torch.cuda.synchronize()
+        torch.testing.assert_close(out[:rows].float(), _ref(a[:rows], w, counts), **tol)
+        assert bool((out[rows:] == 7.0).all())
+    F = max(128, N // 128 * 128)
+    w1 = (torch.randn(E, 2 * F, K, device="cuda") * 0.1).to(torch.bfloat16)
+    pre = torch.empty(rows + 3, 2 * F, dtype=torch.bfloat16, device="cuda")
+    prob = torch.rand(rows + 3, device="cuda")
+    act = G.grouped_gemm_swiglu(a, w1, off, prob, pair=pair, pre_out=pre)
+    torch.cuda.synchronize()
+    h = _ref(a[:rows], w1, counts)
+    torch.testing.assert_close(pre[:rows].float(), h, **tol)
+    torch.testing.assert_close(act[:rows].float(), torch.nn.functional.silu(h[:, :F]) * h[:, F:] * prob[:rows, None], rtol=2.0 ** -8, atol=1e-3)
+
+
 @pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("counts,F,K", [([128], 128, 128), ([200, 56], 256, 256), ([1, 300], 384, 192),
                                         ([700, 3, 257], 512, 512)])
