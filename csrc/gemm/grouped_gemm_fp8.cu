@@ -12,13 +12,24 @@
 // scales differ per 128-wide reduction block, so every block's partial product is a SEPARATE
 // accumulator in TMEM (two of 128 lanes x 256 columns, used alternately) which the epilogue warps
 // read back, scale and add to an f32 running sum in registers ("promotion") while the tensor core
-// already works on the next block. Structure per CTA (persistent, one per SM, 320 threads):
+// already works on the next block.
+// Bound: the promotion. Per block the 8 warps need about 390 cycles (135 for the TMEM reads, 256 for the
+// FMAs) between two hand-overs, the 4 MMAs 512 and the operand traffic through shared memory about
+// 750; with two partials the three do not overlap completely. Hence: registers moved to the promotion
+// warps (168 for all left the loop spilling or reading 32 columns at a time), packed f32x2 FMAs (half
+// the issue slots, same rounding), the buffer handed back before its second half is folded. Measured
+// on one B200 in a loop, SwiGLU fc1: 32 experts x 256 rows, K 7168, F 2048: 465 -> 292 us (1645
+// TFLOP/s); 1 x 16384 rows, K 4096, F 14336: 3321 -> 2225 us (1730 TFLOP/s); plain 331 -> 273 us and
+// 2509 -> 2183 us. Tried and slower: tokens on N as in the bf16 kernel (the scale then differs per
+// column: its shared-memory broadcasts cost 1024 cycles a block, 702 TFLOP/s); two MMAs of 128 columns with a
+// hand-over each (the A tile is read twice: 1593 against 1730).
+// Structure per CTA (persistent, one per SM, 384 threads = three warpgroups):
 //   warp 0      TMA producer: per reduction block one 128 x 128-byte tile of A and one
 //               256 x 128-byte tile of W (128-byte swizzle), 4-stage ring; plain loads of this
 //               GPU's memory, every CTA fetches its own tiles.
 //   warp 1      MMA issuer and TMEM owner: 4 MMAs (K = 32 each) per block, then two commits:
 //               one frees the shared-memory stage, one announces the partial accumulator.
-//   warps 2-9   promotion + epilogue: warp w works on TMEM lanes 32 * (w % 4) and on one half of
+//   warps 4-11  promotion + epilogue: warp w works on TMEM lanes 32 * (w % 4) and on one half of
 //               the columns (128 running sums per thread).
 // Epilogues: plain bf16 store; SwiGLU x prob (weights hold [gate rows | linear rows], a tile
 // multiplies 128 gate and the matching 128 linear rows; each thread keeps gate and linear sums of
@@ -44,7 +55,12 @@ constexpr int EPI_COLS = 32;                                   // output columns
 constexpr int EPI_ROW_BYTES = EPI_COLS * 2 + 16;               // 32 bf16 + pad (bank spread)
 constexpr int EPI_WARP_BYTES = 32 * EPI_ROW_BYTES;
 constexpr int SMEM_BYTES = RING_BYTES + EPI_WARPS * EPI_WARP_BYTES + 1024;
-constexpr int THREADS = 64 + EPI_WARPS * 32;
+constexpr int THREADS = 128 + EPI_WARPS * 32;
+// Registers: 384 threads are launched with 168 each (64512); the first warpgroup goes down to 56 and
+// the two epilogue warpgroups up to 224 (128 running sums, 64 values on the way, scales, addresses):
+// 128 * 56 + 256 * 224 = 64512.
+constexpr int REGS_FIRST = 56, REGS_EPI = 224;
+static_assert(128 * REGS_FIRST + EPI_WARPS * 32 * REGS_EPI <= THREADS * 168, "register split above the launch's total");
 constexpr int kMaxLocalExperts = 256;
 
 struct Tile { int e, row0, valid_rows, nt; };
@@ -52,9 +68,8 @@ struct Tile { int e, row0, valid_rows, nt; };
 // Same tile order as the bf16 kernel: inside an expert, bands of `gm` m-tiles; inside a band m
 // runs fastest, then n (the band of activation rows stays in L2 while the weight tiles pass).
 __device__ __forceinline__ bool decode_tile(int t, const int* s_tile_off, const int* s_row_off, int El,
-                                            int n_tiles, int gm, Tile& out) {
+                                            int n_tiles, int gm, int& e, Tile& out) {
   if (t >= s_tile_off[El]) return false;
-  int e = 0;
   while (e + 1 < El && t >= s_tile_off[e + 1]) ++e;
   const int local = t - s_tile_off[e];
   const int rows = s_row_off[e + 1] - s_row_off[e];
@@ -85,6 +100,21 @@ __device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t a_desc, uint6
       ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// two f32 in one register pair
+__device__ __forceinline__ uint64_t pack2(float v) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "r"(__float_as_uint(v)));
+  return r;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+// 32 columns: running sums acc[16] (pairs) += the partial v times the scale product, each rounded as fmaf rounds
+__device__ __forceinline__ void fold32(uint64_t* acc, const uint32_t* v, uint64_t s) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    asm("{\n.reg .b64 v;\nmov.b64 v, {%1, %2};\nfma.rn.f32x2 %0, v, %3, %0;\n}" : "+l"(acc[i]) : "r"(v[2 * i]), "r"(v[2 * i + 1]), "l"(s));
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -107,32 +137,49 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     for (int b = 0; b < 2; ++b) { mbar_init(&part_full[b], 1); mbar_init(&part_empty[b], EPI_WARPS); }
     s_abort = 0;
     fence_barrier_init();
-    int acc = 0;
-    for (int e = 0; e < p.El; ++e) {
-      int r0 = p.expert_off[e], r1 = p.expert_off[e + 1];
-      r0 = max(0, min(r0, p.max_rows));
-      r1 = max(r0, min(r1, p.max_rows));
-      s_row_off[e] = r0;
-      s_row_off[e + 1] = r1;
-      s_tile_off[e] = acc;
-      acc += ((r1 - r0 + BM - 1) / BM) * p.n_tiles;
-    }
-    s_tile_off[p.El] = acc;
     prefetch_tmap(&map_a);
     prefetch_tmap(&map_b);
   }
   if (warp == 1) tmem_alloc(&s_tmem, 512);
+  if (warp == 2) {
+    // device-side tile table
+    int acc = 0;
+    for (int e0 = 0; e0 < p.El; e0 += 32) {
+      const int e = e0 + lane;
+      int r0 = 0, r1 = 0, tiles = 0;
+      if (e < p.El) {
+        r0 = max(0, min(p.expert_off[e], p.max_rows));
+        r1 = max(r0, min(p.expert_off[e + 1], p.max_rows));
+        tiles = ((r1 - r0 + BM - 1) / BM) * p.n_tiles;
+      }
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+      }
+      if (e < p.El) {
+        s_tile_off[e] = acc + incl - tiles;
+        s_row_off[e] = r0;
+        if (e == p.El - 1) s_row_off[p.El] = r1;
+      }
+      acc += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_tile_off[p.El] = acc;
+  }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = s_tmem;
 
+  if (warp < 4) reg_dec<REGS_FIRST>();
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
       uint32_t it = 0;
+      int e = 0;
       Tile tl;
-      for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, tl) && !*abort; t += gridDim.x) {
+      for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, e, tl) && !*abort; t += gridDim.x) {
         // weight rows of this tile: [gate 128 | linear 128] for swiglu, 256 consecutive rows otherwise
         const int b_first = (EPI == EPI_SWIGLU) ? tl.e * p.w_rows + tl.nt * 128 : tl.e * p.w_rows + tl.nt * BN;
         const int b_second = (EPI == EPI_SWIGLU) ? b_first + p.N : b_first + 128;
@@ -159,8 +206,9 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     if (elect_one()) {
       const uint32_t idesc = instr_desc_e4m3(BM, BN);
       uint32_t it = 0;
+      int e = 0;
       Tile tl;
-      for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, tl) && !*abort; t += gridDim.x) {
+      for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, e, tl) && !*abort; t += gridDim.x) {
         bool ok = true;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
@@ -182,16 +230,17 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         if (!ok) break;
       }
     }
-  } else {
+  } else if (warp >= 4) {
     // ---------------- promotion + epilogue: 8 warps = 4 lane quarters x 2 column halves ----------------
-    const int ew = warp - 2;
+    reg_inc<REGS_EPI>();
+    const int ew = warp - 4;
     const int q = warp & 3;                        // TMEM lanes [32q, 32q+32) (a warp may only touch its own quarter)
     const int half = ew >> 2;                      // which half of the columns
     unsigned char* my_smem = epi_smem + ew * EPI_WARP_BYTES;
     uint32_t it = 0;
+    int e = 0;
     Tile tl;
-    const int kb_ld = p.sa_ld;
-    for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, tl) && !*abort; t += gridDim.x) {
+    for (int t = blockIdx.x; decode_tile(t, s_tile_off, s_row_off, p.El, p.n_tiles, gm, e, tl) && !*abort; t += gridDim.x) {
       const int my_row = tl.row0 + q * 32 + lane;
       const bool row_ok = q * 32 + lane < tl.valid_rows;
       // plain: my 128 columns are one 128-wide weight block; swiglu: 64 gate + the matching 64 linear columns
@@ -201,56 +250,53 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       // the scale index is clamped so that it stays inside the expert's scale rows)
       const int wblk_a = (EPI == EPI_SWIGLU) ? tl.nt : min(tl.nt * 2 + half, p.w_rows / 128 - 1);
       const int wblk_b = (EPI == EPI_SWIGLU) ? p.N / 128 + tl.nt : wblk_a;
-      const float* sw_a = p.sw + ((size_t)tl.e * (p.w_rows / 128) + wblk_a) * k_blocks;
-      const float* sw_b = p.sw + ((size_t)tl.e * (p.w_rows / 128) + wblk_b) * k_blocks;
-      const float* sa_row = p.sa + (size_t)my_row * kb_ld;
-      // the row's routing probability is needed only after the last block: fetch it now
-      float prob = 1.f;
-      if (EPI == EPI_SWIGLU && row_ok && p.row_prob) prob = __ldg(p.row_prob + my_row);
-      float acc[128];
+      const int sw_a = (tl.e * (p.w_rows / 128) + wblk_a) * k_blocks;      // (the launcher checks that these fit)
+      const int sw_b = (tl.e * (p.w_rows / 128) + wblk_b) * k_blocks;
+      const float* sa_row = p.sa + (size_t)my_row * p.sa_ld;
+      // Scales. My row's: the next block's is on its way. The weight blocks': lane i holds those of block
+      // i (mod 32), handed round by shuffles.
+      float sa_nxt = row_ok ? __ldg(sa_row) : 0.f, swl_a = 0.f, swl_b = 0.f;
+      uint64_t acc[64];                              // running sums, two columns each
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-      float sa_next = row_ok ? __ldg(sa_row) : 0.f;
+      for (int i = 0; i < 64; ++i) acc[i] = 0;
       bool ok = true;
       for (int kb = 0; kb < k_blocks; ++kb, ++it) {
         const int buf = it & 1;
-        const float sa_cur = sa_next;
-        if (kb + 1 < k_blocks && row_ok) sa_next = __ldg(sa_row + kb + 1);
-        const float fa = sa_cur * __ldg(sw_a + kb), fb = sa_cur * __ldg(sw_b + kb);
+        if ((kb & 31) == 0) {
+          swl_a = kb + lane < k_blocks ? __ldg(p.sw + sw_a + kb + lane) : 0.f;
+          if (EPI == EPI_SWIGLU) swl_b = kb + lane < k_blocks ? __ldg(p.sw + sw_b + kb + lane) : 0.f;
+        }
+        const float sa_cur = sa_nxt;
+        if (kb + 1 < k_blocks && row_ok) sa_nxt = __ldg(sa_row + kb + 1);
+        const float fa = sa_cur * __shfl_sync(0xffffffffu, swl_a, kb & 31);
+        const float fb = EPI == EPI_SWIGLU ? sa_cur * __shfl_sync(0xffffffffu, swl_b, kb & 31) : fa;
+        const uint64_t fa2 = pack2(fa), fb2 = pack2(fb);
         if (!mbar_wait(&part_full[buf], (it >> 1) & 1, p.status, abort)) { ok = false; break; }
         fence_after_sync();
         const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-        // four loads of 32 columns, software-pipelined: the next load is in flight while the
-        // previous one is folded into the running sums
-        const uint32_t c0 = t_addr + col_a, c1 = t_addr + col_a + 32, c2 = t_addr + col_b, c3 = t_addr + col_b + 32;
         uint32_t v0[32], v1[32];
-        tmem_ld32(c0, v0);
+        tmem_ld32(t_addr + col_a, v0);
+        tmem_ld32(t_addr + col_a + 32, v1);
         tmem_ld_wait();
         tmem_ld_pin(v0);
-        tmem_ld32(c1, v1);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = fmaf(fa, __uint_as_float(v0[i]), acc[i]);
-        tmem_ld_wait();
         tmem_ld_pin(v1);
-        tmem_ld32(c2, v0);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[32 + i] = fmaf(fa, __uint_as_float(v1[i]), acc[32 + i]);
+        fold32(acc, v0, fa2);
+        tmem_ld32(t_addr + col_b, v0);
+        fold32(acc + 16, v1, fa2);
+        tmem_ld32(t_addr + col_b + 32, v1);
         tmem_ld_wait();
         tmem_ld_pin(v0);
-        tmem_ld32(c3, v1);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[64 + i] = fmaf(fb, __uint_as_float(v0[i]), acc[64 + i]);
-        tmem_ld_wait();
         tmem_ld_pin(v1);
-        // every TMEM read of this block is done: hand the buffer back BEFORE the last fold
+        // every TMEM read of this block is done: hand the buffer back before the last folds
         fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&part_empty[buf]);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[96 + i] = fmaf(fb, __uint_as_float(v1[i]), acc[96 + i]);
+        fold32(acc + 32, v0, fb2);
+        fold32(acc + 48, v1, fb2);
       }
       if (!ok) break;
       if (tl.valid_rows <= 0) continue;
+      const float prob = (EPI == EPI_SWIGLU && row_ok && p.row_prob) ? __ldg(p.row_prob + my_row) : 1.f;
       // ---- store: EPI_COLS output columns per pass through the per-warp staging tile ----
       constexpr int PASSES = ((EPI == EPI_SWIGLU) ? 64 : 128) / EPI_COLS;
 #pragma unroll
@@ -261,11 +307,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           const int c = ps * EPI_COLS + 2 * i;
           float a0, a1;
           if (EPI == EPI_SWIGLU) {
-            a0 = silu(acc[c]) * acc[64 + c] * prob;
-            a1 = silu(acc[c + 1]) * acc[64 + c + 1] * prob;
+            a0 = silu(lo2(acc[c / 2])) * lo2(acc[32 + c / 2]) * prob;
+            a1 = silu(hi2(acc[c / 2])) * hi2(acc[32 + c / 2]) * prob;
           } else {
-            a0 = acc[c];
-            a1 = acc[c + 1];
+            a0 = lo2(acc[c / 2]);
+            a1 = hi2(acc[c / 2]);
           }
           __nv_bfloat162 hh = __floats2bfloat162_rn(a0, a1);
           packed[i] = *reinterpret_cast<uint32_t*>(&hh);
@@ -329,6 +375,7 @@ int launch_grouped_gemm_fp8(const void* a, long long a_rows, const void* w, int 
                             cudaStream_t st) {
   using namespace f8;
   if (p.El < 1 || p.El > kMaxLocalExperts || p.K <= 0 || p.K % BKB || p.N <= 0 || p.N % 128 || p.N_out % 8) return 1;
+  if ((long long)p.El * (p.w_rows / 128) * (p.K / BKB) > 0x7fffffff) return 1;
   if (p.w_rows % 128 || p.sa == nullptr || p.sw == nullptr || p.sa_ld < p.K / BKB) return 1;
   if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(w) % 16) return 1;
   if (epi != EPI_PLAIN && epi != EPI_SWIGLU) return 1;

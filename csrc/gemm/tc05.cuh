@@ -215,6 +215,10 @@ __device__ __forceinline__ void tmem_ld_pin16(uint32_t* r) {
       :: "memory");
 }
 
+// ---- registers moved between warpgroups (every warp of an aligned group of four executes them) ----
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---- named barriers of a 128-thread group -----------------------------------------------------
 __device__ __forceinline__ void group_sync(int id) { __syncwarp(); asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(id) : "memory"); }
 // true for every thread of the group if `ok` is true in all of them

@@ -271,7 +271,9 @@ def test_tcgen05_expert_mlp_gradients_match_fp32_autograd(activation):
 
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("counts,N,K", [([128], 256, 128), ([200, 0, 57], 384, 512), ([1, 300, 129, 0], 256, 1024),
-                                        ([513], 128, 7168)])
+                                        ([513], 128, 7168),
+                                        # more experts than a warp, several tiles per CTA, weight scales of two shuffle rounds
+                                        ([5, 0, 140] * 13 + [1], 640, 33 * 128)])
 def test_grouped_gemm_fp8_block_scaled(counts, N, K, swiglu):
     """e4m3 rows with 1x128 scales times e4m3 weights with 128x128 scales, against the fp32 matmul
     of the DEQUANTISED operands (the kernel multiplies exactly those numbers, so only the
