@@ -15,8 +15,15 @@
 //  * no host synchronisation and no host-side state per call: the call's epoch lives in device
 //    memory and is advanced by the kernel itself, regions are double-buffered by its parity,
 //    every kernel argument is constant -> the four kernels can be captured in a CUDA graph;
-//  * send and receive halves are separate launches (receive = bounded wait on the peers'
-//    flags, then local packing / weighted reduction), which also gives hook-style completion.
+//  * the receive half (bounded wait on the peers' flags, then the per-expert counts) is the last
+//    CTA's work of the send launch; with hook-style completion, and with several virtual ranks on
+//    one GPU, it is a launch of its own.
+// Bound: at decode sizes a chain of memory latencies, not bandwidth. What does not depend on
+// another rank (a token's row, its routing, the slots of a combine) is therefore requested before
+// the first wait, a group of one neither signals nor waits, and rows of the rank's own tokens are
+// combined where they lie. Measured as CUDA-graph replays on one B200 (128 tokens x 7168, top-8 of 32,
+// fp8, pull combine): 22.2 -> 12.5 us a round; an eager bf16 round trip of 7 tokens with the experts' output
+// elsewhere 40 -> 28 us, of which the kernels 22 -> 8 us.
 #include <cuda_bf16.h>
 #include "cast.cuh"
 #include "ep.cuh"
@@ -28,9 +35,10 @@ constexpr int kLLThreads = 256;  // 8 warps work on one row together
 
 // Per-op device state (6 ints): [0] committed epoch, [1] committed arrival target,
 // [2] epoch published by the send half, [3] target published by the send half,
-// [4] cumulative count of send CTAs that have finished (signal mode 1), [5] unused.
+// [4] cumulative count of send CTAs that have finished, [5] unused.
 // Send half: works with epoch = [0]+1, target = [1]+grid; CTA 0 publishes them in [2],[3].
-// Receive half (next launch on the stream): reads [2],[3]; CTA 0 commits them to [0],[1].
+// Receive half: the CTA of the send launch that finishes last (every CTA has read [0],[1] by then)
+// commits the pair to [0],[1]; as a launch of its own it reads [2],[3] and CTA 0 commits them.
 // No kernel ever reads a word that another CTA of the same launch writes.
 // The arrival target is a cumulative count modulo 2^32 (it grows by the grid size per call and
 // passes 2^31 after a few hours of decode steps): it is advanced in unsigned arithmetic and compared
@@ -76,25 +84,55 @@ __device__ __forceinline__ LLTick ll_tick_recv(int* st) {
 //     (state[4]); the CTA that completes a multiple of the grid size adds the whole grid size to
 //     the counter on every peer: R remote atomics per rank, at the price of one more hop.
 // Mode 0 measured faster with 2 ranks, mode 1 with 8.
-__device__ __forceinline__ void ll_arrive_on_peers(const LLParams& P, const PeerPtrs& peers, int channel,
-                                                   int* state, unsigned int grid_ctas) {
+// `elect`: also find the CTA that finishes last (its caller does the receive half); returns true in
+// that CTA. A group of one has no counters to keep: the end of the launch, or the election, orders it.
+__device__ __forceinline__ bool ll_arrive_on_peers(const LLParams& P, const PeerPtrs& peers, int channel,
+                                                   int* state, unsigned int grid_ctas, bool elect) {
   __shared__ unsigned int s_add;
+  __shared__ bool s_last;
+  if (P.R == 1 && !elect) return false;
   __syncthreads();
-  if (P.signal_mode == 0) {
-    if (threadIdx.x == 0) s_add = 1u;
-  } else if (threadIdx.x == 0) {
-    fence_acq_rel_sys();
-    const unsigned int prev = atomicAdd(reinterpret_cast<unsigned int*>(state + 4), 1u);
-    const bool last = ((prev + 1u) % grid_ctas) == 0u;
-    // the last CTA acquires what the others published before they counted themselves
-    if (last) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    s_add = last ? grid_ctas : 0u;
+  if (threadIdx.x == 0) {
+    bool last = false;
+    if (P.signal_mode != 0 || elect) {
+      if (P.R == 1) __threadfence();
+      else if (P.signal_mode != 0) fence_acq_rel_sys();
+      const unsigned int prev = atomicAdd(reinterpret_cast<unsigned int*>(state + 4), 1u);
+      last = ((prev + 1u) % grid_ctas) == 0u;
+      // the last CTA acquires what the others published before they counted themselves
+      if (last) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    s_add = P.signal_mode == 0 ? 1u : (last ? grid_ctas : 0u);
+    s_last = last;
   }
   __syncthreads();
   const unsigned int add = s_add;
-  if (add != 0u && threadIdx.x < P.R) {
+  if (P.R > 1 && add != 0u && threadIdx.x < P.R) {
     unsigned int* ctr = reinterpret_cast<unsigned int*>(peers.base[threadIdx.x] + P.flags) + channel * kMaxRanks + P.rank;
     asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(ctr), "r"(add) : "memory");
+  }
+  return elect && s_last;
+}
+
+// Receive half of a dispatch, run by one CTA: wait for every source's arrival, then read (and clear)
+// the per-expert row counters. Nothing is copied.
+__device__ __forceinline__ void ll_publish_counts(const LLParams& P, char* self_base, LLTick tk,
+                                                  int* __restrict__ out_count, int* status) {
+  __shared__ int ok;
+  const int par = tk.epoch & 1;
+  if (threadIdx.x == 0) ok = 1;
+  __syncthreads();
+  if (P.R > 1 && threadIdx.x < P.R) {
+    const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLDispatch * kMaxRanks;
+    if (!wait_counter_reached(flags + threadIdx.x, tk.target, P.timeout_ns, status, kTimeoutLowLatency)) ok = 0;
+  }
+  __syncthreads();
+  int* cnt = reinterpret_cast<int*>(self_base + P.count[par]);
+  for (int el = threadIdx.x; el < P.El; el += kLLThreads) {
+    int c = ok ? __ldcg(&cnt[el]) : 0;
+    c = c < 0 ? 0 : (c > P.R * P.M ? P.R * P.M : c);
+    out_count[el] = c;
+    cnt[el] = 0;                 // this parity is used again two dispatches from now
   }
 }
 
@@ -102,25 +140,55 @@ __device__ __forceinline__ void ll_arrive_on_peers(const LLParams& P, const Peer
 // dispatch, send half: one CTA per token at a time.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kLLThreads)
-ll_dispatch_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
-                        const long long* __restrict__ topk_idx, int* send_cnt_all, int* state,
-                        int* status, int* __restrict__ send_slot) {
+ll_dispatch_send_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, const char* __restrict__ x,
+                        const long long* __restrict__ topk_idx, int* state, int* status,
+                        int* __restrict__ send_slot, int* __restrict__ out_count) {
   __shared__ char* s_dst[kMaxItemsPerToken];
   __shared__ float* s_scl[kMaxItemsPerToken];
   __shared__ int s_n;
   ll_stream_order();
-  const LLTick tk = ll_tick_send(state, gridDim.x);
-  const int epoch = tk.epoch;
-  const int par = epoch & 1;
-  (void)send_cnt_all;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kLLThreads / 32;
   const int row_bytes = P.fp8 ? P.H : P.H * 2;
   const int scale_cols = P.H / 128;
+  const int nsteps = (P.H + 511) / 512, nvec = (P.H * 2) >> 4;
+  // One batch of a row: fp8 up to 4 steps of 512 channels per warp (two vectors per lane each), bf16 up to 4
+  // vectors per thread. The first batch and the routing of a token are requested ahead: before the state
+  // words are read, or while the token before it is stored.
+  uint4 r[8];
+  long long my_e = -1;
+  auto load = [&](int t, int b) {
+    const char* src = x + (size_t)t * P.H * 2;
+    if (P.fp8) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int el = (b + u * nwarps) * 512 + lane * 16;
+        r[2 * u] = make_uint4(0, 0, 0, 0);
+        r[2 * u + 1] = r[2 * u];
+        if (b + u * nwarps < nsteps && el < P.H) {
+          r[2 * u] = ld_global_nc_v4(src + (size_t)el * 2);
+          r[2 * u + 1] = ld_global_nc_v4(src + (size_t)el * 2 + 16);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (b + u * kLLThreads < nvec) r[u] = ld_global_nc_v4(src + ((size_t)(b + u * kLLThreads) << 4));
+    }
+  };
+  const int b_first = P.fp8 ? warp : (int)threadIdx.x, b_step = P.fp8 ? 4 * nwarps : 4 * kLLThreads;
+  const int b_end = P.fp8 ? nsteps : nvec;
+  auto ahead = [&](int t) {
+    if (t >= P.T) return;
+    if (threadIdx.x < P.K) my_e = topk_idx[(size_t)t * P.K + threadIdx.x];
+    load(t, b_first);
+  };
+  ahead(blockIdx.x);
+  if (threadIdx.x == 0) s_n = 0;
+  const LLTick tk = ll_tick_send(state, gridDim.x);
+  const int par = tk.epoch & 1;
   for (int t = blockIdx.x; t < P.T; t += gridDim.x) {
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
     if (threadIdx.x < P.K) {
-      const long long e = topk_idx[(size_t)t * P.K + threadIdx.x];
+      const long long e = my_e;
       int given = -1;
       if (e >= 0 && e < P.E) {
         const int d = (int)e / P.El, el = (int)e % P.El;
@@ -146,28 +214,15 @@ ll_dispatch_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
     }
     __syncthreads();
     const int n = s_n;
-    const char* src = x + (size_t)t * P.H * 2;
-    if (P.fp8) {
-      const int nsteps = (P.H + 511) / 512;
-      // up to 4 steps per warp with all loads issued before the first conversion
-      for (int it0 = warp; it0 < nsteps; it0 += 4 * nwarps) {
-        uint4 a[4], b[4];
+    for (int b = b_first; b < b_end; b += b_step) {
+      if (b != b_first) load(t, b);
+      if (P.fp8) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int el = (it0 + u * nwarps) * 512 + lane * 16;
-          a[u] = make_uint4(0, 0, 0, 0);
-          b[u] = a[u];
-          if (it0 + u * nwarps < nsteps && el < P.H) {
-            a[u] = ld_global_nc_v4(src + (size_t)el * 2);
-            b[u] = ld_global_nc_v4(src + (size_t)el * 2 + 16);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (it0 + u * nwarps >= nsteps) break;       // uniform per warp
-          const int el = (it0 + u * nwarps) * 512 + lane * 16;
+          if (b + u * nwarps >= nsteps) break;       // uniform per warp
+          const int el = (b + u * nwarps) * 512 + lane * 16;
           float scale;
-          const uint4 o = cast_block_fp8(a[u], b[u], &scale);
+          const uint4 o = cast_block_fp8(r[2 * u], r[2 * u + 1], &scale);
           if (el < P.H) {
             for (int j = 0; j < n; ++j) {
               st_global_v4(s_dst[j] + el, o);
@@ -175,49 +230,34 @@ ll_dispatch_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
             }
           }
         }
-      }
-    } else {
-      const int nvec = (P.H * 2) >> 4;
-      for (int v0 = threadIdx.x; v0 < nvec; v0 += 4 * kLLThreads) {
-        uint4 val[4];
+      } else {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (v0 + u * kLLThreads < nvec) val[u] = ld_global_nc_v4(src + ((size_t)(v0 + u * kLLThreads) << 4));
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (v0 + u * kLLThreads < nvec)
-            for (int j = 0; j < n; ++j) st_global_v4(s_dst[j] + ((size_t)(v0 + u * kLLThreads) << 4), val[u]);
+          if (b + u * kLLThreads < nvec)
+            for (int j = 0; j < n; ++j) st_global_v4(s_dst[j] + ((size_t)(b + u * kLLThreads) << 4), r[u]);
       }
     }
-    __syncthreads();
+    if (t + (int)gridDim.x < P.T) {
+      ahead(t + gridDim.x);
+      __syncthreads();                       // everybody has read s_n and the destinations
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+    }
   }
-  ll_arrive_on_peers(P, peers, kChLLDispatch, state, gridDim.x);
+  if (ll_arrive_on_peers(P, peers, kChLLDispatch, state, gridDim.x, out_count != nullptr)) {
+    ll_publish_counts(P, peers.base[P.rank], tk, out_count, status);
+    if (threadIdx.x == 0) { state[0] = tk.epoch; state[1] = (int)tk.target; }
+  }
 }
 
 // ---------------------------------------------------------------------------------------
-// dispatch, receive half: wait for every source's arrival, then read (and clear) the per-expert
-// row counters. One CTA; nothing is copied.
+// dispatch, receive half as a launch of its own (hook-style completion, virtual ranks). One CTA.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kLLThreads)
 ll_dispatch_recv_kernel(LLParams P, char* self_base, int* __restrict__ out_count, int* state, int* status) {
-  __shared__ int ok;
   ll_stream_order();
   const LLTick tk = ll_tick_recv(state);
-  const int par = tk.epoch & 1;
-  if (threadIdx.x == 0) ok = 1;
-  __syncthreads();
-  if (threadIdx.x < P.R) {
-    const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLDispatch * kMaxRanks;
-    if (!wait_counter_reached(flags + threadIdx.x, tk.target, P.timeout_ns, status, kTimeoutLowLatency)) ok = 0;
-  }
-  __syncthreads();
-  int* cnt = reinterpret_cast<int*>(self_base + P.count[par]);
-  for (int el = threadIdx.x; el < P.El; el += kLLThreads) {
-    int c = ok ? __ldcg(&cnt[el]) : 0;
-    c = c < 0 ? 0 : (c > P.R * P.M ? P.R * P.M : c);
-    out_count[el] = c;
-    cnt[el] = 0;                 // this parity is used again two dispatches from now
-  }
+  ll_publish_counts(P, self_base, tk, out_count, status);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -226,7 +266,7 @@ ll_dispatch_recv_kernel(LLParams P, char* self_base, int* __restrict__ out_count
 __global__ void __launch_bounds__(kLLThreads)
 ll_combine_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
                        const int* __restrict__ src_info, const int* __restrict__ count,
-                       int* state, int* status) {
+                       int* state, int* status, int own_in_place) {
   ll_stream_order();
   const LLTick tk = ll_tick_send(state, gridDim.x * gridDim.y);
   const int par = tk.epoch & 1;
@@ -248,6 +288,7 @@ ll_combine_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
       if (lane == 0) set_status(status, kOverflowSlots);
       continue;
     }
+    if (own_in_place && s == P.rank) continue;       // the receive half reads it where it lies
     const char* src = x + ((size_t)el * cap + j) * row_bytes;
     char* dst = peers.base[s] + P.comb_x[par] + ((size_t)t * P.K + k) * row_bytes;
     const int nv = row_bytes >> 4;
@@ -261,22 +302,23 @@ ll_combine_send_kernel(LLParams P, PeerPtrs peers, const char* __restrict__ x,
         if (v0 + u * 32 < nv) st_global_v4(dst + ((size_t)(v0 + u * 32) << 4), buf[u]);
     }
   }
-  ll_arrive_on_peers(P, peers, kChLLCombine, state, gridDim.x * gridDim.y);
+  ll_arrive_on_peers(P, peers, kChLLCombine, state, gridDim.x * gridDim.y, false);
 }
 
 // combine, receive half: out[t] = sum_k w[t,k] * slot(t,k) over k with topk_idx[t,k] >= 0.
 __global__ void __launch_bounds__(kLLThreads)
 ll_combine_recv_kernel(LLParams P, char* self_base, const long long* __restrict__ topk_idx,
                        const float* __restrict__ topk_w, char* __restrict__ out,
-                       int* state, int* status) {
+                       int* state, int* status, const char* __restrict__ own_x, const int* __restrict__ send_slot) {
   __shared__ float s_w[kMaxItemsPerToken];
+  __shared__ const char* s_row[kMaxItemsPerToken];
   __shared__ int ok;
   ll_stream_order();
   const LLTick tk = ll_tick_recv(state);
   const int par = tk.epoch & 1;
   if (threadIdx.x == 0) ok = 1;
   __syncthreads();
-  if (threadIdx.x < P.R) {
+  if (P.R > 1 && threadIdx.x < P.R) {
     const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLCombine * kMaxRanks;
     if (!wait_counter_reached(flags + threadIdx.x, tk.target, P.timeout_ns, status, kTimeoutLowLatency)) ok = 0;
   }
@@ -287,10 +329,19 @@ ll_combine_recv_kernel(LLParams P, char* self_base, const long long* __restrict_
   for (int t = blockIdx.x; t < P.T; t += gridDim.x) {
     if (threadIdx.x < P.K) {
       const long long e = topk_idx[(size_t)t * P.K + threadIdx.x];
-      s_w[threadIdx.x] = (e >= 0 && e < P.E) ? (topk_w ? topk_w[(size_t)t * P.K + threadIdx.x] : 1.f) : 0.f;
+      float w = (e >= 0 && e < P.E) ? (topk_w ? topk_w[(size_t)t * P.K + threadIdx.x] : 1.f) : 0.f;
+      const char* row = self_base + P.comb_x[par] + ((size_t)t * P.K + threadIdx.x) * row_bytes;
+      if (own_x != nullptr && e >= 0 && e < P.E && (int)e / P.El == P.rank) {
+        // an own row: packed row `slot` of local expert e - rank * El, where the experts wrote it
+        const int slot = send_slot[(size_t)t * P.K + threadIdx.x];
+        const size_t cap = (size_t)P.R * P.M;
+        if (slot < 0 || (size_t)slot >= cap) w = 0.f;
+        else row = own_x + ((size_t)((int)e % P.El) * cap + slot) * row_bytes;
+      }
+      s_w[threadIdx.x] = w;
+      s_row[threadIdx.x] = row;
     }
     __syncthreads();
-    const char* base = self_base + P.comb_x[par] + (size_t)t * P.K * row_bytes;
     for (int v = threadIdx.x; v < nvec; v += kLLThreads) {
       float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       for (int k0 = 0; k0 < P.K; k0 += 8) {
@@ -298,7 +349,7 @@ ll_combine_recv_kernel(LLParams P, char* self_base, const long long* __restrict_
 #pragma unroll
         for (int u = 0; u < 8; ++u)       // loads first (independent), then the fp32 accumulation
           if (k0 + u < P.K && s_w[k0 + u] != 0.f)
-            val[u] = ld_global_v4(base + (size_t)(k0 + u) * row_bytes + ((size_t)v << 4));
+            val[u] = ld_global_v4(s_row[k0 + u] + ((size_t)v << 4));
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           if (k0 + u >= P.K) break;
@@ -325,18 +376,40 @@ ll_combine_recv_kernel(LLParams P, char* self_base, const long long* __restrict_
 
 // ---------------------------------------------------------------------------------------
 // combine, pull form: announce, wait, load + reduce. One warp per (token, eighth of the row);
-// the rows of four experts are requested together, so a token costs two NVLink round trips.
+// the rows of up to eight experts are requested together, so a token costs one NVLink round trip
+// for eight of its choices. Lane k looks after choice k; its indices are loaded before the wait.
 // ---------------------------------------------------------------------------------------
-constexpr int kPullGroup = 4;    // contributors whose loads are in flight together
+constexpr int kPullGroup = 8;    // contributors whose loads are in flight together
 constexpr int kPullUnroll = 4;   // 16-byte vectors per lane and contributor
 
 __global__ void __launch_bounds__(kLLThreads)
-ll_combine_pull_kernel(LLParams P, PeerPtrs peers, int phase, const int* __restrict__ send_slot, const long long* __restrict__ topk_idx,
-                       const float* __restrict__ topk_w, char* __restrict__ out, int* state, int* status) {
+ll_combine_pull_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, int phase, const int* __restrict__ send_slot,
+                       const long long* __restrict__ topk_idx, const float* __restrict__ topk_w,
+                       char* __restrict__ out, int* state, int* status, const char* own_x) {
   __shared__ int s_epoch;
   __shared__ unsigned int s_target;
   __shared__ int s_ok;
   ll_stream_order();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kLLThreads / 32;
+  const int row_bytes = P.H * 2;
+  const int nvec = row_bytes >> 4;
+  int parts = (nvec + 32 * kPullUnroll - 1) / (32 * kPullUnroll);   // one batch of loads per warp and contributor
+  if (parts < 1) parts = 1;
+  const int part_vec = (nvec + parts - 1) / parts;
+  const size_t cap = (size_t)P.R * P.M;
+  const int items = P.T * parts, stride = gridDim.x * nwarps;
+  long long my_e = -1;
+  int my_slot = -1;
+  float my_w = 0.f;
+  auto fetch = [&](int it) {
+    if (phase == 1 || it >= items || lane >= P.K) return;
+    const size_t at = (size_t)(it / parts) * P.K + lane;
+    my_e = topk_idx[at];
+    my_slot = send_slot[at];
+    my_w = topk_w ? topk_w[at] : 1.f;
+  };
+  int it = blockIdx.x * nwarps + warp;
+  fetch(it);
   // state: [0] committed epoch, [1] committed arrival target, [2],[3] the pair published by an
   // announce-only launch, [4] CTAs of this launch that have finished
   if (threadIdx.x == 0) {
@@ -354,7 +427,7 @@ ll_combine_pull_kernel(LLParams P, PeerPtrs peers, int phase, const int* __restr
   const int epoch = s_epoch;
   const unsigned int target = s_target;
   char* self_base = peers.base[P.rank];
-  if (phase != 2 && blockIdx.x == 0) {
+  if (P.R > 1 && phase != 2 && blockIdx.x == 0) {
     // announce: my expert output (written by earlier kernels of this stream) may be read
     if ((int)threadIdx.x < P.R) {
       unsigned int* ctr = reinterpret_cast<unsigned int*>(peers.base[threadIdx.x] + P.flags) + kChLLPull * kMaxRanks + P.rank;
@@ -362,23 +435,27 @@ ll_combine_pull_kernel(LLParams P, PeerPtrs peers, int phase, const int* __restr
     }
   }
   if (phase == 1) return;
-  if ((int)threadIdx.x < P.R) {
-    const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLPull * kMaxRanks;
-    if (!wait_counter_reached(flags + threadIdx.x, target, P.timeout_ns, status, kTimeoutLowLatency)) s_ok = 0;
+  if (P.R > 1) {
+    if ((int)threadIdx.x < P.R) {
+      const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLPull * kMaxRanks;
+      if (!wait_counter_reached(flags + threadIdx.x, target, P.timeout_ns, status, kTimeoutLowLatency)) s_ok = 0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (s_ok) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kLLThreads / 32;
-    const int row_bytes = P.H * 2;
-    const int nvec = row_bytes >> 4;
-    int parts = (nvec + 32 * kPullUnroll - 1) / (32 * kPullUnroll);   // one batch of loads per warp and contributor
-    if (parts < 1) parts = 1;
-    const int part_vec = (nvec + parts - 1) / parts;
-    const size_t cap = (size_t)P.R * P.M;
-    const int items = P.T * parts;
-    for (int it = blockIdx.x * nwarps + warp; it < items; it += gridDim.x * nwarps) {
+    for (; it < items; it += stride) {
       const int t = it / parts, part = it % parts;
       const int v_lo = part * part_vec, v_hi = min(nvec, v_lo + part_vec);
+      // the row that dispatch stored for choice `lane`: packed row `slot` of local expert el on rank d
+      const char* my_row = nullptr;
+      float w = 0.f;
+      if (lane < P.K && my_e >= 0 && my_e < P.E && my_slot >= 0 && (size_t)my_slot < cap) {
+        const int d = (int)my_e / P.El, el = (int)my_e % P.El;
+        const char* base = (own_x != nullptr && d == P.rank) ? own_x : peers.base[d] + P.comb_in;
+        my_row = base + ((size_t)el * cap + my_slot) * row_bytes;
+        w = my_w;
+      }
+      fetch(it + stride);
       float acc[kPullUnroll][8];
 #pragma unroll
       for (int u = 0; u < kPullUnroll; ++u)
@@ -389,17 +466,9 @@ ll_combine_pull_kernel(LLParams P, PeerPtrs peers, int phase, const int* __restr
         float wk[kPullGroup];
 #pragma unroll
         for (int g = 0; g < kPullGroup; ++g) {
-          const int k = k0 + g;
-          wk[g] = 0.f;
-          if (k >= P.K) continue;
-          const long long e = topk_idx[(size_t)t * P.K + k];
-          const int slot = send_slot[(size_t)t * P.K + k];
-          if (e < 0 || e >= P.E || slot < 0) continue;
-          const int d = (int)e / P.El, el = (int)e % P.El;
-          if ((size_t)slot >= cap) continue;
-          wk[g] = topk_w ? topk_w[(size_t)t * P.K + k] : 1.f;
-          // the row that dispatch stored for (t, k): packed row `slot` of local expert el on rank d
-          const char* rowp = peers.base[d] + P.comb_in + ((size_t)el * cap + slot) * row_bytes;
+          const char* rowp = reinterpret_cast<const char*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(my_row), (k0 + g) & 31));
+          wk[g] = __shfl_sync(0xffffffffu, w, (k0 + g) & 31);
+          if (k0 + g >= P.K || rowp == nullptr) { wk[g] = 0.f; continue; }
 #pragma unroll
           for (int u = 0; u < kPullUnroll; ++u) {
             const int v = v_lo + u * 32 + lane;
@@ -466,32 +535,33 @@ static void ll_launch(void (*kern)(KArgs...), dim3 grid, bool pdl, cudaStream_t 
 }
 
 void launch_ll_dispatch_send(const LLParams& P, const PeerPtrs& peers, const char* x,
-                             const long long* topk_idx, int* send_cnt, int* state, int* status,
-                             cudaStream_t st, int* send_slot) {
-  ll_launch(ll_dispatch_send_kernel, dim3(P.G), P.pdl != 0, st, P, peers, x, topk_idx, send_cnt, state, status,
-            send_slot);
+                             const long long* topk_idx, int* state, int* status,
+                             cudaStream_t st, int* send_slot, int* out_count) {
+  ll_launch(ll_dispatch_send_kernel, dim3(P.G), P.pdl != 0, st, P, peers, x, topk_idx, state, status, send_slot, out_count);
 }
 void launch_ll_dispatch_recv(const LLParams& P, char* self_base, int* out_count, int* state, int* status,
                              cudaStream_t st) {
   ll_launch(ll_dispatch_recv_kernel, dim3(1), P.pdl != 0, st, P, self_base, out_count, state, status);
 }
 void launch_ll_combine_send(const LLParams& P, const PeerPtrs& peers, const char* x, const int* src_info,
-                            const int* count, int* state, int* status, cudaStream_t st) {
-  ll_launch(ll_combine_send_kernel, dim3(P.El, P.Gc / P.El), P.pdl != 0, st, P, peers, x, src_info, count, state, status);
+                            const int* count, int* state, int* status, bool own_in_place, cudaStream_t st) {
+  ll_launch(ll_combine_send_kernel, dim3(P.El, P.Gc / P.El), P.pdl != 0, st, P, peers, x, src_info, count, state, status,
+            own_in_place ? 1 : 0);
 }
 void launch_ll_combine_recv(const LLParams& P, char* self_base, const long long* topk_idx,
                             const float* topk_w, char* out, int* state, int* status,
-                            int blocks, cudaStream_t st) {
+                            int blocks, const char* own_x, const int* send_slot, cudaStream_t st) {
   int g = P.T < blocks ? P.T : blocks;
   if (g < 1) g = 1;
-  ll_launch(ll_combine_recv_kernel, dim3(g), P.pdl != 0, st, P, self_base, topk_idx, topk_w, out, state, status);
+  ll_launch(ll_combine_recv_kernel, dim3(g), P.pdl != 0, st, P, self_base, topk_idx, topk_w, out, state, status, own_x,
+            send_slot);
 }
 
 void launch_ll_combine_pull(const LLParams& P, const PeerPtrs& peers, int phase, const int* send_slot,
                             const long long* topk_idx, const float* topk_w, char* out, int* state,
-                            int* status, cudaStream_t st) {
+                            int* status, const char* own_x, cudaStream_t st) {
   ll_launch(ll_combine_pull_kernel, dim3(phase == 1 ? 1 : P.G), P.pdl != 0, st, P, peers, phase, send_slot,
-            topk_idx, topk_w, out, state, status);
+            topk_idx, topk_w, out, state, status, own_x);
 }
 
 }  // namespace b200ep

@@ -834,7 +834,6 @@ class Buffer:
                 # because the peers' arrival counters are cumulative
                 self._ll_words = torch.zeros(18, dtype=torch.int32, device=dev)
             self._ll = dict(key=key, carve=carve, words=self._ll_words,
-                            send_cnt=torch.zeros(2 * E, dtype=torch.int32, device=dev),
                             send_slot=torch.full((M * K,), -1, dtype=torch.int32, device=dev))
             self._carve = None
         return self._ll
@@ -849,7 +848,8 @@ class Buffer:
                 (1 if R >= 8 else 0) if Buffer.ll_signal_mode is None else int(Buffer.ll_signal_mode),
                 int(bool(Buffer.ll_overlap_launches)), c.comb_in, *c.range_tab]
 
-    def _ll_dispatch_send(self, x, topk_idx, M, E, use_fp8):
+    def _ll_dispatch_send(self, x, topk_idx, M, E, use_fp8, fused=False):
+        """fused: the same launch also does the receive half (its last CTA waits for the peers)."""
         if x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous():
             raise ValueError("low-latency dispatch takes a contiguous bf16 [tokens, hidden] tensor")
         T, H = x.shape
@@ -866,9 +866,9 @@ class Buffer:
             self.barrier()
         self._ll_dispatch_pending = True
         pv = self._ll_params(st, T, use_fp8)
-        self.C.ll_dispatch_send(pv, self.peers, x, topk_idx, st["send_cnt"], st["words"][0:6], self.status_ptr,
-                                st["send_slot"])
-        return dict(st=st, pv=pv, T=T, H=H, K=K, E=E, M=M, fp8=use_fp8, topk_idx=topk_idx, x=x)
+        count = torch.empty((E // self.group_size,), dtype=torch.int32, device=self.device) if fused else None
+        self.C.ll_dispatch_send(pv, self.peers, x, topk_idx, st["words"][0:6], self.status_ptr, st["send_slot"], count)
+        return dict(st=st, pv=pv, T=T, H=H, K=K, E=E, M=M, fp8=use_fp8, topk_idx=topk_idx, x=x, count=count)
 
     def _ll_dispatch_recv(self, d):
         """Count-only: the rows already lie packed per local expert in the receive region, which is
@@ -876,8 +876,10 @@ class Buffer:
         R, El, M, H = self.group_size, d["E"] // self.group_size, d["M"], d["H"]
         c = d["st"]["carve"]
         rows = R * M
-        out_count = torch.empty((El,), dtype=torch.int32, device=self.device)
-        self.C.ll_dispatch_recv(d["pv"], self.region.local_ptr, out_count, d["st"]["words"][0:6], self.status_ptr)
+        out_count = d["count"]
+        if out_count is None:
+            out_count = torch.empty((El,), dtype=torch.int32, device=self.device)
+            self.C.ll_dispatch_recv(d["pv"], self.region.local_ptr, out_count, d["st"]["words"][0:6], self.status_ptr)
         if d["fp8"]:
             out_x = (self.region.view(c.recv_x[0], (El, rows, H), "float8_e4m3fn"),
                      self.region.view(c.recv_scales[0], (El, rows, H // 128), "float32"))
@@ -899,7 +901,8 @@ class Buffer:
         the returned hook launches the receive half (then fills the same tensors)."""
         compute = self._enter(None, False, False)
         with self._on_stream():
-            d = self._ll_dispatch_send(x, topk_idx, num_max_dispatch_tokens_per_rank, num_experts, use_fp8)
+            d = self._ll_dispatch_send(x, topk_idx, num_max_dispatch_tokens_per_rank, num_experts, use_fp8,
+                                       fused=self._single_launch and not return_recv_hook)
             if return_recv_hook:
                 box = {}
 
@@ -925,7 +928,7 @@ class Buffer:
         El = E // self.group_size
         return self.region.view(st["carve"].comb_in, (El, self.group_size * M, H), "bfloat16")
 
-    def _ll_combine_pull(self, phase: int, topk_idx, topk_weights, handle, out=None):
+    def _ll_combine_pull(self, phase: int, topk_idx, topk_weights, handle, out=None, own_x=None):
         _src, _rng, M, H, E, _count, K = handle
         if phase != 2:
             self._ll_dispatch_pending = False
@@ -937,7 +940,7 @@ class Buffer:
             out = torch.empty((T, H), dtype=torch.bfloat16, device=self.device)
         w = topk_weights.to(torch.float32).contiguous() if topk_weights is not None else None
         self.C.ll_combine_pull(pv, self.peers, phase, st["send_slot"], topk_idx, w, out,
-                               st["words"][12:18], self.status_ptr)
+                               st["words"][12:18], self.status_ptr, own_x)
         return out
 
     def _ll_is_combine_buffer(self, x, handle) -> bool:
@@ -945,15 +948,20 @@ class Buffer:
             return False
         return x.data_ptr() == self.region.local_ptr + self._ll["carve"].comb_in
 
-    def _ll_combine_send(self, x, handle):
-        src_info, _range, M, H, E, count, K = handle
-        st = self._ll_state(E, K, H, M)
+    @staticmethod
+    def _ll_check_combine_input(x):
         if x.dtype != torch.bfloat16 or not x.is_contiguous():
             raise ValueError("low-latency combine takes a contiguous bf16 [E_local, R*M, hidden] tensor")
+
+    def _ll_combine_send(self, x, handle, own_in_place=True):
+        """own_in_place: rows of this rank's own tokens stay where they are; `_ll_combine_recv` reads them there."""
+        src_info, _range, M, H, E, count, K = handle
+        st = self._ll_state(E, K, H, M)
+        self._ll_check_combine_input(x)
         pv = self._ll_params(st, 0, False)
         self._ll_dispatch_pending = False
-        self.C.ll_combine_send(pv, self.peers, x, src_info, count, st["words"][6:12], self.status_ptr)
-        return dict(st=st, H=H)
+        self.C.ll_combine_send(pv, self.peers, x, src_info, count, st["words"][6:12], self.status_ptr, own_in_place)
+        return dict(st=st, H=H, own_x=x if own_in_place else None)
 
     def _ll_combine_recv(self, c, topk_idx, topk_weights, out=None):
         topk_idx = topk_idx.to(torch.int64).contiguous()
@@ -963,7 +971,7 @@ class Buffer:
             out = torch.empty((T, c["H"]), dtype=torch.bfloat16, device=self.device)
         w = topk_weights.to(torch.float32).contiguous() if topk_weights is not None else None
         self.C.ll_combine_recv(pv, self.region.local_ptr, topk_idx, w, out, c["st"]["words"][6:12],
-                               self.status_ptr, max(Buffer.num_sms * 4, 1))
+                               self.status_ptr, max(Buffer.num_sms * 4, 1), c["own_x"], c["st"]["send_slot"])
         return out
 
     @_nvtx("b200ep.ll_combine")
@@ -983,8 +991,15 @@ class Buffer:
                     res = self._ll_combine_pull(2, topk_idx, topk_weights, handle, res)
             ev = self._exit(compute, async_finish, [res])
             return res, ev, ((lambda: res) if return_recv_hook else None)
+        if self.group_size == 1 and not return_recv_hook:
+            # every row is an own row: one kernel, nothing is sent
+            self._ll_check_combine_input(x)
+            with self._on_stream():
+                res = self._ll_combine_pull(0, topk_idx, topk_weights, handle, out, own_x=x)
+            return res, self._exit(compute, async_finish, [res, x]), None
         with self._on_stream():
-            c = self._ll_combine_send(x, handle)
+            # (with a hook the caller may reuse x before the receive half runs: every row goes to its slot)
+            c = self._ll_combine_send(x, handle, own_in_place=not return_recv_hook)
             if return_recv_hook:
                 def hook():
                     with self._on_stream():

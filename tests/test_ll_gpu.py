@@ -186,3 +186,50 @@ def test_low_latency_pull_combine_under_cuda_graph_replay():
         g.check_status()
     finally:
         g.destroy()
+
+
+# one rank, through the public calls: several tokens per CTA, rows of more than one batch of loads, more choices than
+# are loaded together, masked choices; eager and hook-style completion in turn on the same buffer
+@pytest.mark.parametrize("T,H,E,K,fp8", [(1, 1024, 8, 1, True), (7, 4096, 16, 4, False), (300, 512, 8, 8, True),
+                                         (131, 264, 32, 9, False), (5, 17408, 16, 3, True), (3, 16640, 8, 2, False)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_low_latency_one_rank_public_calls(T, H, E, K, fp8, in_place):
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    buf = Buffer(None, Buffer.get_low_latency_nvl_size_hint(T, H, 1, E, K), 0, low_latency_mode=True,
+                 world=LocalWorld.make(1)[0], timeout_s=2.0)
+    try:
+        for rep in range(5):
+            g = torch.Generator().manual_seed(rep)
+            x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+            idx, w = O.make_routing(T, E, K, 50 + rep)
+            idx[T // 2, K - 1] = -1
+            idx_c, w_c = idx.cuda(), w.cuda()
+            hook_d, hook_c = rep in (1, 3), rep in (2, 3)
+            recv, count, handle, _, hook = buf.low_latency_dispatch(x, idx_c, T, E, use_fp8=fp8, return_recv_hook=hook_d)
+            if hook_d:
+                recv, count, handle = hook()
+            assert count.tolist() == [int((idx == e).sum()) for e in range(E)]
+            if fp8:
+                y = (recv[0].float().view(E, T, -1, 128) * recv[1][..., None]).view(E, T, H).to(torch.bfloat16)
+            else:
+                y = recv.clone()
+            y = y * (1 + torch.arange(E, device="cuda", dtype=torch.bfloat16))[:, None, None]     # the experts
+            for e in range(E):
+                y[e, int(count[e]):] = float("nan")                       # rows that nobody owns are never read
+            if in_place:
+                z = buf.get_next_low_latency_combine_buffer(handle)
+                z.copy_(y)
+                y = z
+            out, _, hook = buf.low_latency_combine(y, idx_c, w_c, handle, return_recv_hook=hook_c)
+            if hook_c and out is None:
+                out = hook()
+            factor = torch.where(idx >= 0, (1 + idx).float() * w, torch.zeros(())).sum(1, keepdim=True)
+            # bf16 rounding of the row, of the expert's product and of the result (2^-8 each), e4m3 rows 2^-4
+            tol = 2.0 ** -4 if fp8 else 2.0 ** -7
+            want = x.float().cpu() * factor
+            scale = x.float().abs().amax(1, keepdim=True).cpu() * factor
+            assert bool(((out.float().cpu() - want).abs() <= tol * (want.abs() + (scale * 2.0 ** -5 if fp8 else 1e-3))).all())
+        buf.check_status()
+    finally:
+        buf.destroy()
