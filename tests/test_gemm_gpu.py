@@ -206,6 +206,24 @@ def test_ungated_activation_kernels_match_autograd(kind):
     torch.testing.assert_close(dp, pf.grad, atol=5e-2, rtol=2e-2)
 
 
+# one warp per row (many rows) up to eight (few rows), a row of one vector, rows that leave lanes and warps without work.
+# Tolerance: dh is one bf16 rounding (2^-8 covers a value at the boundary) of f32 arithmetic, dp an f32 sum of F terms.
+@pytest.mark.parametrize("rows,F", [(2500, 264), (2368, 8), (1300, 776), (600, 1416), (37, 2824), (1, 4096), (3, 8)])
+@pytest.mark.parametrize("kind", ["swiglu", "gelu", "silu", "relu"])
+def test_activation_backward_rows_shared_by_warps(rows, F, kind):
+    from gpu_data_transfer_profile_b200.models.experts import activate
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    torch.manual_seed(12)
+    h = torch.randn(rows, F * (2 if kind == "swiglu" else 1), device="cuda").to(torch.bfloat16)
+    p = torch.rand(rows, device="cuda")
+    d = torch.randn(rows, F, device="cuda").to(torch.bfloat16)
+    hf, pf = h.double().requires_grad_(True), p.double().requires_grad_(True)
+    (activate(hf, kind) * pf[:, None]).backward(d.double())
+    dh, dp = G.swiglu_bwd(h, p, d) if kind == "swiglu" else G.act_bwd(h, p, d, kind)
+    torch.testing.assert_close(dh.double(), hf.grad, rtol=2.0 ** -8, atol=2e-6 * 64)
+    torch.testing.assert_close(dp.double(), pf.grad, rtol=1e-5, atol=4e-6 * F ** 0.5)
+
+
 def test_tcgen05_experts_backward_matches_torch_experts():
     from gpu_data_transfer_profile_b200.models.experts import TorchGroupedExperts
     from gpu_data_transfer_profile_b200.models.experts_tcgen05 import Tcgen05GroupedExperts
