@@ -91,6 +91,17 @@ struct CombinePullArgs {
 void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                          const CombinePullArgs& a, int dtype_code, int* status, int blocks, cudaStream_t st);
 
+// Copies n buffers (16-byte aligned, this GPU) in one launch. Returns 0 on success.
+constexpr int kMaxClones = 8;
+struct CloneArgs {
+  const char* src[kMaxClones];
+  char* dst[kMaxClones];
+  long long bytes[kMaxClones];
+  int first_chunk[kMaxClones + 1];   // filled by the launcher
+  int n;
+};
+int launch_clone(CloneArgs a, cudaStream_t st);
+
 void launch_signal(const PeerPtrs& peers, long long flags_off, int channel, int rank, int R,
                    int epoch, cudaStream_t st);
 

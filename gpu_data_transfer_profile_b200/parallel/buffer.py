@@ -580,22 +580,30 @@ class Buffer:
             self._poll_status()       # the host already waited for the kernel's prologue: cheap to look
         reg = dict(zip(("flags", "counts", "recv_x", "recv_scales", "recv_topk_idx", "recv_topk_w",
                         "recv_meta", "recv_prob", "comb_x", "comb_w"), st["regions"]))
-        keep = (lambda t: t) if zero_copy else (lambda t: t.clone())
+        # the views a caller gets; owned copies of all of them leave in one launch
+        views = []
         if st["fp8_out"]:
-            rx = self.region.view(reg["recv_x"], (n_recv, H), "float8_e4m3fn")
-            rs = self.region.view(reg["recv_scales"], (n_recv, H // 128), "float32")
-            recv_x = (keep(rx), keep(rs))
+            views.append(self.region.view(reg["recv_x"], (n_recv, H), "float8_e4m3fn"))
+            views.append(self.region.view(reg["recv_scales"], (n_recv, H // 128), "float32"))
         else:
-            recv_x = keep(self.region.view(reg["recv_x"], (n_recv, H), _ELEM_DTYPE[st["in_dtype"]]))
+            views.append(self.region.view(reg["recv_x"], (n_recv, H), _ELEM_DTYPE[st["in_dtype"]]))
+        n_x = len(views)
+        side = st["mode"] == 0 and st["topk_idx"] is not None
+        if not st["cached"]:
+            if side:
+                views.append(self.region.view(reg["recv_topk_idx"], (n_recv, K), "int64"))
+                views.append(self.region.view(reg["recv_topk_w"], (n_recv, K), "float32"))
+            if st["mode"] == 1:
+                views.append(self.region.view(reg["recv_prob"], (n_recv,), "float32"))
+            views.append(self.region.view(reg["recv_meta"], (n_recv, 2), "int32"))
+        if not zero_copy:
+            views = self.C.clone_views(views)
+        recv_x = tuple(views[:2]) if n_x == 2 else views[0]
         if st["cached"]:
             return recv_x, None, None, per_expert_list, st["handle"]
-        recv_topk_idx = recv_topk_w = recv_prob = None
-        if st["mode"] == 0 and st["topk_idx"] is not None:
-            recv_topk_idx = keep(self.region.view(reg["recv_topk_idx"], (n_recv, K), "int64"))
-            recv_topk_w = keep(self.region.view(reg["recv_topk_w"], (n_recv, K), "float32"))
-        if st["mode"] == 1:
-            recv_prob = keep(self.region.view(reg["recv_prob"], (n_recv,), "float32"))
-        recv_meta = keep(self.region.view(reg["recv_meta"], (n_recv, 2), "int32"))
+        recv_topk_idx, recv_topk_w = (views[n_x], views[n_x + 1]) if side else (None, None)
+        recv_prob = views[n_x] if st["mode"] == 1 else None
+        recv_meta = views[-1]
         handle = DispatchHandle(st["mode"], st["T"], H, K, E, n_recv, st["send_row"], st["send_slot"],
                                 st["meta"], recv_meta, st["topk_idx"], st.get("is_token_in_rank"),
                                 per_expert_list, st["fp8_out"], recv_prob, carve.key, carve.cap)

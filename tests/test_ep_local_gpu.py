@@ -537,3 +537,24 @@ def test_push_combine_reads_own_rows_in_place(R, T, H, E, K, dtype, grouped, wei
         g.check_canaries()
     finally:
         g.destroy()
+
+
+def test_clone_views_copies_every_byte_of_every_buffer():
+    """Sizes around a vector, a CTA's chunk and the grid; an empty buffer between others."""
+    from gpu_data_transfer_profile_b200 import _ext
+    C = _ext.load()
+    g = torch.Generator("cuda").manual_seed(1)
+    sizes = [1, 0, 15, 16, 17, 16384 - 1, 16384 + 33, 16384 * 148 * 8 + 16384 + 5]
+    src = [torch.randint(0, 256, (n,), generator=g, device="cuda", dtype=torch.uint8) for n in sizes]
+    for part in (src, src[:1], src[1:2], []):
+        out = C.clone_views(part)
+        assert len(out) == len(part)
+        for a, b in zip(out, part):
+            assert torch.equal(a, b) and (a.numel() == 0 or a.data_ptr() != b.data_ptr())
+    x = torch.randn(37, 5, 3, device="cuda").to(torch.float8_e4m3fn)
+    y = C.clone_views([x])[0]
+    assert y.dtype == x.dtype and y.shape == x.shape and torch.equal(y.view(torch.uint8), x.view(torch.uint8))
+    with pytest.raises(RuntimeError):
+        C.clone_views([src[4][1:]])                     # not 16-byte aligned
+    with pytest.raises(RuntimeError):
+        C.clone_views(src + src[:1])
