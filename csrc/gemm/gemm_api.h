@@ -87,4 +87,12 @@ int launch_act_fwd(const void* h, const float* p, void* act, const int* n_rows_p
 int launch_act_bwd(const void* h, const float* p, const void* dact, void* dh, float* dp, const int* n_rows_ptr,
                    int max_rows, int F, int kind, cudaStream_t st);
 
+// Router (csrc/gemm/router.cu). Parts of the reduction that launch_router_logits should use; part: f32 [splits, T, E].
+constexpr int kRouterMaxExperts = 1024;
+int router_splits(int T, int E, int H);
+// x: bf16 [T, H], w: f32 [E, H]; H % 8 == 0, 16-byte aligned.
+int launch_router_logits(const void* x, const float* w, float* part, int splits, int T, int E, int H, cudaStream_t st);
+// Softmax over the E logits (the sum of the parts), top-K (K <= 32, E <= kRouterMaxExperts), renormalised: idx int64, prob f32 [T, K].
+int launch_router_topk(const float* part, int splits, int T, int E, int K, long long* idx, float* prob, cudaStream_t st);
+
 }  // namespace b200ep

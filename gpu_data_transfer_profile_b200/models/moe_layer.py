@@ -11,6 +11,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from .. import _ext
 from .experts import build_experts
 from .token_dispatcher import B200TokenDispatcher
 
@@ -20,6 +21,15 @@ def topk_softmax_router(logits: torch.Tensor, topk: int) -> Tuple[torch.Tensor, 
     probs = torch.softmax(logits.float(), dim=-1)
     w, idx = torch.topk(probs, topk, dim=-1)
     return idx, w / w.sum(-1, keepdim=True)
+
+
+def _plain_linear(m: torch.nn.Module) -> bool:
+    """Calling `m` does nothing but x @ weight.T in f32: the fused router may stand in for it."""
+    return (type(m) is torch.nn.Linear and m.bias is None and type(m.weight) is torch.nn.Parameter
+            and m.weight.dtype == torch.float32 and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+            and not (torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks)
+            and not torch.is_autocast_enabled("cuda"))
 
 
 class MoELayer(torch.nn.Module):
@@ -43,11 +53,29 @@ class MoELayer(torch.nn.Module):
         self.dispatcher = B200TokenDispatcher(group, self.num_local_experts, num_experts,
                                               ep_rank * self.num_local_experts, mode=dispatcher_mode, world=world)
 
+    def _route(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor]):
+        """(expert ids, weights). Without gradients the router runs on this library's kernels (f32 like the
+        module's own product); with them it stays the differentiable torch form."""
+        E, K = self.num_experts, self.topk
+        C = _ext.load() if hidden_states.is_cuda and not torch.is_grad_enabled() else None
+        if C is None or E > C.ROUTER_MAX_EXPERTS or K > 32 or torch.compiler.is_compiling() or torch.jit.is_tracing():
+            if router_logits is None:
+                router_logits = self.router(hidden_states.float())
+            return topk_softmax_router(router_logits, K)
+        if router_logits is None:
+            x = hidden_states
+            if (type(x) is torch.Tensor and x.dtype == torch.bfloat16 and x.dim() == 2 and x.is_contiguous()
+                    and x.data_ptr() % 16 == 0 and x.shape[1] % 8 == 0 and x.device == self.router.weight.device
+                    and _plain_linear(self.router) and self.router.weight.shape == (E, x.shape[1])):
+                return C.route(x, self.router.weight, K)
+            router_logits = self.router(x.float())
+        if type(router_logits) is not torch.Tensor or router_logits.dim() != 2 or router_logits.shape[1] > C.ROUTER_MAX_EXPERTS:
+            return topk_softmax_router(router_logits, K)
+        return C.topk_softmax(router_logits.float().contiguous(), K)
+
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
         """hidden_states [T,H]; router_logits [T,E] override the learnable router when given."""
-        if router_logits is None:
-            router_logits = self.router(hidden_states.float())
-        idx, probs = topk_softmax_router(router_logits, self.topk)
+        idx, probs = self._route(hidden_states, router_logits)
         if self.use_fp8 and not torch.is_grad_enabled() and self.dispatcher.mode == "fused":
             rows, tokens_per_expert, row_probs = self.dispatcher.dispatch_fp8(hidden_states, idx, probs)
             El = self.num_local_experts

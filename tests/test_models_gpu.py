@@ -134,3 +134,52 @@ def test_moe_layer_fp8_inference_path_close_to_bf16():
         torch.testing.assert_close(out8.float(), out16.float(), atol=0.06 * scale, rtol=0.1)
     finally:
         A.release_buffers()
+
+
+@pytest.mark.parametrize("T,E,H,K", [(1, 3, 8, 1), (7, 8, 264, 2), (64, 64, 2048, 8), (65, 33, 1000, 4), (130, 160, 7168, 6),
+                                     (300, 256, 512, 8), (66, 1024, 128, 32), (40, 300, 72, 3)])
+def test_router_kernels_against_64_bits(T, E, H, K):
+    """Expert ids and weights from bf16 rows and f32 router weights. The logits are f32 sums of H products: their
+    error against 64 bits stays within a few ulp times sqrt(H), the ids differ only where two logits are closer."""
+    from gpu_data_transfer_profile_b200 import _ext
+    C = _ext.load()
+    torch.manual_seed(5)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    w = torch.randn(E, H, device="cuda") * 0.02
+    idx, prob = C.route(x, w, K)
+    logits = x.double() @ w.double().t()
+    top, ref = torch.topk(torch.softmax(logits, -1), K, dim=-1)
+    eps = 1e-6 * (1 + float(logits.abs().max()))
+    picked = logits.gather(1, idx)
+    assert bool((picked - logits.gather(1, ref)).abs().max() <= eps)            # as good a choice, rank by rank
+    assert all(len(set(r)) == K for r in idx.tolist())
+    want = torch.softmax(logits, -1).gather(1, idx)
+    torch.testing.assert_close(prob.double(), want / want.sum(-1, keepdim=True), rtol=1e-5, atol=1e-7)
+    idx2, prob2 = C.topk_softmax(logits.float().contiguous(), K)
+    assert bool((logits.gather(1, idx2) - logits.gather(1, ref)).abs().max() <= eps)
+    torch.testing.assert_close(prob2.double().sum(-1), torch.ones(T, dtype=torch.float64, device="cuda"), rtol=1e-5, atol=0)
+
+
+def test_router_topk_of_masked_infinite_and_nan_logits():
+    """Masked experts (-inf, the type's lowest value) are chosen last and weigh nothing; equal logits give distinct
+    experts; a row that softmax turns into NaN still names distinct experts in range."""
+    from gpu_data_transfer_profile_b200 import _ext
+    C = _ext.load()
+    E, K, inf = 40, 4, float("inf")
+    rows = torch.zeros(7, E)
+    rows[0, :] = -inf
+    rows[0, [7, 39]] = torch.tensor([1.0, 2.0])                       # two finite, two masked choices
+    rows[1, :] = torch.finfo(torch.float32).min
+    rows[1, 33] = 0.5
+    rows[2, :] = -inf                                                  # nothing but masked: NaN weights
+    rows[3, 5] = float("nan")
+    rows[4, 6] = inf
+    rows[5, 1] = -0.0                                                  # all equal
+    rows[6] = torch.linspace(-3, 3, E)
+    idx, prob = (t.cpu() for t in C.topk_softmax(rows.cuda(), K))
+    assert bool(((idx >= 0) & (idx < E)).all()) and all(len(set(r)) == K for r in idx.tolist())
+    assert idx[0, :2].tolist() == [39, 7] and prob[0, 2:].tolist() == [0.0, 0.0]
+    torch.testing.assert_close(prob[0, :2], torch.softmax(torch.tensor([2.0, 1.0]), 0))
+    assert idx[1, 0] == 33 and prob[1].tolist() == [1.0, 0.0, 0.0, 0.0]
+    assert bool(prob[2].isnan().all()) and bool(prob[3].isnan().all()) and bool(prob[4].isnan().all())
+    assert prob[5].tolist() == [0.25] * 4 and idx[6].tolist() == [39, 38, 37, 36]
