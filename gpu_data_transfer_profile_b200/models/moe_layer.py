@@ -76,11 +76,19 @@ class MoELayer(torch.nn.Module):
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
         """hidden_states [T,H]; router_logits [T,E] override the learnable router when given."""
         idx, probs = self._route(hidden_states, router_logits)
-        if self.use_fp8 and not torch.is_grad_enabled() and self.dispatcher.mode == "fused":
-            rows, tokens_per_expert, row_probs = self.dispatcher.dispatch_fp8(hidden_states, idx, probs)
-            El = self.num_local_experts
-            off = self.dispatcher.handle.meta[2 + El: 2 + El + El + 1]
-            return self.dispatcher.combine(self.experts.forward_fp8(rows, tokens_per_expert, row_probs, expert_off=off))
+        if (not torch.is_grad_enabled() and self.dispatcher.mode == "fused" and hidden_states.dtype == torch.bfloat16
+                and hasattr(self.experts, "forward_fused_combine") and (self.use_fp8 or self.fuse_combine)):
+            # Inference: the rows are consumed where they arrive, before the next dispatch can be issued on this
+            # stream, so they need no copy of their own, and the GEMMs take their tile lists from the device.
+            rows, row_probs, handle = self.dispatcher.dispatch_in_place(hidden_states, idx, probs, use_fp8=self.use_fp8)
+            if self.use_fp8:
+                El = self.num_local_experts
+                off = handle.meta[2 + El: 2 + El + El + 1]
+                return self.dispatcher.combine(self.experts.forward_fp8(rows, (), row_probs, expert_off=off))
+            from . import fused_a2a as A
+            buf = A.get_buffer(self.dispatcher.group, A.get_hidden_bytes(hidden_states), self.dispatcher.world)
+            self.dispatcher.handle = None
+            return self.experts.forward_fused_combine(rows, row_probs, buf, handle)
         rows, tokens_per_expert, row_probs = self.dispatcher.dispatch(hidden_states, idx, probs)
         if (self.fuse_combine and self.dispatcher.mode == "fused" and hasattr(self.experts, "forward_fused_combine")
                 and (not torch.is_grad_enabled() or self.experts.activation == "swiglu")):

@@ -38,9 +38,22 @@ class B200TokenDispatcher:
         self.mode = mode
         self.handle = None
         self.dispatched_probs: Optional[torch.Tensor] = None
-        self.tokens_per_expert: Optional[torch.Tensor] = None
+        self._tokens_per_expert: Optional[torch.Tensor] = None
         self._n_before_permute: Optional[int] = None
         self._reverse_map: Optional[torch.Tensor] = None
+
+    @property
+    def tokens_per_expert(self) -> Optional[torch.Tensor]:
+        """Rows of each local expert of the last dispatch (int64, CPU). After `dispatch_in_place` they are
+        still on the device and are read when somebody asks."""
+        t = self._tokens_per_expert
+        if t is not None and t.is_cuda:
+            t = self._tokens_per_expert = t.to("cpu", torch.int64)
+        return t
+
+    @tokens_per_expert.setter
+    def tokens_per_expert(self, value: Optional[torch.Tensor]) -> None:
+        self._tokens_per_expert = value
 
     # ---- reference-style local glue (mode="deepep") -----------------------------------
     def _indices_to_multihot(self, indices: torch.Tensor, probs: torch.Tensor,
@@ -103,6 +116,33 @@ class B200TokenDispatcher:
             raise RuntimeError(f"tokens_per_expert has length {tpe.numel()}, expected {self.num_local_experts}")
         self.handle, self.tokens_per_expert, self.dispatched_probs = handle, tpe, row_probs
         return rows, tpe, row_probs
+
+    @torch.no_grad()
+    def dispatch_in_place(self, hidden_states, token_indices, token_probs, use_fp8: bool = False):
+        """Forward-only, fused mode, for a caller that consumes the rows at once on the current stream: they (and
+        nothing else) stay views of the receive region, valid until the second next dispatch. Returns (rows, or
+        (e4m3 rows, scales) with use_fp8, one probability per row, handle).
+        A group of one receives exactly its own items, so the host need not wait for the receive count;
+        every index must then name an expert (no -1)."""
+        if self.mode != "fused":
+            raise ValueError("dispatch_in_place is offered by the fused (expert-grouped) dispatcher")
+        x = hidden_states.contiguous()
+        buf = A.get_buffer(self.group, A.get_hidden_bytes(x), self.world)
+        idx = token_indices.contiguous()
+        worst = 0
+        if buf.group_size == 1:
+            H, K = x.shape[1], idx.shape[1]
+            items = idx.numel()
+            # (a region too small for them takes the counted path, which names the overflow)
+            worst = items if 0 < items <= buf._get_carve(self.num_experts, K, H, H * 2, H * 2).cap else 0
+        rows, _, _, _, handle, _ = buf.dispatch(
+            x, topk_idx=idx, topk_weights=token_probs.contiguous().float(), group_by_expert=True,
+            num_experts=self.num_experts, use_fp8=use_fp8, zero_copy=True, num_worst_tokens=worst)
+        El = self.num_local_experts
+        # (what callers may look at later is their own; the rows' view above is for the computation)
+        self.handle, self.dispatched_probs = handle, buf.C.clone_views([handle.recv_prob])[0]
+        self.tokens_per_expert = handle.meta[2:2 + El]
+        return rows, handle.recv_prob, handle
 
     @torch.no_grad()
     def dispatch_fp8(self, hidden_states, token_indices, token_probs):

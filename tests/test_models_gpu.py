@@ -183,3 +183,44 @@ def test_router_topk_of_masked_infinite_and_nan_logits():
     assert idx[1, 0] == 33 and prob[1].tolist() == [1.0, 0.0, 0.0, 0.0]
     assert bool(prob[2].isnan().all()) and bool(prob[3].isnan().all()) and bool(prob[4].isnan().all())
     assert prob[5].tolist() == [0.25] * 4 and idx[6].tolist() == [39, 38, 37, 36]
+
+
+@pytest.mark.parametrize("use_fp8,fuse", [(False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("activation", ["swiglu", "silu"])
+def test_moe_layer_inference_consumes_rows_in_place(use_fp8, fuse, activation):
+    """Two layers of different sizes on one shared buffer, called in turn: the inference path (own router, rows read
+    where they arrive, no host read of the counts) gives what the general path gives, and the dispatcher's record of
+    the last dispatch is the caller's own."""
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A
+    from gpu_data_transfer_profile_b200.models.moe_layer import MoELayer, topk_softmax_router
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    torch.manual_seed(0)
+    world = LocalWorld.make(1)[0]
+    A.configure_buffer(num_max_tokens_per_rank=512, num_topk=4, num_experts=8, group_by_expert=True)
+    try:
+        layers = [MoELayer(512, 256, 8, 4, None, activation=activation, expert_backend="tcgen05", world=world,
+                           use_fp8=use_fp8, fuse_combine=fuse) for _ in range(2)]
+        x = torch.randn(301, 512, device="cuda").to(torch.bfloat16)
+        with torch.no_grad():
+            a = layers[0](x)
+            counts, probs = layers[0].dispatcher.tokens_per_expert, layers[0].dispatcher.dispatched_probs
+            kept = None if probs is None else probs.clone()
+            for _ in range(3):                                       # more dispatches than the region has parities
+                b = layers[1](a)
+            for layer, inp, got in ((layers[0], x, a), (layers[1], a, b)):
+                idx, w = topk_softmax_router(layer.router(inp.float()), 4)
+                if use_fp8:
+                    rows, tpe, rp = layer.dispatcher.dispatch_fp8(inp, idx, w)
+                    y = layer.experts.forward_fp8(rows, tpe, rp)
+                else:
+                    rows, tpe, rp = layer.dispatcher.dispatch(inp, idx, w)
+                    y = layer.experts(rows, tpe, rp)
+                want = layer.dispatcher.combine(y)
+                # weights differ by f32 rounding of the softmax, rows by one bf16 rounding of it
+                torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -6, atol=2.0 ** -8 * float(want.abs().max()))
+        if not use_fp8:
+            assert counts.device.type == "cpu" and int(counts.sum()) == 301 * 4
+            assert torch.equal(probs, kept)
+        A._BUFFERS[(id(None), id(world))].check_status()
+    finally:
+        A.release_buffers()
