@@ -104,26 +104,6 @@ PeerPtrs make_peers(const std::vector<int64_t>& bases) {
   for (size_t i = 0; i < bases.size(); ++i) p.base[i] = ptr<char>(bases[i]);
   return p;
 }
-EpGeom make_geom(const std::vector<int64_t>& v) {
-  TORCH_CHECK(v.size() == 16, "geom needs 16 entries");
-  EpGeom g{};
-  g.rank = (int)v[0]; g.R = (int)v[1]; g.E = (int)v[2]; g.El = (int)v[3]; g.K = (int)v[4];
-  g.T = (int)v[5]; g.mode = (int)v[6]; g.J = (int)v[7]; g.B = (int)v[8]; g.H = (int)v[9];
-  g.cap = (int)v[10]; g.slot_cap = (int)v[11]; g.epoch = (int)v[12]; g.epoch_wait = (int)v[13];
-  g.tail_wait = (int)v[14];
-  g.timeout_ns = (unsigned long long)v[15];
-  TORCH_CHECK(g.R >= 1 && g.R <= kMaxRanks && g.J <= kMaxItemsPerToken && g.K <= kMaxItemsPerToken,
-              "geometry out of range");
-  return g;
-}
-EpRegions make_regions(const std::vector<int64_t>& v) {
-  TORCH_CHECK(v.size() == 11, "regions needs 11 entries");
-  EpRegions r{};
-  r.flags = v[0]; r.counts = v[1]; r.recv_x = v[2]; r.recv_scales = v[3]; r.recv_topk_idx = v[4];
-  r.recv_topk_w = v[5]; r.recv_meta = v[6]; r.recv_prob = v[7]; r.comb_x = v[8]; r.comb_w = v[9];
-  r.pull_info = v[10];
-  return r;
-}
 // meta tensor layout: [n_recv, send_total, expert_cnt[El], expert_off[El+1], src_off[R+1],
 //                      send_base[B], comb_base[B]]
 int64_t meta_ints(const EpGeom& g) {

@@ -129,18 +129,6 @@ class _Carve:
             self.regions.append(d)
         assert off <= nbytes or self.cap == 0
         self.bytes_used = off
-        self._lists = {}
-
-    def region_list(self, notify_parity: int, dispatch_parity: int, combine_parity: int):
-        key = (notify_parity, dispatch_parity, combine_parity)
-        out = self._lists.get(key)
-        if out is None:
-            d, c = self.regions[dispatch_parity], self.regions[combine_parity]
-            out = [self.flags, self.counts[notify_parity], d["recv_x"], d["recv_scales"],
-                   d["recv_topk_idx"], d["recv_topk_w"], d["recv_meta"], d["recv_prob"],
-                   c["comb_x"], c["comb_w"], self.pull_info]
-            self._lists[key] = out
-        return out
 
 
 GUARD_BYTES = 256              # canary band after every receive / combine region
@@ -227,15 +215,15 @@ class Buffer:
             self.status = torch.zeros(4, dtype=torch.int32, device=self.device)
             self.status.view(torch.int64)[1] = self.host_word + 4 * _STATUS_MIRROR_SLOT
             self.counters = torch.zeros(8, dtype=torch.int32, device=self.device)
-            self._ctr = [self.counters[i:i + 1] for i in range(8)]     # views made once, not per call
+            self._fc2_ctr = self.counters[3:4]
             self._side_stream = (torch.cuda.current_stream() if self.world.local
                                  else torch.cuda.Stream(device=self.device))
             self.comm_stream = None
         self._async_outstanding = False
         # One launch may both send and wait for peers only when no other rank shares this GPU.
         self._single_launch = (not self.world.local) or self.group_size == 1
-        self._ws = {}
-        self._layout_ws = None
+        # native half of the normal-mode calls: peers, counters, region layout, scratch
+        self._ctx = self.C.EpContext(self.rank, self.group_size, self.status.data_ptr(), self.host_word, self.counters)
         self._epoch = dict(notify=0, dispatch=0, combine=0, barrier=0, ll_dispatch=0, ll_combine=0)
         self._carve: Optional[_Carve] = None
         self._ll = None
@@ -308,8 +296,12 @@ class Buffer:
                                  self.num_max_recv_tokens, self.combine_slots)
             # paint the guard bands of MY region; peers store into it only after they have seen
             # this rank's next count vector, which is stream-ordered after these fills
-            for _, _, off, n in self._carve.guards:
+            c = self._carve
+            for _, _, off, n in c.guards:
                 self.region.view(off, (n,), "uint8").fill_(CANARY)
+            names = ("recv_x", "recv_scales", "recv_topk_idx", "recv_topk_w", "recv_meta", "recv_prob", "comb_x", "comb_w")
+            self._ctx.set_carve(self.peers, self.num_nvl_bytes, E, K, H, c.cap, c.slot_cap, c.flags, list(c.counts),
+                                [c.regions[0][k] for k in names], [c.regions[1][k] for k in names], c.pull_info)
         return self._carve
 
     def check_canaries(self) -> None:
@@ -326,18 +318,6 @@ class Buffer:
                 bad.append(f"{name}[parity {parity}] at byte {off}")
         if bad:
             raise EpStatusError("guard band overwritten behind " + ", ".join(bad))
-
-    def _geom(self, *, E, K, T, mode, H, cap, slot_cap, epoch, epoch_wait=0, tail_wait=0) -> List[int]:
-        R = self.group_size
-        J, B = (R, R) if mode == 0 else (K, E)
-        return [self.rank, R, E, E // R, K, T, mode, J, B, H, cap, slot_cap, epoch, epoch_wait, tail_wait,
-                self._timeout_ns()]
-
-    def _meta_ints(self, E: int, mode: int, K: int) -> int:
-        R = self.group_size
-        El = E // R
-        B = R if mode == 0 else E
-        return 2 + El + (El + 1) + (R + 1) + 2 * B
 
     def _enter(self, previous_event, allocate_on_comm_stream, async_finish):
         """Pick the stream for this op. Synchronous calls run on the caller's stream: no stream
@@ -418,15 +398,7 @@ class Buffer:
         topk_idx = topk_idx.contiguous()
         compute = self._enter(previous_event, allocate_on_comm_stream, async_finish)
         with self._on_stream():
-            T = topk_idx.shape[0]
-            need = self.C.layout_scratch_ints(T, num_experts, R)
-            if self._layout_ws is None or self._layout_ws.numel() < need:
-                self._layout_ws = torch.empty(need, dtype=torch.int32, device=self.device)
-            counts = torch.empty(R + num_experts, dtype=torch.int32, device=self.device)
-            per_rank, per_expert = counts[:R], counts[R:]
-            in_rank = torch.empty((T, R), dtype=torch.bool, device=self.device)
-            self.C.layout(topk_idx, num_experts, R, per_rank, per_expert, in_rank, self._layout_ws,
-                          self._ctr[4], self.status_ptr)
+            per_rank, per_expert, in_rank = self._ctx.layout(topk_idx, num_experts)
         ev = self._exit(compute, async_finish, (per_rank, per_expert, in_rank, topk_idx))
         return per_rank, None, per_expert, in_rank, ev
 
@@ -498,53 +470,22 @@ class Buffer:
             return st
         self._epoch["notify"] += 1
         st["epoch_n"] = self._epoch["notify"]
-        dev = self.device
-        C_chunks = max((T + self.C.CHUNK_TOKENS - 1) // self.C.CHUNK_TOKENS, 1)
-        key = (max(T, 1), J, C_chunks, B)
-        ws = self._ws.get(key)
-        if ws is None:      # scratch reused by every call of this shape (stream-ordered)
-            ws = (torch.empty((max(T, 1), J), dtype=torch.int32, device=dev),
-                  torch.empty((C_chunks, B), dtype=torch.int32, device=dev))
-            self._ws = {key: ws}
-        st["item_rank"], st["chunk_hist"] = ws
-        n_meta = self._meta_ints(E, mode, K)
-        n_tj = max(T, 1) * J
-        owned = torch.empty(n_meta + 2 * n_tj, dtype=torch.int32, device=dev)   # handle-owned ints
-        st["meta"] = owned[:n_meta]
-        st["send_row"] = owned[n_meta:n_meta + n_tj].view(max(T, 1), J)
-        st["send_slot"] = owned[n_meta + n_tj:].view(max(T, 1), J)
-        regions = carve.region_list(st["epoch_n"] & 1, 0, 0)
-        geom = self._geom(E=E, K=K, T=T, mode=mode, H=H, cap=carve.cap, slot_cap=carve.slot_cap,
-                          epoch=st["epoch_n"])
         per_expert = st.get("num_tokens_per_expert")
         if per_expert is not None and per_expert.dtype != torch.int32:
             per_expert = per_expert.to(torch.int32)
-        self.C.notify_send(geom, regions, self.peers,
-                           st.get("is_token_in_rank") if mode == 0 else None,
-                           st["topk_idx"] if mode == 1 else None,
-                           per_expert if mode == 0 else None,
-                           st["item_rank"], st["chunk_hist"], self._ctr[0], self.status_ptr)
+        st["meta"], st["send_row"], st["send_slot"] = self._ctx.notify(
+            mode, T, st["epoch_n"], self._timeout_ns(), st.get("is_token_in_rank"), st["topk_idx"], per_expert)
         return st
 
     def _dispatch_p2(self, st):
         """The send kernel. One process per GPU: its last CTA also waits for the peers, so the
         receive region is complete when the kernel ends. Virtual ranks on one GPU: the wait is a
         separate launch (`_dispatch_p3`) issued after every rank's send."""
-        carve = st["carve"]
         self._epoch["dispatch"] += 1
         st["epoch_d"] = self._epoch["dispatch"]
-        pn = (st.get("epoch_n", 0)) & 1
-        regions = carve.region_list(pn, st["epoch_d"] & 1, 0)
-        st["regions"] = regions
-        geom = self._geom(E=st["E"], K=st["K"], T=st["T"], mode=st["mode"], H=st["H"], cap=carve.cap,
-                          slot_cap=carve.slot_cap, epoch=st["epoch_d"], epoch_wait=st.get("epoch_n", 0),
-                          tail_wait=1 if self._single_launch else 0)
-        st["geom"] = geom
-        self.C.dispatch_send(geom, regions, self.peers, st["meta"], st["x"], st["fp8"], st["cached"],
-                             st["topk_idx"], st.get("topk_weights"), st.get("item_rank"),
-                             st.get("chunk_hist"), st["send_row"], st["send_slot"],
-                             self._ctr[1], self.host_word, self.status_ptr, self._blocks(),
-                             st.get("scales_in"))
+        self._ctx.send(st["mode"], st["epoch_d"], st.get("epoch_n", 0), self._single_launch, self._timeout_ns(), self._blocks(),
+                       st["meta"], st["x"], st["fp8"], st["cached"], st["topk_idx"], st.get("topk_weights"), st["send_row"],
+                       st["send_slot"], st["scales_in"])
 
     def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1):
         R, E, K, H = self.group_size, st["E"], st["K"], st["H"]
@@ -563,9 +504,9 @@ class Buffer:
                 raise ValueError(f"num_worst_tokens={num_worst_tokens} exceeds the buffer capacity {carve.cap}")
             n_recv, per_expert_list = int(num_worst_tokens), []
         else:
-            if not self.C.host_wait_ge(self.host_word, 0, st["epoch_n"], self.timeout_s + 5.0):
+            found, n_recv, per_expert_list = self._ctx.wait_counts(st["epoch_n"], self.timeout_s + 5.0, El)
+            if not found:
                 raise EpTimeoutError("host timed out waiting for the receive count")
-            n_recv = self.C.host_read_i32(self.host_word, 1)
             if n_recv < 0:
                 torch.cuda.synchronize(self.device)
                 self._clear_status()
@@ -574,12 +515,10 @@ class Buffer:
                 torch.cuda.synchronize(self.device)
                 self._clear_status()
                 raise EpStatusError(f"receive region overflow: {n_recv} rows > capacity {carve.cap}")
-            per_expert_list = self.C.host_read_i32_list(self.host_word, 2, El)
             if expert_alignment > 1:
                 per_expert_list = [align_up(c, expert_alignment) for c in per_expert_list]
             self._poll_status()       # the host already waited for the kernel's prologue: cheap to look
-        reg = dict(zip(("flags", "counts", "recv_x", "recv_scales", "recv_topk_idx", "recv_topk_w",
-                        "recv_meta", "recv_prob", "comb_x", "comb_w"), st["regions"]))
+        reg = carve.regions[st["epoch_d"] & 1]
         # the views a caller gets; owned copies of all of them leave in one launch
         views = []
         if st["fp8_out"]:
@@ -638,6 +577,8 @@ class Buffer:
                                    topk_weights, use_fp8, group_by_expert, num_experts)
             self._dispatch_p2(st)
             out = self._dispatch_p3(st, zero_copy, num_worst_tokens, expert_alignment)
+        if compute is None and not async_finish:
+            return (*out, None)
         flat = []
         for o in out[:3]:
             flat.extend(o if isinstance(o, tuple) else (o,))
@@ -661,73 +602,50 @@ class Buffer:
             raise ValueError("combine dtype is wider than the region reserved at dispatch")
         self._epoch["combine"] += 1
         ep = self._epoch["combine"]
-        regions = carve.region_list(0, 0, ep & 1)
-        geom = self._geom(E=handle.E, K=handle.K, T=handle.T, mode=handle.mode, H=handle.H,
-                          cap=handle.n_recv, slot_cap=carve.slot_cap, epoch=ep)
         if topk_weights is not None:
             topk_weights = topk_weights.to(torch.float32).contiguous()
-        return dict(ep=ep, regions=regions, geom=geom, dtype=x.dtype, topk_w=topk_weights, x=x)
+        return dict(ep=ep, dtype=x.dtype, topk_w=topk_weights, x=x)
 
-    def _combine_outputs(self, st, handle: DispatchHandle):
-        out = torch.empty((handle.T, handle.H), dtype=st["dtype"], device=self.device)
-        out_w = (torch.empty((handle.T, handle.K), dtype=torch.float32, device=self.device)
-                 if st.get("topk_w") is not None else None)
-        return out, out_w
+    def _combine_push(self, role: int, st, handle: DispatchHandle, in_place: bool, weights=None):
+        """role 0: send + wait + reduce in one launch, 1: send, 2: wait + reduce. in_place: rows of this rank's
+        own tokens are read where they lie (both roles must agree)."""
+        x, w = (st["x"], st["topk_w"]) if in_place or role != 2 else (None, None)
+        return self._ctx.combine_push(
+            role, handle.mode, handle.T, handle.n_recv, st["ep"], self._timeout_ns(), max(1, Buffer.num_sms),
+            handle.n_recv_dev if x is not None else None, handle.recv_meta if x is not None else None, x, w,
+            handle.send_slot, weights, handle.send_row if in_place else None, handle.topk_idx if in_place else None,
+            _ELEM_DTYPE[st["dtype"]], st["topk_w"] is not None)
 
     def _combine_p1(self, x, handle: DispatchHandle, topk_weights):
         """Push form, send half as its own launch (several virtual ranks on one GPU)."""
         st = self._combine_prepare(x, handle, topk_weights)
         st["in_place"] = True
-        self.C.combine(st["geom"], st["regions"], self.peers, 1, max(1, Buffer.num_sms), False,
-                       handle.n_recv_dev, handle.recv_meta, x, st["topk_w"], self._ctr[2],
-                       None, None, None, None, self.status_ptr, handle.send_row, handle.topk_idx)
+        self._combine_push(1, st, handle, True)
         return st
 
     def _combine_p2(self, st, handle: DispatchHandle, weights=None):
         """Push form, reduce half as its own launch (waits for every rank's combine flag first)."""
-        out, out_w = self._combine_outputs(st, handle)
         # rows of this rank's own tokens are still where `_combine_p1` found them; the fused fc2 has put
         # every row into its slot
-        here = st.get("in_place", False)
-        self.C.combine(st["geom"], st["regions"], self.peers, 2, max(1, Buffer.num_sms), True,
-                       handle.n_recv_dev if here else None, handle.recv_meta if here else None,
-                       st["x"] if here else None, st["topk_w"] if here else None, self._ctr[2],
-                       handle.send_slot, weights, out, out_w, self.status_ptr,
-                       handle.send_row if here else None, handle.topk_idx if here else None)
-        return out, out_w
+        return self._combine_push(2, st, handle, st.get("in_place", False), weights)
 
     def _combine_fused(self, x, handle: DispatchHandle, topk_weights, weights=None):
         """Push form in ONE launch: every CTA sends its share of the rows, then waits for the peers'
         flags and reduces its share of the tokens (this rank's own rows are reduced where they lie)."""
         st = self._combine_prepare(x, handle, topk_weights)
-        out, out_w = self._combine_outputs(st, handle)
-        self.C.combine(st["geom"], st["regions"], self.peers, 0, max(1, Buffer.num_sms), True,
-                       handle.n_recv_dev, handle.recv_meta, x, st["topk_w"], self._ctr[2],
-                       handle.send_slot, weights, out, out_w, self.status_ptr, handle.send_row, handle.topk_idx)
-        return out, out_w
-
-    def _region_offset(self, t: Optional[torch.Tensor]) -> int:
-        """Byte offset of tensor `t` inside this rank's symmetric region, or -1 if it lies elsewhere."""
-        if t is None or not t.is_cuda or not t.is_contiguous():
-            return -1
-        lo = self.region.local_ptr
-        p = t.data_ptr()
-        if p < lo or p + t.numel() * t.element_size() > lo + self.num_nvl_bytes:
-            return -1
-        return p - lo
+        return self._combine_push(0, st, handle, True, weights)
 
     def _use_pull(self, x, topk_weights) -> bool:
         mode = Buffer.combine_transport
         if mode == "push":
             return False
-        ok = self._region_offset(x) >= 0 and x.data_ptr() % 16 == 0 and (
-            topk_weights is None or (topk_weights.dtype == torch.float32 and self._region_offset(topk_weights) >= 0))
+        ok = self._ctx.can_pull(x, topk_weights)
         if (mode == "pull" or not self.combine_slots) and not ok:
             raise ValueError("this combine can only pull (combine_transport='pull' or a buffer without combine "
                              "slots): x (and topk_weights) must lie inside the symmetric region")
         return ok
 
-    def _combine_pull(self, phase: int, x, handle: DispatchHandle, topk_weights, weights=None, out=None):
+    def _combine_pull(self, phase: int, x, handle: DispatchHandle, topk_weights, weights=None):
         """phase 0: announce + wait + reduce in one launch; 1: announce only; 2: wait + reduce."""
         carve = self._carve
         if carve is None or carve.key[:3] != (handle.E, handle.K, handle.H):
@@ -736,19 +654,8 @@ class Buffer:
             raise ValueError("x must be a [num_recv_tokens, hidden] bf16/fp16/fp32 tensor")
         if phase != 2:
             self._epoch["combine"] += 1
-        ep = self._epoch["combine"]
-        regions = carve.region_list(0, 0, ep & 1)
-        geom = self._geom(E=handle.E, K=handle.K, T=handle.T, mode=handle.mode, H=handle.H,
-                          cap=carve.cap, slot_cap=carve.slot_cap, epoch=ep)
-        if out is None:
-            out = torch.empty((handle.T, handle.H), dtype=x.dtype, device=self.device)
-        out_w = (torch.empty((handle.T, handle.K), dtype=torch.float32, device=self.device)
-                 if topk_weights is not None else None)
-        self.C.combine_pull(geom, regions, self.peers, phase, max(1, Buffer.num_sms),
-                            self._region_offset(x), self._region_offset(topk_weights), int(x.shape[0]),
-                            handle.send_row, handle.topk_idx if handle.mode == 1 else None, weights, out, out_w,
-                            self.status_ptr)
-        return out, out_w
+        return self._ctx.combine_pull(phase, handle.mode, handle.T, self._epoch["combine"], self._timeout_ns(), max(1, Buffer.num_sms),
+                                      x, topk_weights, handle.send_row, handle.topk_idx, weights)
 
     def combine_input(self, num_rows: int, hidden: int, dtype=torch.bfloat16) -> torch.Tensor:
         """A [num_rows, hidden] tensor INSIDE the symmetric region for the expert computation to
@@ -794,6 +701,8 @@ class Buffer:
                 out, out_w = self._combine_p2(st, handle, item_weights)
             if bias is not None:
                 out = out + (bias[0] if isinstance(bias, (tuple, list)) else bias)
+        if compute is None and not async_finish:
+            return out, out_w, None
         ev = self._exit(compute, async_finish, [out, x] + ([out_w] if out_w is not None else []))
         return out, out_w, ev
 
@@ -1074,16 +983,13 @@ def _fused_fc2_send(self: Buffer, act: torch.Tensor, w2: torch.Tensor, handle: D
         raise ValueError("w2 must be [E_local, hidden, ffn] and act bf16")
     self._epoch["combine"] += 1
     ep = self._epoch["combine"]
-    regions = carve.region_list(0, 0, ep & 1)
     El = handle.E // self.group_size
     expert_off = handle.meta[2 + El: 2 + El + El + 1]
     flag_row = self.C.MAX_RANKS * 4 * 2          # byte offset of the combine channel's flag row
-    G.grouped_gemm_combine(act, w2, expert_off, handle.recv_meta, self.peers, regions[8], carve.slot_cap,
-                           self.rank, signal_flag_off=flag_row, epoch=ep, counter=self._ctr[3],
+    G.grouped_gemm_combine(act, w2, expert_off, handle.recv_meta, self.peers, carve.regions[ep & 1]["comb_x"], carve.slot_cap,
+                           self.rank, signal_flag_off=flag_row, epoch=ep, counter=self._fc2_ctr,
                            status_ptr=self.status_ptr)
-    geom = self._geom(E=handle.E, K=handle.K, T=handle.T, mode=1, H=handle.H, cap=handle.n_recv,
-                      slot_cap=carve.slot_cap, epoch=ep)
-    return dict(ep=ep, regions=regions, geom=geom, dtype=torch.bfloat16, topk_w=None)
+    return dict(ep=ep, dtype=torch.bfloat16, topk_w=None)
 
 
 def _fused_fc2_combine(self: Buffer, act: torch.Tensor, w2: torch.Tensor, handle: DispatchHandle,
