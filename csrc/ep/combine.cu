@@ -22,8 +22,9 @@
 // Bound: memory (or NVLink) bandwidth; every reduction asks for the indices of a warp's next item
 // before it loads the rows of the current one, and few tokens are cut into more parts per row on
 // smaller CTAs. Measured on one B200, before and after: push of 2047 tokens x 8 rows of 14 KiB
-// 133 -> 57 us (the slot round trip is gone), push of 96 rows of 2 KiB 14.7 -> 3.7 us, pull of 4096
-// rows of 14 KiB 27.3 -> 22.8 us. One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
+// 133 -> 57 us (the slot round trip is gone) -> 49 us (rows not allocated in L1; 5.4 TB/s), push of 96
+// rows of 2 KiB 14.7 -> 3.7 us, pull of 4096 rows of 14 KiB 27.3 -> 22.8 -> 21.7 us. Tried and slower: half the
+// warps with one or two steps of loads requested ahead (58 us for the first). One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
 // peers are launched after the halves they wait for (all announcements / sends first).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -203,7 +204,7 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
 #pragma unroll
         for (int u = 0; u < kRUnroll; ++u) {
           const int v = v0 + u * 32;
-          if (v < v_end) val[u] = ld_global_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU may have written it
+          if (v < v_end) val[u] = ld_global_once_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU may have written it
         }
 #pragma unroll
         for (int u = 0; u < kRUnroll; ++u)
