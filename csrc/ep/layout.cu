@@ -139,20 +139,19 @@ void launch_layout(const long long* topk_idx, int T, int K, int E, int R, int* p
 //   rank mode   : for every destination rank one ballot over the chunk's tokens;
 //   expert mode : a 32-bit mask per expert in shared memory (bit = token of the chunk that
 //                 chose the expert); an item's rank is the number of lower bits.
-// The last CTA to finish scans the histograms over chunks (turning them into chunk bases),
-// builds this rank's count vector [R rank counts | E expert counts], stores it into every
-// peer's count matrix and releases the notify flag.
+// The histograms are scanned over chunks (they become chunk bases); the totals give this rank's
+// count vector [R rank counts | E expert counts], which one CTA stores into every peer's count
+// matrix before it releases the notify flag.
 // ---------------------------------------------------------------------------------------
 constexpr int kNotifyWarps = 8;
 
 // One chunk of 32 tokens (lane = token) by one warp. `bits` is the warp's [B] bitmask scratch in
-// shared memory (expert mode only).
+// shared memory (expert mode only), `hist` the chunk's row of B counts (shared or global memory).
 template <int MODE>
 __device__ __forceinline__ void notify_chunk(const EpGeom& g, int c, int lane, unsigned int* bits,
                                              const bool* __restrict__ is_in_rank,
                                              const long long* __restrict__ topk_idx,
-                                             int* __restrict__ item_rank, int* chunk_hist,
-                                             int* status) {
+                                             int* __restrict__ item_rank, int* hist, int* status) {
   const int J = g.J, B = g.B, R = g.R, E = g.E, K = g.K;
   const unsigned lt = (1u << lane) - 1u;
   const int t = c * kChunkTokens + lane;
@@ -166,52 +165,87 @@ __device__ __forceinline__ void notify_chunk(const EpGeom& g, int c, int lane, u
       const bool in = (mine >> j) & 1u;
       const unsigned m = __ballot_sync(0xffffffffu, in);
       if (valid) item_rank[(size_t)t * J + j] = in ? __popc(m & lt) : -1;
-      if (lane == 0) chunk_hist[(size_t)c * B + j] = __popc(m);
+      if (lane == 0) hist[j] = __popc(m);
     }
   } else {
+    // eight choices at a time: their loads are independent (one latency), and up to eight stay in registers
+    int e[8];
+    auto load = [&](int k0) {
+      long long v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = (valid && k0 + u < K) ? topk_idx[(size_t)t * K + k0 + u] : -1;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) e[u] = (v[u] >= 0 && v[u] < E) ? (int)v[u] : (v[u] == -1 ? -1 : -2);
+    };
+    load(0);
     for (int b = lane; b < B; b += 32) bits[b] = 0u;
     __syncwarp();
-    bool dup = false;
-    for (int k = 0; k < K; ++k) {
-      const long long e = valid ? topk_idx[(size_t)t * K + k] : -1;
-      if (e >= 0 && e < E) {
-        const unsigned old = atomicOr(&bits[(int)e], 1u << lane);
-        if (old & (1u << lane)) dup = true;     // the same expert twice in one token
-      } else if (e != -1) {
-        set_status(status, kBadExpertIndex);
+    bool dup = false, bad = false;
+    for (int k0 = 0; k0 < K; k0 += 8) {
+      if (k0 > 0) load(k0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (e[u] >= 0) dup |= (atomicOr(&bits[e[u]], 1u << lane) >> lane) & 1u;     // the same expert twice in one token
+        else bad |= e[u] == -2;
       }
     }
-    if (dup) set_status(status, kBadExpertIndex);
+    if (dup || bad) set_status(status, kBadExpertIndex);
     __syncwarp();
-    for (int k = 0; k < K && valid; ++k) {
-      const long long e = topk_idx[(size_t)t * K + k];
-      int r = -1;
-      if (e >= 0 && e < E) {
-        r = __popc(bits[(int)e] & lt);
-        if (dup)                                 // keep the first occurrence only
-          for (int q = 0; q < k; ++q)
-            if (topk_idx[(size_t)t * K + q] == e) r = -1;
+    for (int k0 = 0; k0 < K; k0 += 8) {
+      if (K > 8) load(k0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (!valid || k0 + u >= K) continue;
+        int r = e[u] >= 0 ? __popc(bits[e[u]] & lt) : -1;
+        if (dup && r >= 0)                             // keep the first occurrence only
+          for (int q = 0; q < k0 + u; ++q)
+            if (topk_idx[(size_t)t * K + q] == e[u]) r = -1;
+        item_rank[(size_t)t * J + k0 + u] = r;
       }
-      item_rank[(size_t)t * J + k] = r;
     }
-    for (int b = lane; b < B; b += 32) chunk_hist[(size_t)c * B + b] = __popc(bits[b]);
+    for (int b = lane; b < B; b += 32) hist[b] = __popc(bits[b]);
     __syncwarp();
   }
 }
 
-// Run by ONE CTA after every chunk histogram is visible to it: exclusive scan over chunks per
-// bucket (histograms become chunk bases), this rank's count vector, its copy into every peer's
-// count matrix, and the notify flag. `hist` is [B + R + E] ints of shared memory.
-// The flag store is a system-scope release issued after a CTA barrier that follows the count
-// stores, which orders them before the flag for every observer (release cumulativity).
+// This rank's count vector from its bucket totals `hist` [B], its copy into every peer's count matrix, and
+// the notify flag. Run by one CTA; `vec` is [R + E] ints of shared memory. The flag store is a
+// system-scope release issued after a CTA barrier that follows the count stores, which orders them
+// before the flag for every observer (release cumulativity).
 template <int MODE>
-__device__ __forceinline__ void notify_publish(const EpGeom& g, const EpRegions& rg,
-                                               const PeerPtrs& peers,
+__device__ __forceinline__ void notify_publish(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                                                const int* __restrict__ num_tokens_per_expert,
-                                               int* chunk_hist, int* hist, int C) {
-  const int B = g.B, R = g.R, E = g.E;
+                                               const int* hist, int* vec) {
+  const int R = g.R, E = g.E, V = R + E;
+  if (MODE == 0) {
+    for (int i = threadIdx.x; i < R; i += blockDim.x) vec[i] = hist[i];
+    for (int i = threadIdx.x; i < E; i += blockDim.x)
+      vec[R + i] = num_tokens_per_expert ? num_tokens_per_expert[i] : 0;
+  } else {
+    for (int i = threadIdx.x; i < E; i += blockDim.x) vec[R + i] = hist[i];
+    for (int d = threadIdx.x; d < R; d += blockDim.x) {
+      int s = 0;
+      for (int q = 0; q < g.El; ++q) s += hist[d * g.El + q];
+      vec[d] = s;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < R * V; i += blockDim.x) {
+    const int p = i / V, v = i % V;
+    int* dst = reinterpret_cast<int*>(peers.base[p] + rg.counts) + (size_t)g.rank * V + v;
+    st_relaxed_sys(dst, vec[v]);
+  }
+  __syncthreads();
+  if (threadIdx.x < R) {
+    int* flag = reinterpret_cast<int*>(peers.base[threadIdx.x] + rg.flags) +
+                kChNotify * kMaxRanks + g.rank;
+    st_release_sys(flag, g.epoch);
+  }
+}
+
+// Exclusive scan over chunks per bucket, in place (histograms become chunk bases); totals to hist [B]. One CTA.
+__device__ __forceinline__ void notify_scan(int* chunk_hist, int* hist, int B, int C) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  int* vec = hist + B;                                   // [R+E]
   if (B <= nwarps * 2) {
     // few buckets: one warp per bucket, lanes over chunks, all loads of a pass issued together
     for (int b = warp; b < B; b += nwarps) {
@@ -257,36 +291,11 @@ __device__ __forceinline__ void notify_publish(const EpGeom& g, const EpRegions&
     }
   }
   __syncthreads();
-  const int V = R + E;
-  if (MODE == 0) {
-    for (int i = threadIdx.x; i < R; i += blockDim.x) vec[i] = hist[i];
-    for (int i = threadIdx.x; i < E; i += blockDim.x)
-      vec[R + i] = num_tokens_per_expert ? num_tokens_per_expert[i] : 0;
-  } else {
-    for (int i = threadIdx.x; i < E; i += blockDim.x) vec[R + i] = hist[i];
-    for (int d = threadIdx.x; d < R; d += blockDim.x) {
-      int s = 0;
-      for (int q = 0; q < g.El; ++q) s += hist[d * g.El + q];
-      vec[d] = s;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < R * V; i += blockDim.x) {
-    const int p = i / V, v = i % V;
-    int* dst = reinterpret_cast<int*>(peers.base[p] + rg.counts) + (size_t)g.rank * V + v;
-    st_relaxed_sys(dst, vec[v]);
-  }
-  __syncthreads();
-  if (threadIdx.x < R) {
-    int* flag = reinterpret_cast<int*>(peers.base[threadIdx.x] + rg.flags) +
-                kChNotify * kMaxRanks + g.rank;
-    st_release_sys(flag, g.epoch);
-  }
 }
 
 template <int MODE>
 __global__ void __launch_bounds__(kNotifyWarps * 32)
-notify_send_kernel(EpGeom g, EpRegions rg, PeerPtrs peers, const bool* __restrict__ is_in_rank,
+notify_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, const bool* __restrict__ is_in_rank,
                    const long long* __restrict__ topk_idx,
                    const int* __restrict__ num_tokens_per_expert, int* __restrict__ item_rank,
                    int* chunk_hist, unsigned int* block_counter, int* status) {
@@ -296,35 +305,84 @@ notify_send_kernel(EpGeom g, EpRegions rg, PeerPtrs peers, const bool* __restric
   const int c = blockIdx.x * kNotifyWarps + warp;
   if (c < C)
     notify_chunk<MODE>(g, c, lane, reinterpret_cast<unsigned int*>(sh) + (size_t)warp * g.B,
-                       is_in_rank, topk_idx, item_rank, chunk_hist, status);
+                       is_in_rank, topk_idx, item_rank, chunk_hist + (size_t)c * g.B, status);
   if (!last_block_arrive(block_counter, gridDim.x)) return;
-  notify_publish<MODE>(g, rg, peers, num_tokens_per_expert, chunk_hist,
-                       sh + (MODE == 1 ? kNotifyWarps * g.B : 0), C);
+  int* hist = sh + (MODE == 1 ? kNotifyWarps * g.B : 0);
+  notify_scan(chunk_hist, hist, g.B, C);
+  notify_publish<MODE>(g, rg, peers, num_tokens_per_expert, hist, hist + g.B);
 }
 
-// One thread-block cluster instead of a grid with an arrival counter: the warps of the eight
-// CTAs stride over the chunks, a cluster barrier (release/acquire at cluster scope, which
-// covers the global-memory histograms the other CTAs wrote) replaces the device fence + atomic,
-// and CTA 0 publishes.
+// One thread-block cluster instead of a grid with an arrival counter. Every CTA takes `per` consecutive
+// chunks, keeps their histograms in shared memory and scans them there; the CTAs' totals meet through
+// distributed shared memory, every CTA writes its own chunk bases, CTA 0 publishes. Nothing but the results
+// goes through global memory. (With histograms in global memory, one latency per choice and CTA 0
+// scanning all chunks 2047 tokens x top-8 of 64 experts took 12.1 us, 4096 tokens in rank mode 6.3 us; now
+// 7.6 and
+// 5.0 us on one B200: a chain of launch, index loads, two cluster barriers and the peer stores.)
 template <int MODE>
-__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallClusterThreads)
-notify_send_cluster_kernel(EpGeom g, EpRegions rg, PeerPtrs peers,
+__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallClusterThreads, 1)
+notify_send_cluster_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers,
                            const bool* __restrict__ is_in_rank,
                            const long long* __restrict__ topk_idx,
                            const int* __restrict__ num_tokens_per_expert,
-                           int* __restrict__ item_rank, int* chunk_hist, int* status) {
+                           int* __restrict__ item_rank, int* chunk_base, int per, int* status) {
   extern __shared__ int sh[];
   constexpr int kWarps = kSmallClusterThreads / 32;
   cg::cluster_group cluster = cg::this_cluster();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, B = g.B;
+  int* s_hist = sh;                                  // [per][B] chunk histograms, then bases inside this CTA
+  int* s_tot = s_hist + per * B;                     // [B] totals of this CTA's chunks (read by the others)
+  int* s_base = s_tot + B;                           // [B] chunks of the CTAs before this one; CTA 0: all chunks
+  int* vec = s_base + B;                             // [R + E]
+  unsigned int* bits = reinterpret_cast<unsigned int*>(vec + g.R + g.E) + (size_t)warp * B;    // expert mode
   const int C = g.T > 0 ? (g.T + kChunkTokens - 1) / kChunkTokens : 1;
-  for (int c = blockIdx.x * kWarps + warp; c < C; c += gridDim.x * kWarps)
-    notify_chunk<MODE>(g, c, lane, reinterpret_cast<unsigned int*>(sh) + (size_t)warp * g.B,
-                       is_in_rank, topk_idx, item_rank, chunk_hist, status);
-  cluster.sync();
-  if (cluster.block_rank() != 0) return;
-  notify_publish<MODE>(g, rg, peers, num_tokens_per_expert, chunk_hist,
-                       sh + (MODE == 1 ? kWarps * g.B : 0), C);
+  const int me = cluster.block_rank(), lo = me * per, n = max(0, min(per, C - lo));
+  for (int c = warp; c < n; c += kWarps)
+    notify_chunk<MODE>(g, lo + c, lane, bits, is_in_rank, topk_idx, item_rank, s_hist + c * B, status);
+  __syncthreads();
+  if (B <= 2 * kWarps) {                             // few buckets: a warp per bucket, lanes over chunks
+    for (int b = warp; b < B; b += kWarps) {
+      int carry = 0;
+      for (int c0 = 0; c0 < n; c0 += 32) {
+        const int v = c0 + lane < n ? s_hist[(c0 + lane) * B + b] : 0;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += x;
+        }
+        if (c0 + lane < n) s_hist[(c0 + lane) * B + b] = carry + incl - v;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) s_tot[b] = carry;
+    }
+  } else {
+    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+      int carry = 0;
+      for (int c = 0; c < n; ++c) {
+        const int v = s_hist[c * B + b];
+        s_hist[c * B + b] = carry;
+        carry += v;
+      }
+      s_tot[b] = carry;
+    }
+  }
+  cluster.sync();                                    // every CTA's totals are in place
+  for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    int before = 0, all = 0;
+#pragma unroll
+    for (int r = 0; r < kSmallCluster; ++r) {
+      const int v = cluster.map_shared_rank(s_tot, r)[b];
+      before += r < me ? v : 0;
+      all += v;
+    }
+    s_base[b] = me == 0 ? all : before;
+  }
+  __syncthreads();
+  if (me == 0) notify_publish<MODE>(g, rg, peers, num_tokens_per_expert, s_base, vec);
+  for (int i = threadIdx.x; i < n * B; i += blockDim.x)
+    chunk_base[(size_t)lo * B + i] = s_hist[i] + (me == 0 ? 0 : s_base[i % B]);
+  cluster.sync();                                    // nobody leaves while its totals may still be read
 }
 
 void launch_notify_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
@@ -333,16 +391,20 @@ void launch_notify_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& pe
                         unsigned int* block_counter, int* status, cudaStream_t st) {
   const int C = g.T > 0 ? (g.T + kChunkTokens - 1) / kChunkTokens : 1;
   constexpr int kClusterWarps = kSmallClusterThreads / 32;
-  const size_t csmem = sizeof(int) * ((g.mode == 1 ? kClusterWarps * g.B : 0) + g.B + g.R + g.E);
+  const int per = (C + kSmallCluster - 1) / kSmallCluster;
+  const size_t csmem = sizeof(int) * ((size_t)per * g.B + 2 * g.B + g.R + g.E + (g.mode == 1 ? kClusterWarps * g.B : 0));
+  // one cluster while its CTAs' chunk histograms fit their shared memory; up to 256 tokens one CTA is enough
   if (C > kNotifyWarps && C <= kLayoutClusterMaxTokens / kChunkTokens && csmem <= 200 * 1024) {
     if (g.mode == 0) {
+      if (csmem > 48 * 1024)
+        cudaFuncSetAttribute(notify_send_cluster_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
       notify_send_cluster_kernel<0><<<kSmallCluster, kSmallClusterThreads, csmem, st>>>(
-          g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, status);
+          g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, per, status);
     } else {
       if (csmem > 48 * 1024)
         cudaFuncSetAttribute(notify_send_cluster_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
       notify_send_cluster_kernel<1><<<kSmallCluster, kSmallClusterThreads, csmem, st>>>(
-          g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, status);
+          g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, per, status);
     }
     return;
   }

@@ -558,3 +558,48 @@ def test_clone_views_copies_every_byte_of_every_buffer():
         C.clone_views([src[4][1:]])                     # not 16-byte aligned
     with pytest.raises(RuntimeError):
         C.clone_views(src + src[:1])
+
+
+# the count exchange as one CTA (T <= 256), as one cluster (several chunks per CTA, a last CTA with none, few and many
+# buckets) and as a grid with an arrival counter (histograms beyond a cluster's shared memory); choices above eight
+@pytest.mark.parametrize("R,T,E,K", [(1, 256, 8, 2), (1, 257, 8, 8), (2, 300, 64, 9), (1, 2047, 64, 8), (2, 4096, 256, 8),
+                                     (4, 1025, 16, 3), (1, 60000, 256, 2), (2, 33, 32, 1)])
+def test_row_order_of_the_count_exchange(R, T, E, K):
+    H = 8
+    g = torch.Generator().manual_seed(T)
+    idxs = [torch.rand(T, E, generator=g).topk(K, dim=-1).indices for _ in range(R)]
+    idxs[0][T // 3] = -1                                      # a token without choices
+    grp = _group(R, 256 << 20)
+    El = E // R
+    try:
+        # a row says who sent it: (rank, token) in two exact bf16 pairs of bytes
+        xs = []
+        for r in range(R):
+            x = torch.zeros(T, H)
+            x[:, 0], x[:, 1], x[:, 2] = r, torch.arange(T) // 256, torch.arange(T) % 256
+            xs.append(x.to(torch.bfloat16).cuda())
+        ci = [i.cuda() for i in idxs]
+        for grouped in (True, False):
+            lays = None if grouped else grp.get_dispatch_layout(ci, E)
+            outs = grp.dispatch(xs, layouts=lays, topk_idx=ci, group_by_expert=grouped, num_experts=E)
+            for d in range(R):
+                src, tok = [], []
+                if grouped:
+                    for e in range(d * El, (d + 1) * El):
+                        for r in range(R):
+                            t = (idxs[r] == e).any(1).nonzero().flatten()
+                            src.append(torch.full_like(t, r))
+                            tok.append(t)
+                else:
+                    for r in range(R):
+                        t = ((idxs[r] >= d * El) & (idxs[r] < (d + 1) * El)).any(1).nonzero().flatten()
+                        src.append(torch.full_like(t, r))
+                        tok.append(t)
+                src, tok = torch.cat(src), torch.cat(tok)
+                got = outs[d][0].float().cpu().long()
+                assert got.shape[0] == src.numel()
+                assert torch.equal(got[:, 0], src) and torch.equal(got[:, 1] * 256 + got[:, 2], tok)
+        grp.check_status()
+        grp.check_canaries()
+    finally:
+        grp.destroy()
