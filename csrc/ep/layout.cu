@@ -317,8 +317,7 @@ notify_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peer
 // distributed shared memory, every CTA writes its own chunk bases, CTA 0 publishes. Nothing but the results
 // goes through global memory. (With histograms in global memory, one latency per choice and CTA 0
 // scanning all chunks 2047 tokens x top-8 of 64 experts took 12.1 us, 4096 tokens in rank mode 6.3 us; now
-// 7.6 and
-// 5.0 us on one B200: a chain of launch, index loads, two cluster barriers and the peer stores.)
+// 7.6 and 5.0 us on one B200: a chain of launch, index loads, two cluster barriers and the peer stores.)
 template <int MODE>
 __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallClusterThreads, 1)
 notify_send_cluster_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers,
