@@ -13,6 +13,8 @@ constexpr int kCloneChunk = kCloneThreads * kCloneVecs * 16;      // bytes that 
 
 __global__ void __launch_bounds__(kCloneThreads)
 clone_kernel(const __grid_constant__ CloneArgs a) {
+  stream_order_wait();
+  stream_order_next();
   const int total = a.first_chunk[a.n];
   for (int c = blockIdx.x; c < total; c += gridDim.x) {
     int s = 0;
@@ -50,7 +52,7 @@ int launch_clone(CloneArgs a, cudaStream_t st) {
   a.first_chunk[a.n] = (int)chunks;
   if (chunks == 0) return 0;
   const int grid = (int)(chunks < 148 * 8 ? chunks : 148 * 8);
-  clone_kernel<<<grid, kCloneThreads, 0, st>>>(a);
+  launch_ordered(clone_kernel, grid, kCloneThreads, 0, st, 1, a);
   return 0;
 }
 

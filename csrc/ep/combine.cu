@@ -285,6 +285,8 @@ __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const
 template <typename T>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombineArgs a, int* status) {
+  stream_order_wait();
+  if (g.R == 1) stream_order_next();
   if (a.role != kCombineReduceOnly) combine_send_role(a, g, rg, peers, status);
   if (a.role != kCombineSendOnly) combine_reduce_role<T>(a, g, rg, peers.base[g.rank], status);
 }
@@ -321,11 +323,11 @@ void launch_combine(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
   const ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, a.role == kCombineReduceOnly);
   a.parts = rs.parts;
   if (dtype_code == 0)
-    combine_kernel<__nv_bfloat16><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_kernel<__nv_bfloat16>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else if (dtype_code == 1)
-    combine_kernel<__half><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_kernel<__half>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else
-    combine_kernel<float><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_kernel<float>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
 }
 
 // ---- pull form -----------------------------------------------------------------------------
@@ -334,6 +336,8 @@ __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombinePullArgs a, int* status) {
   __shared__ long long s_info[kMaxRanks][4];
   __shared__ int s_ok;
+  stream_order_wait();
+  if (g.R == 1) stream_order_next();
   const int lane = threadIdx.x & 31;
   char* self_base = peers.base[g.rank];
   if (a.publish && blockIdx.x == 0 && (int)threadIdx.x < g.R) {
@@ -394,11 +398,11 @@ void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& p
   if (!a.pull) rs = ReduceShape{1, 1, 1};
   a.parts = rs.parts;
   if (dtype_code == 0)
-    combine_pull_kernel<__nv_bfloat16><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_pull_kernel<__nv_bfloat16>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else if (dtype_code == 1)
-    combine_pull_kernel<__half><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_pull_kernel<__half>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else
-    combine_pull_kernel<float><<<rs.blocks, rs.warps * 32, 0, st>>>(g, rg, peers, a, status);
+    launch_ordered(combine_pull_kernel<float>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
 }
 
 // Signal only (used when a fused GEMM epilogue has already stored the rows).

@@ -196,6 +196,8 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
                      const int* __restrict__ item_rank, const int* __restrict__ chunk_base,
                      int* send_row, int* send_slot, unsigned int* block_counter, int* host_word,
                      int* status, const float* __restrict__ scales_in) {
+  stream_order_wait();
+  if (g.R == 1) stream_order_next();
   extern __shared__ int dyn[];               // [B] send_base, [B] comb_base, [E] scratch
   __shared__ char* s_dst[kSendWarps][kMaxItemsPerToken];
   __shared__ float* s_scl[kSendWarps][kMaxItemsPerToken];
@@ -375,7 +377,7 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
 }
 
 #define B200EP_LAUNCH_DISPATCH(MODE, FP8, CACHED)                                              \
-  dispatch_send_kernel<MODE, FP8, CACHED><<<blocks, warps * 32, smem, st>>>(                   \
+  launch_ordered(dispatch_send_kernel<MODE, FP8, CACHED>, blocks, warps * 32, smem, st, 1,     \
       g, rg, peers, m, x, row_bytes_in, parts, topk_idx, topk_w, item_rank, chunk_base,        \
       send_row, send_slot, block_counter, host_word, status, scales_in)
 

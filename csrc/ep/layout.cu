@@ -61,6 +61,8 @@ layout_kernel(const long long* __restrict__ topk_idx, int T, int K, int E, int R
               bool* __restrict__ is_token_in_rank, int* partial, unsigned int* block_counter,
               int* status) {
   extern __shared__ int sh[];
+  stream_order_wait();
+  stream_order_next();
   int* he = sh;
   int* hr = sh + E;
   for (int i = threadIdx.x; i < E + R; i += blockDim.x) sh[i] = 0;
@@ -94,6 +96,8 @@ layout_cluster_kernel(const long long* __restrict__ topk_idx, int T, int K, int 
                       bool* __restrict__ is_token_in_rank, int* status) {
   extern __shared__ int sh[];
   cg::cluster_group cluster = cg::this_cluster();
+  stream_order_wait();
+  stream_order_next();
   int* he = sh;
   int* hr = sh + E;
   for (int i = threadIdx.x; i < E + R; i += blockDim.x) sh[i] = 0;
@@ -124,12 +128,12 @@ void launch_layout(const long long* topk_idx, int T, int K, int E, int R, int* p
                    int* status, cudaStream_t st) {
   const size_t smem = (E + R) * sizeof(int);
   if (T > kLayoutThreads && T <= kLayoutClusterMaxTokens && smem <= 48 * 1024) {
-    layout_cluster_kernel<<<kSmallCluster, kSmallClusterThreads, smem, st>>>(
+    launch_ordered(layout_cluster_kernel, kSmallCluster, kSmallClusterThreads, smem, st, 1,
         topk_idx, T, K, E, R, per_rank, per_expert, in_rank, status);
     return;
   }
   const int blocks = T > 0 ? (T + kLayoutThreads - 1) / kLayoutThreads : 1;
-  layout_kernel<<<blocks, kLayoutThreads, smem, st>>>(
+  launch_ordered(layout_kernel, blocks, kLayoutThreads, smem, st, 1,
       topk_idx, T, K, E, R, per_rank, per_expert, in_rank, partial, block_counter, status);
 }
 
@@ -300,6 +304,8 @@ notify_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peer
                    const int* __restrict__ num_tokens_per_expert, int* __restrict__ item_rank,
                    int* chunk_hist, unsigned int* block_counter, int* status) {
   extern __shared__ int sh[];
+  stream_order_wait();
+  stream_order_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int C = g.T > 0 ? (g.T + kChunkTokens - 1) / kChunkTokens : 1;
   const int c = blockIdx.x * kNotifyWarps + warp;
@@ -328,6 +334,8 @@ notify_send_cluster_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerP
   extern __shared__ int sh[];
   constexpr int kWarps = kSmallClusterThreads / 32;
   cg::cluster_group cluster = cg::this_cluster();
+  stream_order_wait();
+  stream_order_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, B = g.B;
   int* s_hist = sh;                                  // [per][B] chunk histograms, then bases inside this CTA
   int* s_tot = s_hist + per * B;                     // [B] totals of this CTA's chunks (read by the others)
@@ -397,12 +405,12 @@ void launch_notify_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& pe
     if (g.mode == 0) {
       if (csmem > 48 * 1024)
         cudaFuncSetAttribute(notify_send_cluster_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
-      notify_send_cluster_kernel<0><<<kSmallCluster, kSmallClusterThreads, csmem, st>>>(
+      launch_ordered(notify_send_cluster_kernel<0>, kSmallCluster, kSmallClusterThreads, csmem, st, 1,
           g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, per, status);
     } else {
       if (csmem > 48 * 1024)
         cudaFuncSetAttribute(notify_send_cluster_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
-      notify_send_cluster_kernel<1><<<kSmallCluster, kSmallClusterThreads, csmem, st>>>(
+      launch_ordered(notify_send_cluster_kernel<1>, kSmallCluster, kSmallClusterThreads, csmem, st, 1,
           g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist, per, status);
     }
     return;
@@ -410,13 +418,13 @@ void launch_notify_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& pe
   const int blocks = (C + kNotifyWarps - 1) / kNotifyWarps;
   const size_t smem = sizeof(int) * ((g.mode == 1 ? kNotifyWarps * g.B : 0) + g.B + g.R + g.E);
   if (g.mode == 0) {
-    notify_send_kernel<0><<<blocks, kNotifyWarps * 32, smem, st>>>(
+    launch_ordered(notify_send_kernel<0>, blocks, kNotifyWarps * 32, smem, st, 1,
         g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist,
         block_counter, status);
   } else {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(notify_send_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    notify_send_kernel<1><<<blocks, kNotifyWarps * 32, smem, st>>>(
+    launch_ordered(notify_send_kernel<1>, blocks, kNotifyWarps * 32, smem, st, 1,
         g, rg, peers, is_in_rank, topk_idx, num_tokens_per_expert, item_rank, chunk_hist,
         block_counter, status);
   }
