@@ -477,15 +477,22 @@ class Buffer:
             mode, T, st["epoch_n"], self._timeout_ns(), st.get("is_token_in_rank"), st["topk_idx"], per_expert)
         return st
 
-    def _dispatch_p2(self, st):
+    def _dispatch_p2(self, st, zero_copy: bool = True, num_worst_tokens: int = 0):
         """The send kernel. One process per GPU: its last CTA also waits for the peers, so the
         receive region is complete when the kernel ends. Virtual ranks on one GPU: the wait is a
-        separate launch (`_dispatch_p3`) issued after every rank's send."""
+        separate launch (`_dispatch_p3`) issued after every rank's send. In a group of one the rows that a
+        caller will own (`zero_copy=False`) go into tensors of their own at once: the host knows a bound on
+        their number, the items sent, before it knows the number."""
         self._epoch["dispatch"] += 1
         st["epoch_d"] = self._epoch["dispatch"]
-        self._ctx.send(st["mode"], st["epoch_d"], st.get("epoch_n", 0), self._single_launch, self._timeout_ns(), self._blocks(),
+        own = 0
+        # (with a caller's bound the region is used: the rows beyond the count keep what it holds there)
+        if self.group_size == 1 and not zero_copy and num_worst_tokens <= 0:
+            items = st["T"] * (st["K"] if st["mode"] == 1 else 1)
+            own = min(max(items, st["handle"].n_recv if st["cached"] else 0), st["carve"].cap)
+        st["own"] = self._ctx.send(st["mode"], st["epoch_d"], st.get("epoch_n", 0), self._single_launch, self._timeout_ns(), self._blocks(),
                        st["meta"], st["x"], st["fp8"], st["cached"], st["topk_idx"], st.get("topk_weights"), st["send_row"],
-                       st["send_slot"], st["scales_in"])
+                       st["send_slot"], st["scales_in"], own)
 
     def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1):
         R, E, K, H = self.group_size, st["E"], st["K"], st["H"]
@@ -518,25 +525,15 @@ class Buffer:
             if expert_alignment > 1:
                 per_expert_list = [align_up(c, expert_alignment) for c in per_expert_list]
             self._poll_status()       # the host already waited for the kernel's prologue: cheap to look
-        reg = carve.regions[st["epoch_d"] & 1]
-        # the views a caller gets; owned copies of all of them leave in one launch
-        views = []
-        if st["fp8_out"]:
-            views.append(self.region.view(reg["recv_x"], (n_recv, H), "float8_e4m3fn"))
-            views.append(self.region.view(reg["recv_scales"], (n_recv, H // 128), "float32"))
-        else:
-            views.append(self.region.view(reg["recv_x"], (n_recv, H), _ELEM_DTYPE[st["in_dtype"]]))
-        n_x = len(views)
         side = st["mode"] == 0 and st["topk_idx"] is not None
-        if not st["cached"]:
-            if side:
-                views.append(self.region.view(reg["recv_topk_idx"], (n_recv, K), "int64"))
-                views.append(self.region.view(reg["recv_topk_w"], (n_recv, K), "float32"))
-            if st["mode"] == 1:
-                views.append(self.region.view(reg["recv_prob"], (n_recv,), "float32"))
-            views.append(self.region.view(reg["recv_meta"], (n_recv, 2), "int32"))
-        if not zero_copy:
-            views = self.C.clone_views(views)
+        n_x = 2 if st["fp8_out"] else 1
+        if st["own"]:
+            # cut to the count in place: a slice would be a view, which autograd treats differently
+            views = [t if t.shape[0] == n_recv else t.resize_((n_recv, *t.shape[1:])) for t in st["own"]]
+        else:
+            views = self._region_outputs(st, carve, n_recv, side)
+            if not zero_copy:
+                views = self.C.clone_views(views)      # owned copies of all of them leave in one launch
         recv_x = tuple(views[:2]) if n_x == 2 else views[0]
         if st["cached"]:
             return recv_x, None, None, per_expert_list, st["handle"]
@@ -547,6 +544,23 @@ class Buffer:
                                 st["meta"], recv_meta, st["topk_idx"], st.get("is_token_in_rank"),
                                 per_expert_list, st["fp8_out"], recv_prob, carve.key, carve.cap)
         return recv_x, recv_topk_idx, recv_topk_w, per_expert_list, handle
+
+    def _region_outputs(self, st, carve, n_recv: int, side: bool) -> List[torch.Tensor]:
+        """Views of what a dispatch received: rows (and fp8 scales), routing ids and weights, probabilities, row table."""
+        H, K, reg = st["H"], st["K"], carve.regions[st["epoch_d"] & 1]
+        if st["fp8_out"]:
+            views = [self.region.view(reg["recv_x"], (n_recv, H), "float8_e4m3fn"),
+                     self.region.view(reg["recv_scales"], (n_recv, H // 128), "float32")]
+        else:
+            views = [self.region.view(reg["recv_x"], (n_recv, H), _ELEM_DTYPE[st["in_dtype"]])]
+        if not st["cached"]:
+            if side:
+                views.append(self.region.view(reg["recv_topk_idx"], (n_recv, K), "int64"))
+                views.append(self.region.view(reg["recv_topk_w"], (n_recv, K), "float32"))
+            if st["mode"] == 1:
+                views.append(self.region.view(reg["recv_prob"], (n_recv,), "float32"))
+            views.append(self.region.view(reg["recv_meta"], (n_recv, 2), "int32"))
+        return views
 
     @_nvtx("b200ep.dispatch")
     def dispatch(self, x, handle: Optional[DispatchHandle] = None, num_tokens_per_rank=None,
@@ -575,7 +589,7 @@ class Buffer:
         with self._on_stream():
             st = self._dispatch_p1(x, handle, is_token_in_rank, num_tokens_per_expert, topk_idx,
                                    topk_weights, use_fp8, group_by_expert, num_experts)
-            self._dispatch_p2(st)
+            self._dispatch_p2(st, zero_copy, num_worst_tokens)
             out = self._dispatch_p3(st, zero_copy, num_worst_tokens, expert_alignment)
         if compute is None and not async_finish:
             return (*out, None)

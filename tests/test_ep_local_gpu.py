@@ -560,6 +560,57 @@ def test_clone_views_copies_every_byte_of_every_buffer():
         C.clone_views(src + src[:1])
 
 
+# a group of one: owned outputs are written where they are owned, and equal the views of the region; T = 0, every
+# choice masked, more items than rows, few and all choices masked
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("form", ["plain", "fp8", "tuple"])
+@pytest.mark.parametrize("T,masked", [(0, 0.0), (1, 0.0), (33, 1.0), (130, 0.4), (257, 0.0)])
+def test_owned_outputs_of_a_group_of_one_equal_the_region_views(T, masked, form, grouped):
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    H, E, K = 256, 8, 3
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+    idx = torch.rand(T, E, generator=g).topk(K, dim=-1).indices
+    idx[torch.rand(T, K, generator=g) < masked] = -1
+    idx, w = idx.cuda(), torch.rand(T, K, generator=g).cuda()
+    if form == "tuple":
+        x = (x.to(torch.float8_e4m3fn), torch.rand(T, H // 128, generator=g).cuda())
+    raw = lambda t: t.contiguous().view(torch.uint8) if t.dtype == torch.float8_e4m3fn else t
+    buf = Buffer(None, 32 << 20, world=LocalWorld.make(1)[0], timeout_s=2.0)
+    try:
+        lay = {} if grouped else dict(zip(("num_tokens_per_rank", "is_token_in_rank"),
+                                          (lambda l: (l[0], l[3]))(buf.get_dispatch_layout(idx, E))))
+        kw = dict(topk_idx=idx, topk_weights=w, num_experts=E, group_by_expert=grouped, use_fp8=form == "fp8", **lay)
+
+        def flat(out):
+            rx, ri, rw, cnt, h, _ = out
+            ts = [*(rx if isinstance(rx, tuple) else (rx,)), ri, rw, h.recv_prob, h.recv_meta, h.send_row[:T], h.send_slot[:T]]
+            return [t for t in ts if t is not None], cnt, h
+
+        own, own_cnt, h = flat(buf.dispatch(x, **kw))
+        view, cnt, _ = flat(buf.dispatch(x, zero_copy=True, **kw))
+        want = [t.clone() for t in view]
+        for _ in range(2):                                     # both parities of the region are written over
+            buf.dispatch((x[0], x[1] + 1) if form == "tuple" else x + 1, zero_copy=True, **kw)
+        again = buf.dispatch(x, handle=h, use_fp8=form == "fp8")[0]
+        again = list(again) if isinstance(again, tuple) else [again]
+        assert own_cnt == cnt and len(own) == len(want)
+        assert h.n_recv == int((idx >= 0).sum() if grouped else (idx >= 0).any(1).sum())
+        for a, b in zip(own, want):
+            assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(raw(a), raw(b))
+        assert own[0]._base is None                            # its own tensor, not a view of a larger one
+        for a, b in zip(again, want):
+            assert a.shape == b.shape and torch.equal(raw(a), raw(b))
+        if form == "plain" and T:
+            back = buf.combine(own[0], h)[0]
+            n = (idx >= 0).sum(1) if grouped else (idx >= 0).any(1)
+            torch.testing.assert_close(back.float(), (x.float() * n[:, None]).to(torch.bfloat16).float())
+        buf.check_status()
+    finally:
+        buf.destroy()
+
+
 # the count exchange as one CTA (T <= 256), as one cluster (several chunks per CTA, a last CTA with none, few and many
 # buckets) and as a grid with an arrival counter (histograms beyond a cluster's shared memory); choices above eight
 @pytest.mark.parametrize("R,T,E,K", [(1, 256, 8, 2), (1, 257, 8, 8), (2, 300, 64, 9), (1, 2047, 64, 8), (2, 4096, 256, 8),
