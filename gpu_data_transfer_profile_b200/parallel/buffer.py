@@ -11,12 +11,13 @@ API parity (call shapes taken from the reference's call sites):
 
 How it works here (all data-path work is in the sm_100a kernels under csrc/ep):
   1. `notify_send`  counts + stable positions of every item, count vectors stored to all peers.
-  2. `notify_wait`  bounded wait for the peers' counts, prefix sums -> exact destination rows;
-                    N_recv goes to pinned host memory (no device synchronise).
-  3. `dispatch_send` one pass over the local tokens: optional fp8 1x128 cast, 16-byte LSU
-                    stores straight into the final row of each destination's receive region.
-  4. bounded wait for the peers' done-flags; outputs are views (zero-copy) or clones.
-  Combine pushes rows back into per-item slots on the source and reduces them there.
+  2. `dispatch_send` bounded wait for the peers' counts, prefix sums -> exact destination rows (N_recv goes to
+                    pinned host memory, no device synchronise); then one pass over the local tokens: optional
+                    fp8 1x128 cast, 16-byte LSU stores straight into the final row of each destination's receive
+                    region, and a bounded wait for the peers' done-flags.
+  3. outputs are views (zero-copy) or owned tensors (copied in one launch; written directly in a group of one).
+  Combine pulls rows that lie in the symmetric region, or pushes rows into per-item slots on the source and
+  reduces them there (rows of this rank's own tokens are read where they lie).
   Regions are double-buffered by epoch parity, flags are monotonically increasing epochs.
 
 Each op is split into phases (`_dispatch_p1/_p2/_p3`, `_combine_p1/_p2`) so that several
