@@ -35,7 +35,7 @@ constexpr int kLLThreads = 256;  // 8 warps work on one row together
 
 // Per-op device state (6 ints): [0] committed epoch, [1] committed arrival target,
 // [2] epoch published by the send half, [3] target published by the send half,
-// [4] cumulative count of send CTAs that have finished, [5] unused.
+// [4] CTAs of the running send launch that have finished (0 between launches), [5] unused.
 // Send half: works with epoch = [0]+1, target = [1]+grid; CTA 0 publishes them in [2],[3].
 // Receive half: the CTA of the send launch that finishes last (every CTA has read [0],[1] by then)
 // commits the pair to [0],[1]; as a launch of its own it reads [2],[3] and CTA 0 commits them.
@@ -80,12 +80,16 @@ __device__ __forceinline__ LLTick ll_tick_recv(int* st) {
 // (the grid size is the same on every rank). Two ways to get there (P.signal_mode):
 //  0: every CTA makes its stores visible system-wide and adds 1 to the counter on every peer:
 //     no CTA waits for the others, but a receiver takes R x grid remote atomics on R words;
-//  1: every CTA makes its stores visible and counts itself on a LOCAL cumulative counter
-//     (state[4]); the CTA that completes a multiple of the grid size adds the whole grid size to
-//     the counter on every peer: R remote atomics per rank, at the price of one more hop.
+//  1: every CTA makes its stores visible and counts itself on a LOCAL counter (state[4]); the CTA
+//     that completes the grid adds the whole grid size to the counter on every peer: R remote
+//     atomics per rank, at the price of one more hop.
 // Mode 0 measured faster with 2 ranks, mode 1 with 8.
 // `elect`: also find the CTA that finishes last (its caller does the receive half); returns true in
 // that CTA. A group of one has no counters to keep: the end of the launch, or the election, orders it.
+// The CTA that completes the grid sets the local counter back to 0 for the next launch, which is ordered
+// after this one. (A count that runs on from launch to launch and is taken modulo the grid names a
+// CTA in the middle of the grid once a buffer has seen two grid sizes, or when it passes 2^32 with a
+// grid that does not divide it.)
 __device__ __forceinline__ bool ll_arrive_on_peers(const LLParams& P, const PeerPtrs& peers, int channel,
                                                    int* state, unsigned int grid_ctas, bool elect) {
   __shared__ unsigned int s_add;
@@ -98,9 +102,12 @@ __device__ __forceinline__ bool ll_arrive_on_peers(const LLParams& P, const Peer
       if (P.R == 1) __threadfence();
       else if (P.signal_mode != 0) fence_acq_rel_sys();
       const unsigned int prev = atomicAdd(reinterpret_cast<unsigned int*>(state + 4), 1u);
-      last = ((prev + 1u) % grid_ctas) == 0u;
+      last = prev == grid_ctas - 1u;
       // the last CTA acquires what the others published before they counted themselves
-      if (last) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (last) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        state[4] = 0;
+      }
     }
     s_add = P.signal_mode == 0 ? 1u : (last ? grid_ctas : 0u);
     s_last = last;

@@ -233,3 +233,43 @@ def test_low_latency_one_rank_public_calls(T, H, E, K, fp8, in_place):
         buf.check_status()
     finally:
         buf.destroy()
+
+
+# one buffer that serves several bounds on the tokens of a call, so that the grid of its send kernels changes: powers
+# of two and not, fewer tokens than the bound (idle CTAs), odd and even numbers of calls before each change
+@pytest.mark.parametrize("signal_mode", [0, 1])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_low_latency_token_bound_changes_on_one_buffer(signal_mode, in_place, monkeypatch):
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    monkeypatch.setattr(Buffer, "ll_signal_mode", signal_mode)
+    H, E, K = 512, 16, 4
+    buf = Buffer(None, Buffer.get_low_latency_nvl_size_hint(200, H, 1, E, K), 0, low_latency_mode=True,
+                 world=LocalWorld.make(1)[0], timeout_s=2.0)
+    try:
+        for rep, (M, T) in enumerate([(96, 96), (128, 128), (96, 5), (96, 96), (128, 100), (7, 7), (128, 128), (100, 99),
+                                      (7, 3), (1, 1), (200, 200), (128, 128)]):
+            g = torch.Generator().manual_seed(rep)
+            x = torch.randn(T, H, generator=g).to(torch.bfloat16)
+            idx, w = O.make_routing(T, E, K, 90 + rep)
+            xc, ic, wc = x.cuda(), idx.cuda(), w.cuda()
+            recv, count, handle, _, _ = buf.low_latency_dispatch(xc, ic, M, E, use_fp8=False)
+            cnt = count.tolist()
+            assert cnt == [int((idx == e).sum()) for e in range(E)]
+            src = handle[0].cpu()
+            for e in range(E):
+                _, s_t, s_k = _unpack(src[e, :cnt[e]])
+                assert len(set(src[e, :cnt[e]].tolist())) == cnt[e]
+                assert bool((idx[s_t, s_k] == e).all()) and torch.equal(recv[e, :cnt[e]].cpu(), x[s_t])
+            y = recv.clone()
+            if in_place:
+                y = buf.get_next_low_latency_combine_buffer(handle)
+                y.copy_(recv)
+            out, _, hook = buf.low_latency_combine(y, ic, wc, handle, return_recv_hook=rep % 3 == 0)
+            out = hook() if out is None else out
+            # one bf16 rounding of a sum whose weights add up to one within f32 rounding
+            torch.testing.assert_close(out.float(), xc.float() * wc.sum(1, keepdim=True), atol=1e-6, rtol=2.0 ** -7)
+            assert buf._ll_words.view(3, 6)[:, 4].tolist() == [0, 0, 0]       # no count is carried into the next launch
+        buf.check_status()
+    finally:
+        buf.destroy()
