@@ -59,7 +59,7 @@ struct CombineArgs {
   // With send_row (both roles; [T][J] row of (token, item) at its destination) rows whose source is this rank take
   // no slot: the send role skips them, the reduce role reads them from x / topk_w. Null: every row has a slot.
   const int* send_row;
-  const long long* topk_idx; // [T][K] (expert mode, with send_row: which rank holds item k)
+  const int* comb_base;      // [B] first slot of every bucket (expert mode, with send_row: which slots are of own rows)
   int parts;                 // filled by the launcher
 };
 
@@ -82,7 +82,8 @@ struct CombinePullArgs {
   int wait;                  // 1: wait for every peer's announcement of this epoch
   int pull;                  // 1: do the reduction (0 = announce only)
   const int* send_row;       // [T][J] row of (token, item) at its destination
-  const long long* topk_idx; // [T][K] (expert mode: which rank holds item k)
+  const int* send_slot;      // [T][J] and
+  const int* comb_base;      // [B] first slot of every bucket (expert mode: which rank holds the item)
   const float* weights;      // optional [T][J]
   char* out;                 // [T][H]
   float* out_topk_w;         // optional [T][K]

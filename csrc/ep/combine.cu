@@ -155,7 +155,7 @@ __device__ void combine_send_role(const CombineArgs& a, const EpGeom& g, const E
 // Lane j < J looks after contributor j: Index holds what it reads for an item, `fetch(t)` issues
 // those loads and `resolve(t, index, &side)` turns them into the address of the row (null: none)
 // and of its side values. fetch runs one item ahead.
-struct Index { int row, slot; long long expert; float w; };
+struct Index { int row, slot; float w; };
 
 __device__ __forceinline__ int reduce_first(int parts, int warp) { return (warp / parts) * gridDim.x + blockIdx.x; }
 
@@ -256,22 +256,25 @@ __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const
   const float* comb_w = reinterpret_cast<const float*>(self_base + rg.comb_w);
   const bool in_place = a.send_row != nullptr;
   const int n_rows = in_place ? min(*a.n_recv_ptr, g.cap) : 0;
+  // slots of own rows: lane `rank` in rank mode, a range in expert mode (one bucket after the other)
+  int own_lo = lane == g.rank ? 0 : 0x7fffffff, own_hi = 0x7fffffff;
+  if (in_place && g.mode == 1) {
+    own_lo = a.comb_base[g.rank * g.El];
+    if (g.rank + 1 < g.R) own_hi = a.comb_base[(g.rank + 1) * g.El];
+  }
   auto fetch = [&](int t) {
-    Index ix{-1, -1, -1, 1.f};
+    Index ix{-1, -1, 1.f};
     if (t < g.T && lane < J) {
       const size_t at = (size_t)t * J + lane;
       ix.slot = a.send_slot[at];
-      if (in_place) {
-        ix.row = a.send_row[at];
-        ix.expert = g.mode == 0 ? (long long)lane * g.El : a.topk_idx[at];
-      }
+      if (in_place) ix.row = a.send_row[at];
       if (a.weights) ix.w = a.weights[at];
     }
     return ix;
   };
   auto resolve = [&](int t, const Index& ix, const float** side) -> const char* {
     if (ix.slot < 0 || ix.slot >= g.slot_cap) return nullptr;
-    if (in_place && ix.expert >= 0 && ix.expert < g.E && (int)ix.expert / g.El == g.rank) {
+    if (in_place && ix.slot >= own_lo && ix.slot < own_hi) {
       if (ix.row < 0 || ix.row >= n_rows) return nullptr;
       *side = a.topk_w + (size_t)ix.row * wk;
       return a.x + (size_t)ix.row * row_bytes;
@@ -335,6 +338,7 @@ template <typename T>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombinePullArgs a, int* status) {
   __shared__ long long s_info[kMaxRanks][4];
+  __shared__ int s_first[kMaxRanks];
   __shared__ int s_ok;
   stream_order_wait();
   if (g.R == 1) stream_order_next();
@@ -361,6 +365,7 @@ combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pee
       const long long* info = reinterpret_cast<const long long*>(self_base + rg.pull_info) + threadIdx.x * 4;
       for (int q = 0; q < 3; ++q) s_info[threadIdx.x][q] = __ldcg(&info[q]);
     }
+    if (g.mode == 1) s_first[threadIdx.x] = a.comb_base[threadIdx.x * g.El];
   }
   __syncthreads();
   if (!s_ok) return;
@@ -368,19 +373,19 @@ combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pee
   const int row_bytes = g.H * (int)sizeof(T);
   const int wk = g.mode == 0 ? g.K : 1;
   auto fetch = [&](int t) {
-    Index ix{-1, -1, -1, 1.f};
+    Index ix{-1, -1, 1.f};
     if (t < g.T && lane < J) {
       const size_t at = (size_t)t * J + lane;
       ix.row = a.send_row[at];
-      ix.expert = g.mode == 0 ? (long long)lane * g.El : a.topk_idx[at];
+      if (g.mode == 1) ix.slot = a.send_slot[at];
       if (a.weights) ix.w = a.weights[at];
     }
     return ix;
   };
   auto resolve = [&](int t, const Index& ix, const float** side) -> const char* {
     if (ix.row < 0) return nullptr;
-    const int d = (ix.expert >= 0 && ix.expert < g.E) ? (int)ix.expert / g.El : -1;
-    if (d < 0 || (long long)ix.row >= s_info[d][2] || s_info[d][0] < 0) {
+    const int d = g.mode == 0 ? lane : rank_of_slot(s_first, g.R, ix.slot);
+    if ((long long)ix.row >= s_info[d][2] || s_info[d][0] < 0) {
       set_status(status, kOverflowSlots);       // the peer did not announce that many rows
       return nullptr;
     }

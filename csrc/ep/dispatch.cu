@@ -201,6 +201,7 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
   extern __shared__ int dyn[];               // [B] send_base, [B] comb_base, [E] scratch
   __shared__ char* s_dst[kSendWarps][kMaxItemsPerToken];
   __shared__ float* s_scl[kSendWarps][kMaxItemsPerToken];
+  __shared__ int s_first[kMaxRanks];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int J = g.J, K = g.K, El = g.El;
   const int row_bytes_out = FP8 ? g.H : row_bytes_in;
@@ -211,6 +212,10 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
   int* s_send_base = dyn;
   int* s_comb_base = dyn + g.B;
 
+  if (CACHED && MODE == 1) {                 // where each rank's slots begin (from the handle)
+    if ((int)threadIdx.x < g.R) s_first[threadIdx.x] = m.comb_base[threadIdx.x * El];
+    __syncthreads();
+  }
   int n_tokens = g.T;
   // 16-byte vectors of one part of a row (bf16/raw: input vectors; fp8: steps of 512 channels)
   const int nvec = row_bytes_in >> 4;
@@ -241,7 +246,7 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
     const int t = it / parts, part = it - t * parts;
     int row = -1, slot = -1, d = 0;
     if (lane < J) {
-      long long e = (MODE == 1) ? topk_idx[(size_t)t * K + lane] : 0;
+      long long e = (MODE == 1 && !CACHED) ? topk_idx[(size_t)t * K + lane] : 0;
       if (CACHED) {
         row = send_row[(size_t)t * J + lane];
         slot = send_slot[(size_t)t * J + lane];
@@ -269,7 +274,9 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
           send_slot[(size_t)t * J + lane] = slot;
         }
       }
-      d = (MODE == 0) ? lane : (int)(e >= 0 && e < g.E ? e / El : 0);
+      if (MODE == 0) d = lane;
+      else if (CACHED) d = rank_of_slot(s_first, g.R, slot);
+      else d = (int)(e >= 0 && e < g.E ? e / El : 0);
       if (row >= 0) {
         char* pb = peers.base[d];
         if (part == 0) {

@@ -73,4 +73,13 @@ struct EpMeta {
   int* send_total;        // [1] number of slots used on this rank
 };
 
+// Rank that holds the item of slot `slot` (expert mode). Slots are given out bucket by bucket in rank order, so
+// those of the items that went to rank d begin at first[d] = comb_base[d * El]. Combine and cached dispatch find
+// the rank this way, from the handle alone: the caller's index tensor may hold other choices by then.
+__device__ __forceinline__ int rank_of_slot(const int* first, int R, int slot) {
+  int d = 0;
+  for (int q = 1; q < R; ++q) d += slot >= first[q] ? 1 : 0;
+  return d;
+}
+
 }  // namespace b200ep

@@ -69,7 +69,7 @@ class DispatchHandle:
     send_slot: torch.Tensor        # [T,J] int32 slot in my combine region (-1 = none)
     meta: torch.Tensor             # int32 device metadata (counts, prefixes, chunk boundaries)
     recv_meta: torch.Tensor        # [n_recv,2] int32 {slot at source, source rank}
-    topk_idx: Optional[torch.Tensor]
+    topk_idx: Optional[torch.Tensor]       # as given to dispatch; not read again: the caller may refill it
     is_token_in_rank: Optional[torch.Tensor]
     num_recv_tokens_per_expert_list: List[int] = field(default_factory=list)
     fp8: bool = False
@@ -428,7 +428,7 @@ class Buffer:
             if handle.T != T or handle.H != H:
                 raise ValueError("cached handle does not match x")
             st.update(mode=handle.mode, K=handle.K, E=handle.E, handle=handle,
-                      topk_idx=handle.topk_idx, topk_weights=None)
+                      topk_idx=None, topk_weights=None)
         else:
             mode = 1 if group_by_expert else 0
             if topk_idx is not None:
@@ -627,8 +627,8 @@ class Buffer:
         x, w = (st["x"], st["topk_w"]) if in_place or role != 2 else (None, None)
         return self._ctx.combine_push(
             role, handle.mode, handle.T, handle.n_recv, st["ep"], self._timeout_ns(), max(1, Buffer.num_sms),
-            handle.n_recv_dev if x is not None else None, handle.recv_meta if x is not None else None, x, w,
-            handle.send_slot, weights, handle.send_row if in_place else None, handle.topk_idx if in_place else None,
+            handle.meta, handle.recv_meta if x is not None else None, x, w,
+            handle.send_slot, weights, handle.send_row if in_place else None,
             _ELEM_DTYPE[st["dtype"]], st["topk_w"] is not None)
 
     def _combine_p1(self, x, handle: DispatchHandle, topk_weights):
@@ -670,7 +670,7 @@ class Buffer:
         if phase != 2:
             self._epoch["combine"] += 1
         return self._ctx.combine_pull(phase, handle.mode, handle.T, self._epoch["combine"], self._timeout_ns(), max(1, Buffer.num_sms),
-                                      x, topk_weights, handle.send_row, handle.topk_idx, weights)
+                                      x, topk_weights, handle.send_row, handle.send_slot, handle.meta, weights)
 
     def combine_input(self, num_rows: int, hidden: int, dtype=torch.bfloat16) -> torch.Tensor:
         """A [num_rows, hidden] tensor INSIDE the symmetric region for the expert computation to

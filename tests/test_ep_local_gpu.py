@@ -654,3 +654,39 @@ def test_row_order_of_the_count_exchange(R, T, E, K):
         grp.check_canaries()
     finally:
         grp.destroy()
+
+
+# the handle alone says where a row went: the caller may refill the index tensor after dispatch (static buffers under graph
+# replay, interleaved micro-batches), whether the choices are masked or name experts of another rank by then
+@pytest.mark.parametrize("R", [1, 2, 4])
+@pytest.mark.parametrize("pull", [False, True])
+@pytest.mark.parametrize("change", ["masked", "moved"])
+def test_combine_and_cached_dispatch_after_the_index_tensor_is_refilled(R, pull, change):
+    T, H, E, K = 130, 256, 8, 3
+    xs, idxs, ws = _mk(R, T, H, E, K, seed=31)
+    for i in idxs:
+        i[i == E - 1] = -1                                # an expert without rows: the last of the last rank
+        i[0] = -1
+    g = _group(R)
+    try:
+        cx, ci, cw = [x.cuda() for x in xs], [i.cuda() for i in idxs], [w.cuda() for w in ws]
+        outs = g.dispatch(cx, topk_idx=ci, topk_weights=cw, group_by_expert=True, num_experts=E, zero_copy=pull)
+        rows = [o[0].clone() for o in outs]
+        for i in ci:
+            i.copy_(torch.full_like(i, -1) if change == "masked" else (i + max(1, E // R)) % E)
+        handles = [o[4] for o in outs]
+        ys = [o[0].mul_(1 + d) if pull else o[0] * (1 + d) for d, o in enumerate(outs)]
+        comb = g.combine(ys, handles, topk_weights=[h.recv_prob for h in handles])
+        for r in range(R):
+            valid = idxs[r] >= 0
+            factor = torch.where(valid, 1.0 + idxs[r] // (E // R), torch.zeros(())).sum(1, keepdim=True)
+            # factors up to 12 and bf16 rows: one rounding of the row's product, one of the sum
+            torch.testing.assert_close(comb[r][0].cpu().float(), xs[r].float() * factor, rtol=2.0 ** -7, atol=1e-6)
+            assert torch.equal(comb[r][1].cpu(), torch.where(valid, ws[r], torch.zeros(())))
+        again = g.dispatch(cx, handles=handles)
+        for d in range(R):
+            assert torch.equal(again[d][0], rows[d])
+        g.check_status()
+        g.check_canaries()
+    finally:
+        g.destroy()

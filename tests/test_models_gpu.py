@@ -224,3 +224,27 @@ def test_moe_layer_inference_consumes_rows_in_place(use_fp8, fuse, activation):
         A._BUFFERS[(id(None), id(world))].check_status()
     finally:
         A.release_buffers()
+
+
+def test_exchange_backward_after_the_index_tensor_is_refilled():
+    """A static routing buffer that is refilled between the forward and the backward pass of an exchange."""
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    T, H, E, K = 200, 256, 8, 2
+    world = LocalWorld.make(1)[0]
+    A.configure_buffer(num_max_tokens_per_rank=T, num_topk=K, num_experts=E, group_by_expert=True)
+    try:
+        g = torch.Generator().manual_seed(0)
+        x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda().requires_grad_(True)
+        idx = torch.rand(T, E, generator=g).topk(K, dim=-1).indices.cuda()
+        w = torch.rand(T, K, generator=g).cuda().requires_grad_(True)
+        dy = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+        rows, probs, _, handle = A.FusedDispatchGrouped.apply(x, idx, w, E, None, world)
+        out = A.FusedCombineGrouped.apply(rows, None, handle, world)
+        idx.fill_(-1)
+        (out.float() * dy.float()).sum().add(3 * probs.sum()).backward()
+        assert torch.equal(out, 2 * x)
+        assert torch.equal(x.grad, 2 * dy) and torch.equal(w.grad, torch.full_like(w, 3.0))
+        A._BUFFERS[(id(None), id(world))].check_status()
+    finally:
+        A.release_buffers()
