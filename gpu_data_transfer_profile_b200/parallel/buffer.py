@@ -350,7 +350,9 @@ class Buffer:
         caller's stream."""
         return torch.cuda.stream(self.comm_stream) if self.comm_stream is not None else _NULL_CONTEXT
 
-    def _exit(self, compute, async_finish, tensors) -> Optional[EventOverlap]:
+    def _exit(self, compute, async_finish, tensors, held=()) -> Optional[EventOverlap]:
+        """tensors: outputs and inputs that both streams use; held: what else the op's kernels read. The event of an
+        asynchronous op keeps all of them alive: the caller may drop its own references before the kernels run."""
         if compute is None:
             return EventOverlap(EventHandle()) if async_finish else None
         for t in tensors:
@@ -358,7 +360,7 @@ class Buffer:
                 t.record_stream(compute)
         if async_finish:
             self._async_outstanding = True
-            return EventOverlap(EventHandle(self.comm_stream), tuple(tensors))
+            return EventOverlap(EventHandle(self.comm_stream), (*tensors, *held))
         compute.wait_stream(self.comm_stream)
         return None
 
@@ -597,7 +599,8 @@ class Buffer:
         flat = []
         for o in out[:3]:
             flat.extend(o if isinstance(o, tuple) else (o,))
-        ev = self._exit(compute, async_finish, [t for t in flat if t is not None] + [x])
+        ev = self._exit(compute, async_finish, [t for t in flat if t is not None] + [x],
+                        [t for t in st.values() if isinstance(t, torch.Tensor)])
         return (*out, ev)
 
     # ---- combine ---------------------------------------------------------------------
@@ -718,7 +721,8 @@ class Buffer:
                 out = out + (bias[0] if isinstance(bias, (tuple, list)) else bias)
         if compute is None and not async_finish:
             return out, out_w, None
-        ev = self._exit(compute, async_finish, [out, x] + ([out_w] if out_w is not None else []))
+        ev = self._exit(compute, async_finish, [out, x] + ([out_w] if out_w is not None else []),
+                        (topk_weights, item_weights, bias, handle.send_row, handle.send_slot, handle.meta, handle.recv_meta))
         return out, out_w, ev
 
     # ---- low-latency mode -------------------------------------------------------------
@@ -842,11 +846,11 @@ class Buffer:
                     with self._on_stream():
                         box["out"] = self._ll_dispatch_recv(d)
                     return box["out"]
-                ev = self._exit(compute, async_finish, [x])
+                ev = self._exit(compute, async_finish, [x], (d["topk_idx"],))
                 return None, None, None, ev, hook
             recv_x, count, handle = self._ll_dispatch_recv(d)
         flat = list(recv_x) if isinstance(recv_x, tuple) else [recv_x]
-        ev = self._exit(compute, async_finish, flat + [count, x])
+        ev = self._exit(compute, async_finish, flat + [count, x], (d["topk_idx"],))
         return recv_x, count, handle, ev, None
 
     def get_next_low_latency_combine_buffer(self, handle) -> torch.Tensor:
@@ -921,14 +925,14 @@ class Buffer:
                 res = self._ll_combine_pull(0 if self._single_launch else 1, topk_idx, topk_weights, handle, out)
                 if not self._single_launch:
                     res = self._ll_combine_pull(2, topk_idx, topk_weights, handle, res)
-            ev = self._exit(compute, async_finish, [res])
+            ev = self._exit(compute, async_finish, [res], (topk_idx, topk_weights))
             return res, ev, ((lambda: res) if return_recv_hook else None)
         if self.group_size == 1 and not return_recv_hook:
             # every row is an own row: one kernel, nothing is sent
             self._ll_check_combine_input(x)
             with self._on_stream():
                 res = self._ll_combine_pull(0, topk_idx, topk_weights, handle, out, own_x=x)
-            return res, self._exit(compute, async_finish, [res, x]), None
+            return res, self._exit(compute, async_finish, [res, x], (topk_idx, topk_weights)), None
         with self._on_stream():
             # (with a hook the caller may reuse x before the receive half runs: every row goes to its slot)
             c = self._ll_combine_send(x, handle, own_in_place=not return_recv_hook)
@@ -936,9 +940,9 @@ class Buffer:
                 def hook():
                     with self._on_stream():
                         return self._ll_combine_recv(c, topk_idx, topk_weights, out)
-                return None, self._exit(compute, async_finish, [x]), hook
+                return None, self._exit(compute, async_finish, [x], (handle[0], handle[5])), hook
             res = self._ll_combine_recv(c, topk_idx, topk_weights, out)
-        return res, self._exit(compute, async_finish, [res, x]), None
+        return res, self._exit(compute, async_finish, [res, x], (topk_idx, topk_weights, handle[0], handle[5])), None
 
 
 class _LLCarve:

@@ -690,3 +690,40 @@ def test_combine_and_cached_dispatch_after_the_index_tensor_is_refilled(R, pull,
         g.check_canaries()
     finally:
         g.destroy()
+
+
+def _side_stream_buffer(nbytes, **kw):
+    """A group of one whose asynchronous calls run on a communication stream, as those of a process group do."""
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    world = LocalWorld.make(1)[0]
+    world.local = False
+    return Buffer(None, nbytes, world=world, timeout_s=2.0, **kw)
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+def test_asynchronous_calls_hold_what_their_kernels_read(grouped):
+    T, H, E, K = 64, 256, 8, 2
+    (x,), (idx,), (w,) = _mk(1, T, H, E, K)
+    x, idx, w = x.cuda(), idx.cuda(), w.cuda()
+    buf = _side_stream_buffer(32 << 20)
+    held = lambda ev: {t.data_ptr() for t in ev.extra_tensors if isinstance(t, torch.Tensor)}
+    try:
+        _, _, per_expert, in_rank, ev = (None,) * 5 if grouped else buf.get_dispatch_layout(idx, E, async_finish=True)
+        rx, _, rw, _, h, ev = buf.dispatch(x, topk_idx=idx, topk_weights=w, is_token_in_rank=in_rank, num_tokens_per_expert=per_expert,
+                                           num_experts=E, group_by_expert=grouped, async_finish=True, previous_event=ev)
+        read = [x, idx, w, h.send_row, h.send_slot, h.meta] + ([] if grouped else [in_rank, per_expert])
+        assert {t.data_ptr() for t in read} <= held(ev)
+        side = h.recv_prob if grouped else rw
+        iw = torch.rand(T, K if grouped else 1, device="cuda")
+        bias = torch.ones(T, H, dtype=torch.bfloat16, device="cuda")
+        out, out_w, ev = buf.combine(rx, h, topk_weights=side, item_weights=iw, bias=bias, async_finish=True)
+        read = [rx, side, iw, bias, h.send_row, h.send_slot, h.meta, h.recv_meta]
+        assert {t.data_ptr() for t in read} <= held(ev)
+        ev.current_stream_wait()
+        want = x.float() * iw.sum(1, keepdim=True)
+        torch.testing.assert_close(out.float(), want.to(torch.bfloat16).float() + 1, rtol=2.0 ** -7, atol=2.0 ** -7)
+        assert torch.equal(out_w, w)
+        buf.check_status()
+    finally:
+        buf.destroy()
