@@ -727,3 +727,33 @@ def test_asynchronous_calls_hold_what_their_kernels_read(grouped):
         buf.check_status()
     finally:
         buf.destroy()
+
+
+def test_outgrown_scratch_is_kept_for_the_communication_stream():
+    """Scratch made by a synchronous call and used by an asynchronous one: when a larger call replaces it while the
+    communication stream still has work, the allocator may not hand the old blocks out on the caller's stream."""
+    H, E, K = 256, 8, 2
+    inputs = []
+    for T in (64, 4096):
+        (x,), (idx,), _ = _mk(1, T, H, E, K)
+        inputs.append((x.cuda(), idx.cuda()))
+    buf = _side_stream_buffer(96 << 20)
+    kw = dict(num_experts=E, group_by_expert=True, zero_copy=True)
+    pending = lambda: sum(b["state"] == "active_pending_free" for s in torch.cuda.memory_snapshot() for b in s["blocks"])
+    try:
+        (x, idx), (big, big_idx) = inputs
+        keep = [buf.get_dispatch_layout(idx, E), buf.dispatch(x, topk_idx=idx, num_worst_tokens=64 * K, **kw)]
+        torch.cuda.synchronize()
+        before = pending()
+        torch.cuda._sleep(1 << 29)                            # about a quarter of a second; the communication stream follows it
+        keep.append(buf.dispatch(x, topk_idx=idx, num_worst_tokens=64 * K, async_finish=True, **kw))
+        keep.append(buf.dispatch(big, topk_idx=big_idx, num_worst_tokens=4096 * K, async_finish=True, **kw))
+        held_back = pending()
+        keep[-1][5].current_stream_wait()
+        torch.cuda.synchronize()
+        assert held_back >= before + 2                        # item positions and chunk counts of the small call
+        rows = torch.sort(big_idx.flatten(), stable=True).indices // K
+        assert torch.equal(keep[-1][0], big[rows])
+        buf.check_status()
+    finally:
+        buf.destroy()
