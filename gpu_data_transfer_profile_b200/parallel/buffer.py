@@ -531,8 +531,11 @@ class Buffer:
         side = st["mode"] == 0 and st["topk_idx"] is not None
         n_x = 2 if st["fp8_out"] else 1
         if st["own"]:
-            # cut to the count in place: a slice would be a view, which autograd treats differently
-            views = [t if t.shape[0] == n_recv else t.resize_((n_recv, *t.shape[1:])) for t in st["own"]]
+            views = st["own"]
+            if views[0].shape[0] != n_recv:
+                # masked choices: tensors of the exact size, so that the rows nobody sent keep no memory (nor come
+                # along when a tensor is saved), at the price of the copy that leaving the region costs
+                views = self.C.clone_views([t[:n_recv] for t in views])
         else:
             views = self._region_outputs(st, carve, n_recv, side)
             if not zero_copy:

@@ -757,3 +757,28 @@ def test_outgrown_scratch_is_kept_for_the_communication_stream():
         buf.check_status()
     finally:
         buf.destroy()
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("masked", [0.0, 0.4, 1.0])
+def test_owned_outputs_hold_no_more_memory_than_their_rows(masked, grouped):
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    T, H, E, K = 300, 256, 8, 3
+    g = torch.Generator().manual_seed(0)
+    idx = torch.rand(T, E, generator=g).topk(K, dim=-1).indices
+    idx[torch.rand(T, generator=g) < masked] = -1
+    x, idx, w = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda(), idx.cuda(), torch.rand(T, K, generator=g).cuda()
+    buf = Buffer(None, 32 << 20, world=LocalWorld.make(1)[0], timeout_s=2.0)
+    try:
+        lay = {} if grouped else dict(zip(("num_tokens_per_rank", "is_token_in_rank"),
+                                          (lambda l: (l[0], l[3]))(buf.get_dispatch_layout(idx, E))))
+        for fp8 in (False, True):
+            rx, ri, rw, _, h, _ = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, group_by_expert=grouped,
+                                               use_fp8=fp8, **lay)
+            for t in [*(rx if fp8 else (rx,)), ri, rw, h.recv_prob, h.recv_meta]:
+                if t is not None:
+                    assert t.shape[0] == h.n_recv and t._base is None and t.untyped_storage().nbytes() == t.nbytes
+        buf.check_status()
+    finally:
+        buf.destroy()
