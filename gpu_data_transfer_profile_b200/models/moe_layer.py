@@ -23,9 +23,14 @@ def topk_softmax_router(logits: torch.Tensor, topk: int) -> Tuple[torch.Tensor, 
     return idx, w / w.sum(-1, keepdim=True)
 
 
+_LINEAR_FORWARD = torch.nn.Linear.forward
+
+
 def _plain_linear(m: torch.nn.Module) -> bool:
-    """Calling `m` does nothing but x @ weight.T in f32: the fused router may stand in for it."""
+    """Calling `m` does nothing but x @ weight.T in f32: the fused router may stand in for it. (Libraries that wrap
+    modules put a `forward` of their own on the instance or the class.)"""
     return (type(m) is torch.nn.Linear and m.bias is None and type(m.weight) is torch.nn.Parameter
+            and "forward" not in vars(m) and torch.nn.Linear.forward is _LINEAR_FORWARD
             and m.weight.dtype == torch.float32 and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
             and not (torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks)

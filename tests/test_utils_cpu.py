@@ -288,3 +288,27 @@ def test_clock_sample_summary_takes_the_loaded_half_and_names_reasons():
     hot = "0, 1200, 1965, 950.0, 0x40, Not Active, Active, Not Active, Not Active\n"
     assert "hw_thermal_slowdown" in parse_clock_csv(busy + hot)["reasons"]
     assert parse_clock_csv("garbage\n")["sm_mhz"] is None
+
+
+def test_fused_router_stands_in_for_an_untouched_linear_only(monkeypatch):
+    import torch
+    from gpu_data_transfer_profile_b200.models.moe_layer import _plain_linear
+    make = lambda **k: torch.nn.Linear(16, 4, bias=False, **k)
+    assert _plain_linear(make())
+    wrapped = make()
+    inner = wrapped.forward
+    wrapped.forward = lambda x: inner(x) + 1                       # how wrapping libraries attach themselves
+    assert not _plain_linear(wrapped)
+    del wrapped.forward
+    assert _plain_linear(wrapped)
+    hooked = make()
+    hook = hooked.register_forward_hook(lambda m, a, o: o + 1)
+    assert not _plain_linear(hooked)
+    hook.remove()
+    assert _plain_linear(hooked)
+    assert not _plain_linear(torch.nn.Linear(16, 4)) and not _plain_linear(make(dtype=torch.float64))
+    assert not _plain_linear(type("Sub", (torch.nn.Linear,), {})(16, 4, bias=False))
+    plain = make()
+    forward = torch.nn.Linear.forward
+    monkeypatch.setattr(torch.nn.Linear, "forward", lambda self, x: forward(self, x) + 1)
+    assert not _plain_linear(plain)
