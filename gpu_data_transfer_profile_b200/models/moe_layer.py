@@ -10,6 +10,7 @@ from __future__ import annotations
 from typing import Optional, Tuple
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from .. import _ext
 from .experts import build_experts
@@ -37,6 +38,12 @@ def _plain_linear(m: torch.nn.Module) -> bool:
             and not torch.is_autocast_enabled("cuda"))
 
 
+def _carries_more(t: Optional[torch.Tensor]) -> bool:
+    """A tensor with a forward-mode tangent or inside a function transform: the inference path, which knows nothing of
+    either, would drop what it carries without a word; the autograd functions of the general path refuse it."""
+    return t is not None and (torch._C._functorch.is_functorch_wrapped_tensor(t) or unpack_dual(t).tangent is not None)
+
+
 class MoELayer(torch.nn.Module):
     def __init__(self, hidden_size: int, ffn_hidden_size: int, num_experts: int, topk: int, group=None, *,
                  ep_size: int = 1, ep_rank: int = 0, dtype=torch.bfloat16, activation: str = "swiglu",
@@ -58,11 +65,11 @@ class MoELayer(torch.nn.Module):
         self.dispatcher = B200TokenDispatcher(group, self.num_local_experts, num_experts,
                                               ep_rank * self.num_local_experts, mode=dispatcher_mode, world=world)
 
-    def _route(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor]):
-        """(expert ids, weights). Without gradients the router runs on this library's kernels (f32 like the
-        module's own product); with them it stays the differentiable torch form."""
+    def _route(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor], inference: bool):
+        """(expert ids, weights). For inference the router runs on this library's kernels (f32 like the
+        module's own product); otherwise it stays the differentiable torch form."""
         E, K = self.num_experts, self.topk
-        C = _ext.load() if hidden_states.is_cuda and not torch.is_grad_enabled() else None
+        C = _ext.load() if hidden_states.is_cuda and inference else None
         if C is None or E > C.ROUTER_MAX_EXPERTS or K > 32 or torch.compiler.is_compiling() or torch.jit.is_tracing():
             if router_logits is None:
                 router_logits = self.router(hidden_states.float())
@@ -80,8 +87,10 @@ class MoELayer(torch.nn.Module):
 
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
         """hidden_states [T,H]; router_logits [T,E] override the learnable router when given."""
-        idx, probs = self._route(hidden_states, router_logits)
-        if (not torch.is_grad_enabled() and self.dispatcher.mode == "fused" and hidden_states.dtype == torch.bfloat16
+        inference = not (torch.is_grad_enabled() or _carries_more(hidden_states) or _carries_more(router_logits)
+                         or _carries_more(getattr(self.router, "weight", None)))
+        idx, probs = self._route(hidden_states, router_logits, inference)
+        if (inference and self.dispatcher.mode == "fused" and hidden_states.dtype == torch.bfloat16
                 and hasattr(self.experts, "forward_fused_combine") and (self.use_fp8 or self.fuse_combine)):
             # Inference: the rows are consumed where they arrive, before the next dispatch can be issued on this
             # stream, so they need no copy of their own, and the GEMMs take their tile lists from the device.

@@ -248,3 +248,41 @@ def test_exchange_backward_after_the_index_tensor_is_refilled():
         A._BUFFERS[(id(None), id(world))].check_status()
     finally:
         A.release_buffers()
+
+
+@pytest.fixture
+def small_layer():
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A
+    from gpu_data_transfer_profile_b200.models.moe_layer import MoELayer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    torch.manual_seed(0)
+    world = LocalWorld.make(1)[0]
+    A.configure_buffer(num_max_tokens_per_rank=128, num_topk=2, num_experts=4, group_by_expert=True)
+    yield lambda **kw: MoELayer(256, 128, 4, 2, None, expert_backend="tcgen05", world=world, **kw)
+    A.release_buffers()
+
+
+@pytest.mark.parametrize("where", ["input", "logits", "router", "jvp", "vmap"])
+def test_moe_layer_inference_refuses_tangents_and_transforms(small_layer, where):
+    """Nothing on the way has a forward-mode or batching rule: refused, not dropped."""
+    import torch.autograd.forward_ad as fwad
+    layer = small_layer()
+    x, logits = torch.randn(65, 256, device="cuda").to(torch.bfloat16), torch.randn(65, 4, device="cuda")
+    with torch.no_grad():
+        want = layer(x)
+        if where == "vmap":
+            with pytest.raises(RuntimeError):
+                torch.vmap(layer)(x[None])
+        elif where == "jvp":
+            with pytest.raises(RuntimeError):
+                torch.func.jvp(layer, (x,), (torch.ones_like(x),))
+        else:
+            with fwad.dual_level():
+                dual = lambda t: fwad.make_dual(t, torch.ones_like(t))
+                with pytest.raises(NotImplementedError):
+                    if where == "router":
+                        torch.func.functional_call(layer, {"router.weight": dual(layer.router.weight.detach())}, (x,))
+                    else:
+                        layer(dual(x)) if where == "input" else layer(x, dual(logits))
+                assert torch.equal(layer(x), want)           # plain tensors inside a dual level: the usual path
+        assert torch.equal(layer(x), want)
