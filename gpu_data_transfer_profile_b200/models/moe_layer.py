@@ -14,6 +14,7 @@ from torch.autograd.forward_ad import unpack_dual
 
 from .. import _ext
 from .experts import build_experts
+from .experts_tcgen05 import Tcgen05GroupedExperts
 from .token_dispatcher import B200TokenDispatcher
 
 
@@ -36,6 +37,16 @@ def _plain_linear(m: torch.nn.Module) -> bool:
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
             and not (torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks)
             and not torch.is_autocast_enabled("cuda"))
+
+
+# What `MoELayer`'s inference path stands in for or hands views and device-side counts to. Where a program subclasses,
+# wraps or replaces one of these, its own version is called as the general path calls it.
+_OWN_DISPATCHER = {n: vars(B200TokenDispatcher)[n] for n in ("dispatch", "dispatch_fp8", "dispatch_in_place")}
+_OWN_EXPERTS = {n: vars(Tcgen05GroupedExperts)[n] for n in ("forward_fused_combine", "forward_fp8")}
+
+
+def _unchanged(obj, methods) -> bool:
+    return all(n not in getattr(obj, "__dict__", ()) and getattr(type(obj), n, None) is f for n, f in methods.items())
 
 
 def _carries_more(t: Optional[torch.Tensor]) -> bool:
@@ -91,7 +102,8 @@ class MoELayer(torch.nn.Module):
                          or _carries_more(getattr(self.router, "weight", None)))
         idx, probs = self._route(hidden_states, router_logits, inference)
         if (inference and self.dispatcher.mode == "fused" and hidden_states.dtype == torch.bfloat16
-                and hasattr(self.experts, "forward_fused_combine") and (self.use_fp8 or self.fuse_combine)):
+                and (self.use_fp8 or self.fuse_combine)
+                and _unchanged(self.dispatcher, _OWN_DISPATCHER) and _unchanged(self.experts, _OWN_EXPERTS)):
             # Inference: the rows are consumed where they arrive, before the next dispatch can be issued on this
             # stream, so they need no copy of their own, and the GEMMs take their tile lists from the device.
             rows, row_probs, handle = self.dispatcher.dispatch_in_place(hidden_states, idx, probs, use_fp8=self.use_fp8)
@@ -103,6 +115,11 @@ class MoELayer(torch.nn.Module):
             buf = A.get_buffer(self.dispatcher.group, A.get_hidden_bytes(hidden_states), self.dispatcher.world)
             self.dispatcher.handle = None
             return self.experts.forward_fused_combine(rows, row_probs, buf, handle)
+        if self.use_fp8 and not torch.is_grad_enabled() and self.dispatcher.mode == "fused":
+            rows, tokens_per_expert, row_probs = self.dispatcher.dispatch_fp8(hidden_states, idx, probs)
+            El = self.num_local_experts
+            off = self.dispatcher.handle.meta[2 + El: 2 + El + El + 1]
+            return self.dispatcher.combine(self.experts.forward_fp8(rows, tokens_per_expert, row_probs, expert_off=off))
         rows, tokens_per_expert, row_probs = self.dispatcher.dispatch(hidden_states, idx, probs)
         if (self.fuse_combine and self.dispatcher.mode == "fused" and hasattr(self.experts, "forward_fused_combine")
                 and (not torch.is_grad_enabled() or self.experts.activation == "swiglu")):

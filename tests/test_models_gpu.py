@@ -286,3 +286,70 @@ def test_moe_layer_inference_refuses_tangents_and_transforms(small_layer, where)
                         layer(dual(x)) if where == "input" else layer(x, dual(logits))
                 assert torch.equal(layer(x), want)           # plain tensors inside a dual level: the usual path
         assert torch.equal(layer(x), want)
+
+
+@pytest.mark.parametrize("use_fp8", [False, True])
+def test_moe_layer_inference_calls_replaced_dispatchers_and_experts(small_layer, use_fp8, monkeypatch):
+    from gpu_data_transfer_profile_b200.models.experts_tcgen05 import Tcgen05GroupedExperts
+    from gpu_data_transfer_profile_b200.models.token_dispatcher import B200TokenDispatcher
+    layer = small_layer(use_fp8=use_fp8)
+    x = torch.randn(65, 256, device="cuda").to(torch.bfloat16)
+    name = "dispatch_fp8" if use_fp8 else "dispatch"
+    seen = []
+
+    def noted(fn):
+        def f(*a, **k):
+            seen.append(fn.__name__)
+            return fn(*a, **k)
+        return f
+
+    class Sub(B200TokenDispatcher):
+        def dispatch(self, *a):
+            seen.append("dispatch")
+            return super().dispatch(*a)
+
+        def dispatch_fp8(self, *a):
+            seen.append("dispatch_fp8")
+            return super().dispatch_fp8(*a)
+
+    class Other:                                          # a dispatcher that has nothing but what the general path calls
+        def __init__(self, d):
+            self.d, self.mode, self.group, self.world = d, d.mode, d.group, d.world
+        handle = property(lambda self: self.d.handle, lambda self, v: setattr(self.d, "handle", v))
+
+        def dispatch(self, *a):
+            seen.append("dispatch")
+            return self.d.dispatch(*a)
+
+        def dispatch_fp8(self, *a):
+            seen.append("dispatch_fp8")
+            return self.d.dispatch_fp8(*a)
+
+        def combine(self, y):
+            return self.d.combine(y)
+
+    class Experts(Tcgen05GroupedExperts):
+        def forward_fp8(self, hidden_states, tokens_per_expert, routed_probs, expert_off=None):
+            seen.append(sum(int(v) for v in tokens_per_expert))
+            return super().forward_fp8(hidden_states, tokens_per_expert, routed_probs, expert_off)
+
+        def forward_fused_combine(self, rows, routed_probs, buffer, handle):
+            seen.append(sum(handle.num_recv_tokens_per_expert_list))
+            return super().forward_fused_combine(rows, routed_probs, buffer, handle)
+
+    with torch.no_grad():
+        want = layer(x)
+        own = layer.dispatcher
+        for d in (Sub(None, 4, 4, 0, world=own.world), Other(own)):
+            layer.dispatcher = d
+            # the same rows through the same kernels; the weights come from the same router
+            assert torch.equal(layer(x), want) and seen.pop() == name and not seen
+        layer.dispatcher = own
+        setattr(own, name, noted(getattr(own, name)))                         # wrapped on the instance
+        assert torch.equal(layer(x), want) and seen.pop() == name and not seen
+        delattr(own, name)
+        with monkeypatch.context() as m:                                      # wrapped on the class
+            m.setattr(B200TokenDispatcher, name, noted(getattr(B200TokenDispatcher, name)))
+            assert torch.equal(layer(x), want) and seen.pop() == name and not seen
+        layer.experts.__class__ = Experts
+        assert torch.equal(layer(x), want) and seen.pop() == 65 * 2 and not seen
