@@ -24,7 +24,9 @@
 // smaller CTAs. Measured on one B200, before and after: push of 2047 tokens x 8 rows of 14 KiB
 // 133 -> 57 us (the slot round trip is gone) -> 49 us (rows not allocated in L1; 5.4 TB/s), push of 96
 // rows of 2 KiB 14.7 -> 3.7 us, pull of 4096 rows of 14 KiB 27.3 -> 22.8 -> 21.7 us. Tried and slower: half the
-// warps with one or two steps of loads requested ahead (58 us for the first). One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
+// warps with one or two steps of loads requested ahead (58 us for the first). What keeps the push at 5.4 TB/s (63 % of
+// the DRAM peak) is loads in flight: 64 registers a thread hold one contributor's four vectors, and the 16-bit forms
+// already spill (80 and 60 bytes of stores a thread in push and pull). One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
 // peers are launched after the halves they wait for (all announcements / sends first).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

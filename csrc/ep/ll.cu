@@ -14,16 +14,16 @@
 //    barrier when two dispatches follow each other;
 //  * no host synchronisation and no host-side state per call: the call's epoch lives in device
 //    memory and is advanced by the kernel itself, regions are double-buffered by its parity,
-//    every kernel argument is constant -> the four kernels can be captured in a CUDA graph;
+//    every kernel argument is constant -> dispatch and combine can be captured in a CUDA graph;
 //  * the receive half (bounded wait on the peers' flags, then the per-expert counts) is the last
 //    CTA's work of the send launch; with hook-style completion, and with several virtual ranks on
 //    one GPU, it is a launch of its own.
 // Bound: at decode sizes a chain of memory latencies, not bandwidth. What does not depend on
 // another rank (a token's row, its routing, the slots of a combine) is therefore requested before
 // the first wait, a group of one neither signals nor waits, and rows of the rank's own tokens are
-// combined where they lie. Measured as CUDA-graph replays on one B200 (128 tokens x 7168, top-8 of 32,
-// fp8, pull combine): 22.2 -> 12.5 us a round; an eager bf16 round trip of 7 tokens with the experts' output
-// elsewhere 40 -> 28 us, of which the kernels 22 -> 8 us.
+// combined where they lie. Measured on one B200, inputs rotated from pass to pass: a CUDA-graph replay
+// (128 tokens x 7168, top-8 of 32, fp8, pull combine) 22.5 -> 13.2 us, of which the two kernels 6.0 + 5.4 us; an eager
+// bf16 round trip of 7 tokens with the experts' output elsewhere 42 -> 28 us, host time for the most part.
 #include <cuda_bf16.h>
 #include "cast.cuh"
 #include "ep.cuh"
@@ -382,8 +382,9 @@ ll_combine_recv_kernel(LLParams P, char* self_base, const long long* __restrict_
 
 
 // ---------------------------------------------------------------------------------------
-// combine, pull form: announce, wait, load + reduce. One warp per (token, eighth of the row);
-// the rows of up to eight experts are requested together, so a token costs one NVLink round trip
+// combine, pull form: announce, wait, load + reduce. One warp per (token, part of the row), a part
+// being one batch of loads: at most 128 vectors of 16 bytes (a row of 7168 is seven parts, one of 1024 a single
+// part). The rows of up to eight experts are requested together, so a token costs one NVLink round trip
 // for eight of its choices. Lane k looks after choice k; its indices are loaded before the wait.
 // ---------------------------------------------------------------------------------------
 constexpr int kPullGroup = 8;    // contributors whose loads are in flight together

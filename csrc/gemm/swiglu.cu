@@ -106,8 +106,9 @@ act_fwd_kernel(const char* __restrict__ h, const float* __restrict__ p, char* __
 // row is a warp shuffle, plus one pass through shared memory when several warps share it.
 // Bound: memory bandwidth (5 elements moved per output element with SwiGLU, 3 without). One warp per row
 // keeps all loads of two vectors per operand in flight and needs no block barrier: with a CTA per row and two
-// barriers 12001 rows of F = 1408 took 46 us (3.7 TB/s) and 8190 of F = 2048 39 us, now 32.9
-// and 32.8 (5.1 TB/s); 16384 of F = 14336 390 -> 386 us (6.1 TB/s).
+// barriers 12001 rows of F = 1408 took 49.7 us and 8190 of F = 2048 39.4 us, now 37.3 and 35.3 (4.5 and 4.8 TB/s);
+// 16384 of F = 14336 398 -> 389 us (6.0 TB/s), 512 of it 26.1 -> 25.1 (events around the call, inputs beyond L2). The
+// gated forms of up to four warps a row spill 16 to 28 bytes a thread at the 64 registers that four CTAs per SM leave.
 // ---------------------------------------------------------------------------------------
 template <bool GATED>
 __device__ __forceinline__ float bwd_vec(const uint4& vg, const uint4& vl, const uint4& vd, float pr, int kind, uint4* og, uint4* ol) {
@@ -160,7 +161,7 @@ act_bwd_rows_kernel(const char* __restrict__ h, const float* __restrict__ p, con
       const char* d = dact + (size_t)r * F * 2;
       char* og = dh + (size_t)r * ld;
       char* ol = og + (size_t)F * 2;
-      constexpr int U = WPR == kBwdWarps ? 1 : 2, STEP = 32 * WPR;     // a CTA per row: more CTAs rather than deeper loads (512 x 14336: 16.5 -> 15.9 us)
+      constexpr int U = WPR == kBwdWarps ? 1 : 2, STEP = 32 * WPR;     // a CTA per row: more CTAs rather than deeper loads (512 x 14336, kernel alone: 16.5 -> 15.9 us)
       for (int v0 = sub * 32 + lane; v0 < nvec; v0 += U * STEP) {
         uint4 vg[U], vl[U], vd[U];
 #pragma unroll

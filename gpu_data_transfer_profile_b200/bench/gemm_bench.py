@@ -109,7 +109,7 @@ def main() -> int:
             fns["wgrad1_tcgen05" + tag] = lambda pair=pair: G.grouped_wgrad(dh, x, off, out=dw1, pair=pair)
             fns["wgrad2_tcgen05" + tag] = lambda pair=pair: G.grouped_wgrad(dy, act, off, out=dw2, pair=pair)
             flops["wgrad1_tcgen05" + tag], flops["wgrad2_tcgen05" + tag] = f1, f2
-            # data gradients: the forward weights read in place as an N-major operand
+            # data gradients: the forward weights read in place as an M-major operand
             fns["dgrad1_tcgen05" + tag] = lambda pair=pair: G.grouped_gemm(dh, w1, off, out=out, pair=pair, w_kn=True)
             fns["dgrad2_tcgen05" + tag] = lambda pair=pair: G.grouped_gemm(dy, w2, off, out=dact, pair=pair, w_kn=True)
             flops["dgrad1_tcgen05" + tag], flops["dgrad2_tcgen05" + tag] = f1, f2

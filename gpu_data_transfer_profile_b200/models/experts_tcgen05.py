@@ -3,7 +3,7 @@
 Forward: fc1 with SwiGLU x probability fused into its epilogue (one kernel), fc2 either as a
 plain grouped GEMM or with the combine send fused into its epilogue (`forward_fused_combine`).
 Tile scheduling reads the per-expert row offsets on the device. Backward (SwiGLU path): the two
-data gradients run on the same grouped GEMM reading the forward weights in place as an N-major
+data gradients run on the same grouped GEMM reading the forward weights in place as an M-major
 operand, the two weight gradients on the ragged-reduction kernel (`ops.gemm.grouped_wgrad`), the
 element-wise part on the fused SwiGLU backward kernel; no library GEMM and no host-side split.
 gelu / silu / relu (`DeepEP_Megatron/test_deepep_moe_dispatch_combine.py:516-526`) take the same
@@ -35,7 +35,7 @@ def _wgrad(dy, a, counts, out_shape, expert_off=None):
 class _GroupedMLP(torch.autograd.Function):
     """Training path. SwiGLU: fc1 (tcgen05; the epilogue applies SwiGLU x prob AND stores the
     pre-activation h for backward) -> fc2 (tcgen05). Backward: fused swiglu backward kernel, both dgrads on
-    the tcgen05 grouped GEMM (weights read in place, N-major), both wgrads on the tcgen05
+    the tcgen05 grouped GEMM (weights read in place, M-major), both wgrads on the tcgen05
     ragged-reduction kernel."""
 
     @staticmethod
