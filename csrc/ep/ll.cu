@@ -86,7 +86,7 @@ __device__ __forceinline__ LLTick ll_tick_recv(int* st) {
 // Mode 0 measured faster with 2 ranks, mode 1 with 8.
 // `elect`: also find the CTA that finishes last (its caller does the receive half); returns true in
 // that CTA. A group of one has no counters to keep: the end of the launch, or the election, orders it.
-// The CTA that completes the grid sets the local counter back to 0 for the next launch, which is ordered
+// The count of the CTA that completes the grid wraps to 0 for the next launch, which is ordered
 // after this one. (A count that runs on from launch to launch and is taken modulo the grid names a
 // CTA in the middle of the grid once a buffer has seen two grid sizes, or when it passes 2^32 with a
 // grid that does not divide it.)
@@ -101,13 +101,10 @@ __device__ __forceinline__ bool ll_arrive_on_peers(const LLParams& P, const Peer
     if (P.signal_mode != 0 || elect) {
       if (P.R == 1) __threadfence();
       else if (P.signal_mode != 0) fence_acq_rel_sys();
-      const unsigned int prev = atomicAdd(reinterpret_cast<unsigned int*>(state + 4), 1u);
-      last = prev == grid_ctas - 1u;
+      // counts up to grid_ctas - 1 and then wraps to 0
+      last = atomicInc(reinterpret_cast<unsigned int*>(state + 4), grid_ctas - 1u) == grid_ctas - 1u;
       // the last CTA acquires what the others published before they counted themselves
-      if (last) {
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        state[4] = 0;
-      }
+      if (last) asm volatile("fence.acq_rel.gpu;" ::: "memory");
     }
     s_add = P.signal_mode == 0 ? 1u : (last ? grid_ctas : 0u);
     s_last = last;
