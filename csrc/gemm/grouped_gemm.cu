@@ -352,7 +352,7 @@ grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_consta
       fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if (CG == 1) mbar_arrive(&acc_empty[buf]); else mbar_arrive_cluster(&acc_empty[buf], 0);
+        if (CG == 1) mbar_arrive(&acc_empty[buf]); else mbar_arrive_cluster_tmem(&acc_empty[buf], 0);
       }
     }
   }

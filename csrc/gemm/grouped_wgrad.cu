@@ -286,7 +286,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
       fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if (CG == 1) mbar_arrive(&acc_empty[buf]); else mbar_arrive_cluster(&acc_empty[buf], 0);
+        if (CG == 1) mbar_arrive(&acc_empty[buf]); else mbar_arrive_cluster_tmem(&acc_empty[buf], 0);
       }
     }
   }
