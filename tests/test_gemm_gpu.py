@@ -287,6 +287,27 @@ def test_tcgen05_expert_mlp_gradients_match_fp32_autograd(activation):
     torch.testing.assert_close(mod.weight2.grad.float(), w2.grad, atol=6e-2, rtol=5e-2)
 
 
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("N", [8, 128, 136, 256, 264, 384, 392])
+def test_grouped_wgrad_last_tile_columns(N, pair):
+    """Widths at which the last tile of columns is fetched 128 or 256 wide, ragged rows, empty experts, more offsets than a
+    warp has lanes, against f64: products of bf16 are exact in f32, so a result is off by its own rounding (2^-9) and by
+    f32 sums of up to 150 terms (2^-16 of their magnitudes)."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    torch.manual_seed(N)
+    M, counts = 256, [65, 0, 150, 1, 16] + [3] * 30
+    g = torch.randn(sum(counts), M, device="cuda").to(torch.bfloat16)
+    x = torch.randn(sum(counts), N, device="cuda").to(torch.bfloat16)
+    off = G.offsets_from_counts(counts, "cuda")
+    out = G.grouped_wgrad(g, x, off, pair=pair).double()
+    r = 0
+    for e, c in enumerate(counts):
+        ge, xe = g[r:r + c].double(), x[r:r + c].double()
+        ref = ge.t() @ xe
+        assert bool(((out[e] - ref).abs() <= ref.abs() * 2 ** -8 + (ge.abs().t() @ xe.abs()) * 2 ** -16).all()), e
+        r += c
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("counts,N,K", [([128], 256, 128), ([200, 0, 57], 384, 512), ([1, 300, 129, 0], 256, 1024),
                                         ([513], 128, 7168),
