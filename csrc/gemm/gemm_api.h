@@ -94,5 +94,7 @@ int router_splits(int T, int E, int H);
 int launch_router_logits(const void* x, const float* w, float* part, int splits, int T, int E, int H, cudaStream_t st);
 // Softmax over the E logits (the sum of the parts), top-K (K <= 32, E <= kRouterMaxExperts), renormalised: idx int64, prob f32 [T, K].
 int launch_router_topk(const float* part, int splits, int T, int E, int K, long long* idx, float* prob, cudaStream_t st);
+// Gradient of the logits from that of the weights: gw f32 [T, K] -> dlogits f32 [T, E].
+int launch_router_topk_bwd(const long long* idx, const float* w, const float* gw, int T, int E, int K, float* dlogits, cudaStream_t st);
 
 }  // namespace b200ep

@@ -25,6 +25,26 @@ def topk_softmax_router(logits: torch.Tensor, topk: int) -> Tuple[torch.Tensor, 
     return idx, w / w.sum(-1, keepdim=True)
 
 
+class _TopkSoftmax(torch.autograd.Function):
+    """`topk_softmax_router` on this library's kernels, one launch forward and one backward (f32 like the torch form)."""
+
+    @staticmethod
+    def forward(ctx, logits, topk):
+        idx, w = _ext.load().topk_softmax(logits, topk)
+        ctx.num_experts = logits.shape[1]
+        ctx.save_for_backward(idx, w)
+        ctx.mark_non_differentiable(idx)
+        return idx, w
+
+    @staticmethod
+    def backward(ctx, _grad_idx, grad_w):
+        idx, w = ctx.saved_tensors
+        if torch.is_grad_enabled():          # a graph of the backward is asked for
+            d = w * (grad_w - (w * grad_w).sum(-1, keepdim=True))
+            return torch.zeros((w.shape[0], ctx.num_experts), dtype=w.dtype, device=w.device).scatter(1, idx, d), None
+        return _ext.load().topk_softmax_bwd(idx, w, grad_w.float().contiguous(), ctx.num_experts), None
+
+
 _LINEAR_FORWARD = torch.nn.Linear.forward
 
 
@@ -78,13 +98,18 @@ class MoELayer(torch.nn.Module):
 
     def _route(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor], inference: bool):
         """(expert ids, weights). For inference the router runs on this library's kernels (f32 like the
-        module's own product); otherwise it stays the differentiable torch form."""
+        module's own product); for training the logits are the module's own, softmax and choice this library's."""
         E, K = self.num_experts, self.topk
         C = _ext.load() if hidden_states.is_cuda and inference else None
         if C is None or E > C.ROUTER_MAX_EXPERTS or K > 32 or torch.compiler.is_compiling() or torch.jit.is_tracing():
             if router_logits is None:
                 router_logits = self.router(hidden_states.float())
-            return topk_softmax_router(router_logits, K)
+            l = router_logits
+            if (not inference and type(l) is torch.Tensor and l.is_cuda and l.dim() == 2 and 1 <= K <= min(32, l.shape[1])
+                    and l.get_device() == torch.cuda.current_device() and l.shape[1] <= _ext.load().ROUTER_MAX_EXPERTS and not _carries_more(l)
+                    and not torch.compiler.is_compiling() and not torch.jit.is_tracing()):
+                return _TopkSoftmax.apply(l.float().contiguous(), K)
+            return topk_softmax_router(l, K)
         if router_logits is None:
             x = hidden_states
             if (type(x) is torch.Tensor and x.dtype == torch.bfloat16 and x.dim() == 2 and x.is_contiguous()

@@ -353,3 +353,40 @@ def test_moe_layer_inference_calls_replaced_dispatchers_and_experts(small_layer,
             assert torch.equal(layer(x), want) and seen.pop() == name and not seen
         layer.experts.__class__ = Experts
         assert torch.equal(layer(x), want) and seen.pop() == 65 * 2 and not seen
+
+
+@pytest.mark.parametrize("T,E,K", [(1, 1, 1), (9, 8, 2), (33, 64, 8), (7, 257, 32), (5, 1024, 3)])
+def test_training_router_matches_the_torch_form(T, E, K):
+    """Choice, renormalised weights and the logits' gradient on this library's kernels against the torch form in f64 (an
+    f32 softmax and its gradient: a few units of 2^-24 relative to values of at most one times the incoming gradient), in
+    rows with a masked expert, with not-a-number, and through a second derivative."""
+    from gpu_data_transfer_profile_b200.models.moe_layer import _TopkSoftmax, topk_softmax_router
+    gen = torch.Generator().manual_seed(T * E)
+    logits = torch.randn(T, E, generator=gen).cuda() * 3
+    if E > K:
+        logits[0, 0] = -float("inf")
+    gw = torch.randn(T, K, generator=gen).cuda()
+    l = logits.clone().requires_grad_(True)
+    idx, w = _TopkSoftmax.apply(l, K)
+    l64 = logits.double().requires_grad_(True)
+    top, idx64 = torch.topk(torch.softmax(l64, -1), K, dim=-1)
+    w64 = top / top.sum(-1, keepdim=True)
+    assert torch.equal(idx, idx64) and not idx.requires_grad
+    torch.testing.assert_close(w.double(), w64, atol=0, rtol=2 ** -19)
+    (g,) = torch.autograd.grad(w, l, gw, create_graph=True)
+    (g64,) = torch.autograd.grad(w64, l64, gw.double(), create_graph=True)
+    bound = dict(atol=2 ** -18 * float(gw.abs().max()), rtol=0)
+    torch.testing.assert_close(g.double(), g64, **bound)
+    (gg,) = torch.autograd.grad(g.square().sum(), l)
+    (gg64,) = torch.autograd.grad(g64.square().sum(), l64)
+    torch.testing.assert_close(gg.double(), gg64, atol=2 ** -16 * float(gw.abs().max()) ** 2, rtol=1e-4)
+    idx, w = _TopkSoftmax.apply(l, K)
+    (g,) = torch.autograd.grad(w, l, gw)                     # the kernel
+    torch.testing.assert_close(g.double(), g64, **bound)
+    l = logits.clone()
+    l[-1] = float("nan")
+    l.requires_grad_(True)
+    (g,) = torch.autograd.grad(_TopkSoftmax.apply(l, K)[1], l, gw)
+    lt = l.detach().clone().requires_grad_(True)
+    (gt,) = torch.autograd.grad(topk_softmax_router(lt, K)[1], lt, gw)
+    assert bool(g[-1].isnan().all()) and bool(gt[-1].isnan().all()) and not bool(g[:-1].isnan().any())
