@@ -38,6 +38,7 @@ namespace b200ep {
 constexpr int kCombWarps = 32;   // one CTA of 1024 threads per SM
 constexpr int kCUnroll = 4;
 constexpr int kRUnroll = 4;      // vectors per lane in flight per contributor when reducing
+constexpr int kOneUnroll = 8;    // ... when a token has one contributor and no running sums take registers (4096 rows of 14 KiB, pull: 24.8 -> 22.8 us on a device timeline)
 
 // ---- element helpers -------------------------------------------------------------------
 template <typename T> struct Vec16;
@@ -161,7 +162,7 @@ struct Index { int row, slot; float w; };
 
 __device__ __forceinline__ int reduce_first(int parts, int warp) { return (warp / parts) * gridDim.x + blockIdx.x; }
 
-template <typename T, typename Fetch, typename Resolve>
+template <typename T, bool ONE, typename Fetch, typename Resolve>
 __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* out, float* out_topk_w,
                                              Fetch fetch, Resolve resolve) {
   __shared__ const char* s_row[kCombWarps][kMaxItemsPerToken];
@@ -190,6 +191,25 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
     const unsigned vmask = __ballot_sync(0xffffffffu, mine != nullptr);
     __syncwarp();
     ix = fetch(t + per_round);
+    if (ONE) {                       // J == 1: nothing to sum up, the registers hold loads instead
+      const char* rowp = s_row[warp][0];
+      const float w = s_w[warp][0];
+      for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kOneUnroll) {
+        uint4 val[kOneUnroll];
+#pragma unroll
+        for (int u = 0; u < kOneUnroll; ++u)
+          if (vmask != 0 && v0 + u * 32 < v_end) val[u] = ld_global_once_v4(rowp + ((size_t)(v0 + u * 32) << 4));
+#pragma unroll
+        for (int u = 0; u < kOneUnroll; ++u) {
+          if (v0 + u * 32 >= v_end) continue;
+          float acc[Vec16<T>::N];
+#pragma unroll
+          for (int q = 0; q < Vec16<T>::N; ++q) acc[q] = 0.f;
+          if (vmask != 0) Vec16<T>::acc(acc, val[u], w);
+          st_global_v4(out + (size_t)t * row_bytes + ((size_t)(v0 + u * 32) << 4), Vec16<T>::pack(acc));
+        }
+      }
+    } else
     // kRUnroll vectors per lane and contributor are loaded together (independent loads in flight),
     // then accumulated in fp32; contributors are visited one after the other.
     for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kRUnroll) {
@@ -236,7 +256,7 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
 }
 
 // ---- push form: reduce role ----------------------------------------------------------------
-template <typename T>
+template <typename T, bool ONE>
 __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const EpRegions& rg,
                                     char* self_base, int* status) {
   __shared__ int s_ok;
@@ -284,16 +304,16 @@ __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const
     *side = comb_w + (size_t)ix.slot * wk;
     return comb + (size_t)ix.slot * row_bytes;
   };
-  reduce_items<T>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
+  reduce_items<T, ONE>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombineArgs a, int* status) {
   stream_order_wait();
   if (g.R == 1) stream_order_next();
   if (a.role != kCombineReduceOnly) combine_send_role(a, g, rg, peers, status);
-  if (a.role != kCombineSendOnly) combine_reduce_role<T>(a, g, rg, peers.base[g.rank], status);
+  if (a.role != kCombineSendOnly) combine_reduce_role<T, ONE>(a, g, rg, peers.base[g.rank], status);
 }
 
 int combine_max_ctas() {
@@ -328,15 +348,15 @@ void launch_combine(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
   const ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, a.role == kCombineReduceOnly);
   a.parts = rs.parts;
   if (dtype_code == 0)
-    launch_ordered(combine_kernel<__nv_bfloat16>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_kernel<__nv_bfloat16, true> : combine_kernel<__nv_bfloat16, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else if (dtype_code == 1)
-    launch_ordered(combine_kernel<__half>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_kernel<__half, true> : combine_kernel<__half, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else
-    launch_ordered(combine_kernel<float>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_kernel<float, true> : combine_kernel<float, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
 }
 
 // ---- pull form -----------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool ONE>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombinePullArgs a, int* status) {
   __shared__ long long s_info[kMaxRanks][4];
@@ -394,7 +414,7 @@ combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pee
     *side = reinterpret_cast<const float*>(peers.base[d] + s_info[d][1]) + (size_t)ix.row * wk;
     return peers.base[d] + s_info[d][0] + (size_t)ix.row * row_bytes;
   };
-  reduce_items<T>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
+  reduce_items<T, ONE>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
 void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
@@ -405,11 +425,11 @@ void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& p
   if (!a.pull) rs = ReduceShape{1, 1, 1};
   a.parts = rs.parts;
   if (dtype_code == 0)
-    launch_ordered(combine_pull_kernel<__nv_bfloat16>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_pull_kernel<__nv_bfloat16, true> : combine_pull_kernel<__nv_bfloat16, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else if (dtype_code == 1)
-    launch_ordered(combine_pull_kernel<__half>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_pull_kernel<__half, true> : combine_pull_kernel<__half, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
   else
-    launch_ordered(combine_pull_kernel<float>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+    launch_ordered(g.J == 1 ? combine_pull_kernel<float, true> : combine_pull_kernel<float, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
 }
 
 // Signal only (used when a fused GEMM epilogue has already stored the rows).
