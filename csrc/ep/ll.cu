@@ -16,14 +16,16 @@
 //    memory and is advanced by the kernel itself, regions are double-buffered by its parity,
 //    every kernel argument is constant -> dispatch and combine can be captured in a CUDA graph;
 //  * the receive half (bounded wait on the peers' flags, then the per-expert counts) is the last
-//    CTA's work of the send launch; with hook-style completion, and with several virtual ranks on
+//    CTA's work of the send launch (of a CTA more in a group of one, which counts the choices); with hook-style completion, and with several virtual ranks on
 //    one GPU, it is a launch of its own.
 // Bound: at decode sizes a chain of memory latencies, not bandwidth. What does not depend on
 // another rank (a token's row, its routing, the slots of a combine) is therefore requested before
 // the first wait, a group of one neither signals nor waits, and rows of the rank's own tokens are
 // combined where they lie. Measured on one B200, inputs rotated from pass to pass: a CUDA-graph replay
-// (128 tokens x 7168, top-8 of 32, fp8, pull combine) 22.5 -> 13.2 us, of which the two kernels 6.0 + 5.4 us; an eager
-// bf16 round trip of 7 tokens with the experts' output elsewhere 42 -> 28 us, host time for the most part.
+// (128 tokens x 7168, top-8 of 32, fp8, pull combine) 22.5 -> 13.1 us, then 10.3 us with the rows counted by a CTA of
+// its own, epochs committed as soon as they are read and overlapping launches in a group of one (send kernel
+// 6.3 -> 4.2 us on a device timeline); an eager bf16 round trip of 7 tokens with the experts' output elsewhere 42 -> 28 us, host
+// time for the most part.
 #include <cuda_bf16.h>
 #include "cast.cuh"
 #include "ep.cuh"
@@ -32,13 +34,16 @@
 namespace b200ep {
 
 constexpr int kLLThreads = 256;  // 8 warps work on one row together
+constexpr int kLLHistExperts = 1024;   // experts that the counting CTA of a group of one has room for
 
 // Per-op device state (6 ints): [0] committed epoch, [1] committed arrival target,
 // [2] epoch published by the send half, [3] target published by the send half,
 // [4] CTAs of the running send launch that have finished (0 between launches), [5] unused.
 // Send half: works with epoch = [0]+1, target = [1]+grid; CTA 0 publishes them in [2],[3].
 // Receive half: the CTA of the send launch that finishes last (every CTA has read [0],[1] by then)
-// commits the pair to [0],[1]; as a launch of its own it reads [2],[3] and CTA 0 commits them.
+// commits the pair to [0],[1]; as a launch of its own it reads [2],[3] and CTA 0 commits them. Where nothing but
+// that commit needs an election (combine, a group of one) the CTAs count themselves as soon as they have read the pair:
+// at the end of a kernel of 5 us the round trip of that atomic is a tenth of it.
 // No kernel ever reads a word that another CTA of the same launch writes.
 // The arrival target is a cumulative count modulo 2^32 (it grows by the grid size per call and
 // passes 2^31 after a few hours of decode steps): it is advanced in unsigned arithmetic and compared
@@ -74,6 +79,33 @@ __device__ __forceinline__ LLTick ll_tick_recv(int* st) {
   }
   __syncthreads();
   return LLTick{s_e, (unsigned int)s_t};
+}
+// Commits epoch and target once every CTA of the launch has read the old pair; called by one thread of each CTA after
+// a barrier that follows the CTA's read.
+__device__ __forceinline__ void ll_commit_when_read(int* state, int epoch, unsigned int target) {
+  if (atomicInc(reinterpret_cast<unsigned int*>(state + 4), gridDim.x - 1u) == gridDim.x - 1u) {
+    state[0] = epoch;
+    state[1] = (int)target;
+  }
+}
+// A group of one: rows per expert straight from the choices, by a CTA of its own, while the others move the rows; no CTA
+// has to find out that it is the last one. The row counters of the other parity, which nobody uses now, are made
+// ready for the next dispatch.
+__device__ __forceinline__ void ll_count_choices(const LLParams& P, char* self_base, int par,
+                                                 const long long* __restrict__ topk_idx, int* __restrict__ out_count) {
+  __shared__ int s_hist[kLLHistExperts];
+  for (int e = threadIdx.x; e < P.E; e += kLLThreads) s_hist[e] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < P.T * P.K; i += kLLThreads) {
+    const long long e = topk_idx[i];
+    if (e >= 0 && e < P.E) atomicAdd(&s_hist[(int)e], 1);
+  }
+  __syncthreads();
+  int* next = reinterpret_cast<int*>(self_base + P.count[par ^ 1]);
+  for (int e = threadIdx.x; e < P.E; e += kLLThreads) {
+    out_count[e] = min(s_hist[e], P.M);
+    next[e] = 0;
+  }
 }
 // Every CTA of a send kernel ends with this. A receiver waits for this rank's arrival counter
 // (one per peer and channel, cumulative) to reach the target, i.e. for ALL CTAs of the sender
@@ -137,6 +169,7 @@ __device__ __forceinline__ void ll_publish_counts(const LLParams& P, char* self_
     c = c < 0 ? 0 : (c > P.R * P.M ? P.R * P.M : c);
     out_count[el] = c;
     cnt[el] = 0;                 // this parity is used again two dispatches from now
+    if (P.R == 1) reinterpret_cast<int*>(self_base + P.count[par ^ 1])[el] = 0;      // (left over by ll_count_choices)
   }
 }
 
@@ -186,11 +219,21 @@ ll_dispatch_send_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, cons
     if (threadIdx.x < P.K) my_e = topk_idx[(size_t)t * P.K + threadIdx.x];
     load(t, b_first);
   };
-  ahead(blockIdx.x);
+  // a group of one that also does the receive half has one CTA more than the P.G that move rows
+  const bool counts = out_count != nullptr && (int)gridDim.x > P.G;
+  const bool counter = counts && (int)blockIdx.x == P.G;
+  if (!counter) ahead(blockIdx.x);
   if (threadIdx.x == 0) s_n = 0;
-  const LLTick tk = ll_tick_send(state, gridDim.x);
+  const LLTick tk = ll_tick_send(state, P.G);
   const int par = tk.epoch & 1;
-  for (int t = blockIdx.x; t < P.T; t += gridDim.x) {
+  if (counts) {
+    if (threadIdx.x == kLLThreads - 1) ll_commit_when_read(state, tk.epoch, tk.target);
+    if (counter) {
+      ll_count_choices(P, peers.base[P.rank], par, topk_idx, out_count);
+      return;
+    }
+  }
+  for (int t = blockIdx.x; t < P.T; t += P.G) {
     if (threadIdx.x < P.K) {
       const long long e = my_e;
       int given = -1;
@@ -241,14 +284,14 @@ ll_dispatch_send_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, cons
             for (int j = 0; j < n; ++j) st_global_v4(s_dst[j] + ((size_t)(b + u * kLLThreads) << 4), r[u]);
       }
     }
-    if (t + (int)gridDim.x < P.T) {
-      ahead(t + gridDim.x);
+    if (t + P.G < P.T) {
+      ahead(t + P.G);
       __syncthreads();                       // everybody has read s_n and the destinations
       if (threadIdx.x == 0) s_n = 0;
       __syncthreads();
     }
   }
-  if (ll_arrive_on_peers(P, peers, kChLLDispatch, state, gridDim.x, out_count != nullptr)) {
+  if (!counts && ll_arrive_on_peers(P, peers, kChLLDispatch, state, gridDim.x, out_count != nullptr)) {
     ll_publish_counts(P, peers.base[P.rank], tk, out_count, status);
     if (threadIdx.x == 0) { state[0] = tk.epoch; state[1] = (int)tk.target; }
   }
@@ -440,6 +483,7 @@ ll_combine_pull_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, int p
     }
   }
   if (phase == 1) return;
+  if (threadIdx.x == kLLThreads - 1) ll_commit_when_read(state, epoch, target);
   if (P.R > 1) {
     if ((int)threadIdx.x < P.R) {
       const int* flags = reinterpret_cast<const int*>(self_base + P.flags) + kChLLPull * kMaxRanks;
@@ -510,16 +554,6 @@ ll_combine_pull_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, int p
       }
     }
   }
-  // the CTA that finishes last commits the epoch (every CTA has read the old one by then)
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned int prev = atomicAdd(reinterpret_cast<unsigned int*>(state + 4), 1u);
-    if (prev == gridDim.x - 1) {
-      state[4] = 0;
-      state[0] = epoch;
-      state[1] = (int)target;
-    }
-  }
 }
 
 // ---- launchers -------------------------------------------------------------------------
@@ -542,7 +576,8 @@ static void ll_launch(void (*kern)(KArgs...), dim3 grid, bool pdl, cudaStream_t 
 void launch_ll_dispatch_send(const LLParams& P, const PeerPtrs& peers, const char* x,
                              const long long* topk_idx, int* state, int* status,
                              cudaStream_t st, int* send_slot, int* out_count) {
-  ll_launch(ll_dispatch_send_kernel, dim3(P.G), P.pdl != 0, st, P, peers, x, topk_idx, state, status, send_slot, out_count);
+  const bool counts = P.R == 1 && out_count != nullptr && P.E <= kLLHistExperts;
+  ll_launch(ll_dispatch_send_kernel, dim3(P.G + (counts ? 1 : 0)), P.pdl != 0, st, P, peers, x, topk_idx, state, status, send_slot, out_count);
 }
 void launch_ll_dispatch_recv(const LLParams& P, char* self_base, int* out_count, int* state, int* status,
                              cudaStream_t st) {

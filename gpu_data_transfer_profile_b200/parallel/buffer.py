@@ -752,8 +752,9 @@ class Buffer:
     # are placed while its predecessor still runs and wait in their first instruction until it has
     # completed, so launch latencies overlap (also inside a captured CUDA graph). On one GPU a replay of
     # 128 fp8 tokens takes 12.3 us either way, of 128 bf16 tokens 14.3 -> 13.9, of one token 11.5 -> 10.3, an eager
-    # round 27.2 -> 26.3 us (one set of inputs, back to back). Off by default because of the last measurement
-    # with 2 ranks, taken while the receive half was a launch of its own: eager dispatch got slower there (45 -> 54 us).
+    # round 27.2 -> 26.3 us (one set of inputs, back to back). A group of one always does so. Off by default for others
+    # because of the last measurement with 2 ranks, taken while the receive half was a launch of its own: eager
+    # dispatch got slower there (45 -> 54 us).
     ll_overlap_launches: bool = False
 
     def _ll_state(self, E: int, K: int, H: int, M: int):
@@ -787,7 +788,7 @@ class Buffer:
         return [self.rank, R, E, El, K, H, M, T, int(fp8), 0, *c.count, *c.recv_x, *c.recv_scales,
                 *c.recv_src, *c.comb_x, self._timeout_ns(), *c.recv_tag, min(M, 128), El * Buffer.LL_SPLIT,
                 (1 if R >= 8 else 0) if Buffer.ll_signal_mode is None else int(Buffer.ll_signal_mode),
-                int(bool(Buffer.ll_overlap_launches)), c.comb_in, *c.range_tab]
+                int(bool(Buffer.ll_overlap_launches) or R == 1), c.comb_in, *c.range_tab]
 
     def _ll_dispatch_send(self, x, topk_idx, M, E, use_fp8, fused=False):
         """fused: the same launch also does the receive half (its last CTA waits for the peers)."""

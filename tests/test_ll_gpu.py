@@ -273,3 +273,34 @@ def test_low_latency_token_bound_changes_on_one_buffer(signal_mode, in_place, mo
         buf.check_status()
     finally:
         buf.destroy()
+
+
+@pytest.mark.parametrize("E,M", [(8, 160), (1024, 9), (1032, 9)])
+def test_low_latency_counts_of_a_group_of_one(E, M):
+    """A group of one counts rows from the choices in a CTA of its own (up to 1024 experts; more take the counters)
+    and readies the other parity's row counters: calls that do and calls with a hook in any order, no tokens, one,
+    more tokens than CTAs that move rows, masked choices. Rows per expert and the combined rows are exact."""
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.local import LocalGroup
+    H, K = 256, 4
+    g = LocalGroup(1, Buffer.get_low_latency_nvl_size_hint(M, H, 1, E, K), timeout_s=2.0)
+    try:
+        b = g.buffers[0]
+        gen = torch.Generator().manual_seed(E)
+        for rep, (hooked, T) in enumerate([(0, M), (1, M), (1, 3), (0, 1), (0, 0), (0, M), (1, 1), (0, M - 1), (0, M), (1, M), (0, M)]):
+            x = torch.randn(T, H, generator=gen).to(torch.bfloat16).cuda()
+            idx = torch.stack([torch.randperm(E, generator=gen)[:K] for _ in range(T)]) if T else torch.zeros(0, K, dtype=torch.int64)
+            idx[torch.rand(idx.shape, generator=gen) < 0.2] = -1
+            idx, keep = idx.cuda(), (idx >= 0)
+            if hooked:
+                *_, hook = b.low_latency_dispatch(x, idx, M, E, use_fp8=False, return_recv_hook=True)
+                recv, count, handle = hook()
+            else:
+                recv, count, handle, _, _ = b.low_latency_dispatch(x, idx, M, E, use_fp8=False)
+            want = torch.bincount(idx[idx >= 0].cpu(), minlength=E)
+            assert torch.equal(count.cpu().long(), want), (rep, hooked, T)
+            out, _, _ = b.low_latency_combine(recv, idx, torch.ones(T, K, device="cuda"), handle)
+            assert torch.equal(out, (x.float() * keep.sum(1, keepdim=True).cuda()).to(torch.bfloat16)), (rep, hooked, T)
+        g.check_status()
+    finally:
+        g.destroy()
