@@ -775,9 +775,12 @@ class Buffer:
                 # device-resident op state (epochs and arrival targets); lives as long as the buffer
                 # because the peers' arrival counters are cumulative
                 self._ll_words = torch.zeros(18, dtype=torch.int32, device=dev)
-            self._ll = dict(key=key, carve=carve, words=self._ll_words,
-                            send_slot=torch.full((M * K,), -1, dtype=torch.int32, device=dev))
-            self._carve = None
+            ll = dict(key=key, carve=carve, words=self._ll_words,
+                      send_slot=torch.full((M * K,), -1, dtype=torch.int32, device=dev))
+            self._ll = self._carve = None          # (whatever lay in the region is gone, also if the shape is refused)
+            ll["ctx"] = self.C.LLContext(self._ll_params(ll, 0, False), self.peers, self._ll_words, ll["send_slot"],
+                                         self.status_ptr)
+            self._ll = ll
         return self._ll
 
     def _ll_params(self, st, T: int, fp8: bool):
@@ -787,8 +790,13 @@ class Buffer:
         El = E // R
         return [self.rank, R, E, El, K, H, M, T, int(fp8), 0, *c.count, *c.recv_x, *c.recv_scales,
                 *c.recv_src, *c.comb_x, self._timeout_ns(), *c.recv_tag, min(M, 128), El * Buffer.LL_SPLIT,
-                (1 if R >= 8 else 0) if Buffer.ll_signal_mode is None else int(Buffer.ll_signal_mode),
-                int(bool(Buffer.ll_overlap_launches) or R == 1), c.comb_in, *c.range_tab]
+                self._ll_signal(), int(self._ll_overlap()), c.comb_in, *c.range_tab]
+
+    def _ll_signal(self) -> int:
+        return (1 if self.group_size >= 8 else 0) if Buffer.ll_signal_mode is None else int(Buffer.ll_signal_mode)
+
+    def _ll_overlap(self) -> bool:
+        return bool(Buffer.ll_overlap_launches) or self.group_size == 1
 
     def _ll_dispatch_send(self, x, topk_idx, M, E, use_fp8, fused=False):
         """fused: the same launch also does the receive half (its last CTA waits for the peers)."""
@@ -807,10 +815,8 @@ class Buffer:
             # peer has consumed the previous one. A combine in between proves that; without one, drain.
             self.barrier()
         self._ll_dispatch_pending = True
-        pv = self._ll_params(st, T, use_fp8)
-        count = torch.empty((E // self.group_size,), dtype=torch.int32, device=self.device) if fused else None
-        self.C.ll_dispatch_send(pv, self.peers, x, topk_idx, st["words"][0:6], self.status_ptr, st["send_slot"], count)
-        return dict(st=st, pv=pv, T=T, H=H, K=K, E=E, M=M, fp8=use_fp8, topk_idx=topk_idx, x=x, count=count)
+        count = st["ctx"].dispatch(x, topk_idx, bool(use_fp8), fused, self._timeout_ns(), self._ll_signal(), self._ll_overlap())
+        return dict(st=st, T=T, H=H, K=K, E=E, M=M, fp8=use_fp8, topk_idx=topk_idx, x=x, count=count)
 
     def _ll_dispatch_recv(self, d):
         """Count-only: the rows already lie packed per local expert in the receive region, which is
@@ -821,7 +827,7 @@ class Buffer:
         out_count = d["count"]
         if out_count is None:
             out_count = torch.empty((El,), dtype=torch.int32, device=self.device)
-            self.C.ll_dispatch_recv(d["pv"], self.region.local_ptr, out_count, d["st"]["words"][0:6], self.status_ptr)
+            self.C.ll_dispatch_recv(self._ll_params(d["st"], d["T"], d["fp8"]), self.region.local_ptr, out_count, d["st"]["words"][0:6], self.status_ptr)
         if d["fp8"]:
             out_x = (self.region.view(c.recv_x[0], (El, rows, H), "float8_e4m3fn"),
                      self.region.view(c.recv_scales[0], (El, rows, H // 128), "float32"))
@@ -876,14 +882,8 @@ class Buffer:
             self._ll_dispatch_pending = False
         st = self._ll_state(E, K, H, M)
         topk_idx = topk_idx.to(torch.int64).contiguous()
-        T = topk_idx.shape[0]
-        pv = self._ll_params(st, T, False)
-        if out is None:
-            out = torch.empty((T, H), dtype=torch.bfloat16, device=self.device)
         w = topk_weights.to(torch.float32).contiguous() if topk_weights is not None else None
-        self.C.ll_combine_pull(pv, self.peers, phase, st["send_slot"], topk_idx, w, out,
-                               st["words"][12:18], self.status_ptr, own_x)
-        return out
+        return st["ctx"].combine_pull(phase, topk_idx, w, out, own_x, self._timeout_ns(), self._ll_signal(), self._ll_overlap())
 
     def _ll_is_combine_buffer(self, x, handle) -> bool:
         if self._ll is None:
