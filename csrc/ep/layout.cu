@@ -243,7 +243,10 @@ __device__ __forceinline__ void notify_publish(const EpGeom& g, const EpRegions&
   if (threadIdx.x < R) {
     int* flag = reinterpret_cast<int*>(peers.base[threadIdx.x] + rg.flags) +
                 kChNotify * kMaxRanks + g.rank;
-    st_release_sys(flag, g.epoch);
+    // (a group of one has nobody who waits; the end of the launch orders the counts for what follows. The release
+    // cost 4 us of 10: 2047 tokens, top-8 of 64, device timeline of one B200)
+    if (R == 1) st_relaxed_sys(flag, g.epoch);
+    else st_release_sys(flag, g.epoch);
   }
 }
 
