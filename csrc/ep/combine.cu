@@ -24,10 +24,10 @@
 // smaller CTAs. Measured on one B200, before and after: push of 2047 tokens x 8 rows of 14 KiB
 // 133 -> 57 us (the slot round trip is gone) -> 49 us (rows not allocated in L1; 5.4 TB/s), push of 96
 // rows of 2 KiB 14.7 -> 3.7 us, pull of 4096 rows of 14 KiB 27.3 -> 22.8 -> 21.7 us. Tried and slower: half the
-// warps with one or two steps of loads requested ahead (58 us for the first). What keeps the push at 5.4 TB/s (63 % of
-// the DRAM peak) is loads in flight: 64 registers a thread hold one contributor's four vectors, and the 16-bit forms
-// already spill (80 and 60 bytes of stores a thread in push and pull). One CTA of up to 1024 threads per SM. With several virtual ranks on one GPU the halves that wait for
-// peers are launched after the halves they wait for (all announcements / sends first).
+// warps with one or two steps of loads requested ahead (58 us for the first), rows brought to a ring in shared memory by bulk
+// copies (55). Twice the loads in flight leave the push at 49 us: with the 117 MB that the dispatch before it left to be
+// written back it is HBM that bounds it. One CTA of up to 1024 threads per SM. With several virtual ranks on one
+// GPU the halves that wait for peers are launched after the halves they wait for (all announcements / sends first).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "ep.cuh"
@@ -37,8 +37,16 @@ namespace b200ep {
 
 constexpr int kCombWarps = 32;   // one CTA of 1024 threads per SM
 constexpr int kCUnroll = 4;
-constexpr int kRUnroll = 4;      // vectors per lane in flight per contributor when reducing
-constexpr int kOneUnroll = 8;    // ... when a token has one contributor and no running sums take registers (4096 rows of 14 KiB, pull: 24.8 -> 22.8 us on a device timeline)
+// Loads that a lane has in flight in a reduction, and the running sums that go with them, as a token's contributors J
+// allow: U vectors of each of G contributors, 64 registers a thread in all. One contributor needs no sums (4096 rows of
+// 14 KiB, pull: 24.8 -> 22.8 us on a device timeline); eight rows of a vector at a time need the sums of that vector only (1024
+// tokens x 8 rows of 4 KiB: 10.7 -> 8.5 us; 2047 x 8 of 14 KiB stay at 49, HBM with what the dispatch left to be written back).
+template <int FORM> struct Batch;
+template <> struct Batch<0> { static constexpr int U = 4, G = 1; };     // J == 2
+template <> struct Batch<1> { static constexpr int U = 8, G = 1; };     // J == 1
+template <> struct Batch<2> { static constexpr int U = 2, G = 4; };     // J == 3, 4
+template <> struct Batch<3> { static constexpr int U = 1, G = 8; };     // J >= 5
+static int batch_form(int J) { return J == 1 ? 1 : J == 2 ? 0 : J <= 4 ? 2 : 3; }
 
 // ---- element helpers -------------------------------------------------------------------
 template <typename T> struct Vec16;
@@ -162,7 +170,7 @@ struct Index { int row, slot; float w; };
 
 __device__ __forceinline__ int reduce_first(int parts, int warp) { return (warp / parts) * gridDim.x + blockIdx.x; }
 
-template <typename T, bool ONE, typename Fetch, typename Resolve>
+template <typename T, int FORM, typename Fetch, typename Resolve>
 __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* out, float* out_topk_w,
                                              Fetch fetch, Resolve resolve) {
   __shared__ const char* s_row[kCombWarps][kMaxItemsPerToken];
@@ -182,58 +190,66 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
   for (; t < g.T; t += per_round) {
     const float* side = nullptr;
     const char* mine = nullptr;
-    if (lane < J) {
-      mine = resolve(t, ix, &side);
-      s_row[warp][lane] = mine;
-      s_side[warp][lane] = side;
-      s_w[warp][lane] = ix.w;
-    }
+    if (lane < J) mine = resolve(t, ix, &side);
+    // the contributors that there are, closed up in ascending order
     const unsigned vmask = __ballot_sync(0xffffffffu, mine != nullptr);
+    const int n = __popc(vmask);
+    if (mine != nullptr) {
+      const int at = __popc(vmask & ((1u << lane) - 1u));
+      s_row[warp][at] = mine;
+      s_side[warp][at] = side;
+      s_w[warp][at] = ix.w;
+    }
     __syncwarp();
     ix = fetch(t + per_round);
-    if (ONE) {                       // J == 1: nothing to sum up, the registers hold loads instead
-      const char* rowp = s_row[warp][0];
-      const float w = s_w[warp][0];
-      for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kOneUnroll) {
-        uint4 val[kOneUnroll];
+    constexpr int U = Batch<FORM>::U, G = Batch<FORM>::G, N = Vec16<T>::N;
+    for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * U) {
+      if (FORM == 1) {
+        uint4 val[U];
+        const char* rowp = s_row[warp][0];
+        const float w = s_w[warp][0];
 #pragma unroll
-        for (int u = 0; u < kOneUnroll; ++u)
-          if (vmask != 0 && v0 + u * 32 < v_end) val[u] = ld_global_once_v4(rowp + ((size_t)(v0 + u * 32) << 4));
+        for (int u = 0; u < U; ++u)
+          if (n != 0 && v0 + u * 32 < v_end) val[u] = ld_global_once_v4(rowp + ((size_t)(v0 + u * 32) << 4));
 #pragma unroll
-        for (int u = 0; u < kOneUnroll; ++u) {
+        for (int u = 0; u < U; ++u) {
           if (v0 + u * 32 >= v_end) continue;
-          float acc[Vec16<T>::N];
+          float acc[N];
 #pragma unroll
-          for (int q = 0; q < Vec16<T>::N; ++q) acc[q] = 0.f;
-          if (vmask != 0) Vec16<T>::acc(acc, val[u], w);
+          for (int q = 0; q < N; ++q) acc[q] = 0.f;
+          if (n != 0) Vec16<T>::acc(acc, val[u], w);
           st_global_v4(out + (size_t)t * row_bytes + ((size_t)(v0 + u * 32) << 4), Vec16<T>::pack(acc));
         }
+        continue;
       }
-    } else
-    // kRUnroll vectors per lane and contributor are loaded together (independent loads in flight),
-    // then accumulated in fp32; contributors are visited one after the other.
-    for (int v0 = part * part_vec + lane; v0 < v_end; v0 += 32 * kRUnroll) {
-      float acc[kRUnroll][Vec16<T>::N];
+      float acc[U][N];
 #pragma unroll
-      for (int u = 0; u < kRUnroll; ++u)
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int q = 0; q < Vec16<T>::N; ++q) acc[u][q] = 0.f;
-      for (unsigned mm = vmask; mm; mm &= mm - 1) {
-        const int j = __ffs(mm) - 1;
-        const char* rowp = s_row[warp][j];
-        const float wj = s_w[warp][j];
-        uint4 val[kRUnroll];
+        for (int q = 0; q < N; ++q) acc[u][q] = 0.f;
+      for (int k0 = 0; k0 < n; k0 += G) {
+        uint4 val[G][U];
 #pragma unroll
-        for (int u = 0; u < kRUnroll; ++u) {
-          const int v = v0 + u * 32;
-          if (v < v_end) val[u] = ld_global_once_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU may have written it
+        for (int c = 0; c < G; ++c) {
+          if (k0 + c >= n) continue;
+          const char* rowp = s_row[warp][k0 + c];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int v = v0 + u * 32;
+            if (v < v_end) val[c][u] = ld_global_once_v4(rowp + ((size_t)v << 4));   // coherent path: another GPU may have written it
+          }
         }
 #pragma unroll
-        for (int u = 0; u < kRUnroll; ++u)
-          if (v0 + u * 32 < v_end) Vec16<T>::acc(acc[u], val[u], wj);
+        for (int c = 0; c < G; ++c) {
+          if (k0 + c >= n) continue;
+          const float w = s_w[warp][k0 + c];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (v0 + u * 32 < v_end) Vec16<T>::acc(acc[u], val[c][u], w);
+        }
       }
 #pragma unroll
-      for (int u = 0; u < kRUnroll; ++u) {
+      for (int u = 0; u < U; ++u) {
         const int v = v0 + u * 32;
         if (v < v_end) st_global_v4(out + (size_t)t * row_bytes + ((size_t)v << 4), Vec16<T>::pack(acc[u]));
       }
@@ -243,7 +259,7 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
         // rank mode: [T,K] = sum over destination ranks of the K side values of each row
         if (lane < g.K) {
           float s = 0.f;
-          for (unsigned mm = vmask; mm; mm &= mm - 1) s += s_side[warp][__ffs(mm) - 1][lane];
+          for (int k = 0; k < n; ++k) s += s_side[warp][k][lane];
           out_topk_w[(size_t)t * g.K + lane] = s;
         }
       } else if (lane < J) {
@@ -256,7 +272,7 @@ __device__ __forceinline__ void reduce_items(const EpGeom& g, int parts, char* o
 }
 
 // ---- push form: reduce role ----------------------------------------------------------------
-template <typename T, bool ONE>
+template <typename T, int FORM>
 __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const EpRegions& rg,
                                     char* self_base, int* status) {
   __shared__ int s_ok;
@@ -304,16 +320,16 @@ __device__ void combine_reduce_role(const CombineArgs& a, const EpGeom& g, const
     *side = comb_w + (size_t)ix.slot * wk;
     return comb + (size_t)ix.slot * row_bytes;
   };
-  reduce_items<T, ONE>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
+  reduce_items<T, FORM>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
-template <typename T, bool ONE>
+template <typename T, int FORM>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombineArgs a, int* status) {
   stream_order_wait();
   if (g.R == 1) stream_order_next();
   if (a.role != kCombineReduceOnly) combine_send_role(a, g, rg, peers, status);
-  if (a.role != kCombineSendOnly) combine_reduce_role<T, ONE>(a, g, rg, peers.base[g.rank], status);
+  if (a.role != kCombineSendOnly) combine_reduce_role<T, FORM>(a, g, rg, peers.base[g.rank], status);
 }
 
 int combine_max_ctas() {
@@ -347,16 +363,17 @@ void launch_combine(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
   if (g.R == 1 && a.send_row != nullptr && a.role == kCombineBoth) { a.role = kCombineReduceOnly; a.wait = 0; }
   const ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, a.role == kCombineReduceOnly);
   a.parts = rs.parts;
-  if (dtype_code == 0)
-    launch_ordered(g.J == 1 ? combine_kernel<__nv_bfloat16, true> : combine_kernel<__nv_bfloat16, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
-  else if (dtype_code == 1)
-    launch_ordered(g.J == 1 ? combine_kernel<__half, true> : combine_kernel<__half, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
-  else
-    launch_ordered(g.J == 1 ? combine_kernel<float, true> : combine_kernel<float, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+  auto go = [&](auto... forms) {
+    decltype(&combine_kernel<float, 0>) all[] = {forms...};
+    launch_ordered(all[batch_form(g.J)], rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+  };
+  if (dtype_code == 0) go(combine_kernel<__nv_bfloat16, 0>, combine_kernel<__nv_bfloat16, 1>, combine_kernel<__nv_bfloat16, 2>, combine_kernel<__nv_bfloat16, 3>);
+  else if (dtype_code == 1) go(combine_kernel<__half, 0>, combine_kernel<__half, 1>, combine_kernel<__half, 2>, combine_kernel<__half, 3>);
+  else go(combine_kernel<float, 0>, combine_kernel<float, 1>, combine_kernel<float, 2>, combine_kernel<float, 3>);
 }
 
 // ---- pull form -----------------------------------------------------------------------------
-template <typename T, bool ONE>
+template <typename T, int FORM>
 __global__ void __launch_bounds__(kCombWarps * 32, 1)
 combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs peers, CombinePullArgs a, int* status) {
   __shared__ long long s_info[kMaxRanks][4];
@@ -414,7 +431,7 @@ combine_pull_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pee
     *side = reinterpret_cast<const float*>(peers.base[d] + s_info[d][1]) + (size_t)ix.row * wk;
     return peers.base[d] + s_info[d][0] + (size_t)ix.row * row_bytes;
   };
-  reduce_items<T, ONE>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
+  reduce_items<T, FORM>(g, a.parts, a.out, a.out_topk_w, fetch, resolve);
 }
 
 void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
@@ -424,12 +441,13 @@ void launch_combine_pull(const EpGeom& g, const EpRegions& rg, const PeerPtrs& p
   ReduceShape rs = reduce_shape(g.T, g.H * (dtype_code == 2 ? 4 : 2), blocks, true);
   if (!a.pull) rs = ReduceShape{1, 1, 1};
   a.parts = rs.parts;
-  if (dtype_code == 0)
-    launch_ordered(g.J == 1 ? combine_pull_kernel<__nv_bfloat16, true> : combine_pull_kernel<__nv_bfloat16, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
-  else if (dtype_code == 1)
-    launch_ordered(g.J == 1 ? combine_pull_kernel<__half, true> : combine_pull_kernel<__half, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
-  else
-    launch_ordered(g.J == 1 ? combine_pull_kernel<float, true> : combine_pull_kernel<float, false>, rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+  auto go = [&](auto... forms) {
+    decltype(&combine_pull_kernel<float, 0>) all[] = {forms...};
+    launch_ordered(all[batch_form(g.J)], rs.blocks, rs.warps * 32, 0, st, 1, g, rg, peers, a, status);
+  };
+  if (dtype_code == 0) go(combine_pull_kernel<__nv_bfloat16, 0>, combine_pull_kernel<__nv_bfloat16, 1>, combine_pull_kernel<__nv_bfloat16, 2>, combine_pull_kernel<__nv_bfloat16, 3>);
+  else if (dtype_code == 1) go(combine_pull_kernel<__half, 0>, combine_pull_kernel<__half, 1>, combine_pull_kernel<__half, 2>, combine_pull_kernel<__half, 3>);
+  else go(combine_pull_kernel<float, 0>, combine_pull_kernel<float, 1>, combine_pull_kernel<float, 2>, combine_pull_kernel<float, 3>);
 }
 
 // Signal only (used when a fused GEMM epilogue has already stored the rows).
