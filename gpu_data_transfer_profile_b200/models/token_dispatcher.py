@@ -20,7 +20,11 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..parallel.buffer import Buffer
 from . import fused_a2a as A
+
+# a program that replaces or wraps `Buffer.dispatch` has its own called
+_BUFFER_DISPATCH = vars(Buffer)["dispatch"]
 
 
 class B200TokenDispatcher:
@@ -135,12 +139,17 @@ class B200TokenDispatcher:
             items = idx.numel()
             # (a region too small for them takes the counted path, which names the overflow)
             worst = items if 0 < items <= buf._get_carve(self.num_experts, K, H, H * 2, H * 2).cap else 0
-        rows, _, _, _, handle, _ = buf.dispatch(
-            x, topk_idx=idx, topk_weights=token_probs.contiguous().float(), group_by_expert=True,
-            num_experts=self.num_experts, use_fp8=use_fp8, zero_copy=True, num_worst_tokens=worst)
         El = self.num_local_experts
-        # (what callers may look at later is their own; the rows' view above is for the computation)
-        self.handle, self.dispatched_probs = handle, buf.C.clone_views([handle.recv_prob])[0]
+        weights = token_probs.contiguous().float()
+        # (what callers may look at later is their own; the rows' view is for the computation)
+        if worst and getattr(type(buf), "dispatch", None) is _BUFFER_DISPATCH and "dispatch" not in vars(buf):
+            rows, handle = buf._dispatch_own_probs(x, idx, weights, self.num_experts, use_fp8, worst)
+            self.handle, self.dispatched_probs = handle, handle.recv_prob
+        else:
+            rows, _, _, _, handle, _ = buf.dispatch(
+                x, topk_idx=idx, topk_weights=weights, group_by_expert=True,
+                num_experts=self.num_experts, use_fp8=use_fp8, zero_copy=True, num_worst_tokens=worst)
+            self.handle, self.dispatched_probs = handle, buf.C.clone_views([handle.recv_prob])[0]
         self.tokens_per_expert = handle.meta[2:2 + El]
         return rows, handle.recv_prob, handle
 

@@ -481,7 +481,7 @@ class Buffer:
             mode, T, st["epoch_n"], self._timeout_ns(), st.get("is_token_in_rank"), st["topk_idx"], per_expert)
         return st
 
-    def _dispatch_p2(self, st, zero_copy: bool = True, num_worst_tokens: int = 0):
+    def _dispatch_p2(self, st, zero_copy: bool = True, num_worst_tokens: int = 0, own_probs: int = 0):
         """The send kernel. One process per GPU: its last CTA also waits for the peers, so the
         receive region is complete when the kernel ends. Virtual ranks on one GPU: the wait is a
         separate launch (`_dispatch_p3`) issued after every rank's send. In a group of one the rows that a
@@ -496,9 +496,9 @@ class Buffer:
             own = min(max(items, st["handle"].n_recv if st["cached"] else 0), st["carve"].cap)
         st["own"] = self._ctx.send(st["mode"], st["epoch_d"], st.get("epoch_n", 0), self._single_launch, self._timeout_ns(), self._blocks(),
                        st["meta"], st["x"], st["fp8"], st["cached"], st["topk_idx"], st.get("topk_weights"), st["send_row"],
-                       st["send_slot"], st["scales_in"], own, st.get("is_token_in_rank"), st.get("per_expert"))
+                       st["send_slot"], st["scales_in"], own, st.get("is_token_in_rank"), st.get("per_expert"), own_probs)
 
-    def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1):
+    def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1, own_probs: int = 0):
         R, E, K, H = self.group_size, st["E"], st["K"], st["H"]
         El = E // R
         carve = st["carve"]
@@ -531,7 +531,10 @@ class Buffer:
             self._poll_status()       # the host already waited for the kernel's prologue: cheap to look
         side = st["mode"] == 0 and st["topk_idx"] is not None
         n_x = 2 if st["fp8_out"] else 1
-        if st["own"]:
+        if own_probs:
+            views = self._region_outputs(st, carve, n_recv, side)
+            views[n_x] = st["own"][0]
+        elif st["own"]:
             views = st["own"]
             if views[0].shape[0] != n_recv:
                 # masked choices: tensors of the exact size, so that the rows nobody sent keep no memory (nor come
@@ -606,6 +609,17 @@ class Buffer:
         ev = self._exit(compute, async_finish, [t for t in flat if t is not None] + [x],
                         [t for t in st.values() if isinstance(t, torch.Tensor)])
         return (*out, ev)
+
+    @_nvtx("b200ep.dispatch")
+    def _dispatch_own_probs(self, x, topk_idx, topk_weights, num_experts: int, use_fp8: bool, rows: int):
+        """A group of one, expert mode: `rows` rows (the number of choices) in the region, their probabilities in a tensor
+        of the caller's own. -> (recv_x | (recv_x_fp8, scales), handle)"""
+        self._enter(None, False, False)
+        with self._on_stream():
+            st = self._dispatch_p1(x, None, None, None, topk_idx, topk_weights, use_fp8, True, num_experts)
+            self._dispatch_p2(st, True, rows, rows)
+            recv_x, _, _, _, handle = self._dispatch_p3(st, True, rows, 1, rows)
+        return recv_x, handle
 
     # ---- combine ---------------------------------------------------------------------
     def _combine_prepare(self, x, handle: DispatchHandle, topk_weights):
