@@ -30,17 +30,12 @@ void launch_barrier(const PeerPtrs& peers, long long flags_off, int rank, int R,
 // g.tail_wait = 1 makes the last CTA wait for the peers' dispatch flags (never with several
 // virtual ranks on one GPU: use launch_wait_flags on the dispatch channel after all ranks' sends).
 // host_word: mapped pinned ints [0]=notify epoch served, [1]=N_recv, [2..2+El) per-expert counts.
-// Rank mode in a group of one, up to kOwnCountTokens tokens: the send kernel counts from own_flags (is_token_in_rank)
-// itself and no launch_notify_send goes before it. (The flags are read by every CTA: 16 KiB each at the bound.)
-constexpr int kOwnCountTokens = 16384;
-inline bool dispatch_counts_itself(int mode, int R, long long T) { return mode == 0 && R == 1 && T > 0 && T <= kOwnCountTokens; }
 void launch_dispatch_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                           const EpMeta& m, const char* x, int row_bytes_in, bool fp8, bool cached,
                           const long long* topk_idx, const float* topk_w, const int* item_rank,
                           const int* chunk_base, int* send_row, int* send_slot,
                           unsigned int* block_counter, int* host_word, int* status, int blocks,
-                          cudaStream_t st, const float* scales_in = nullptr,
-                          const bool* own_flags = nullptr, const int* own_per_expert = nullptr);
+                          cudaStream_t st, const float* scales_in = nullptr);
 
 enum CombineRole : int { kCombineBoth = 0, kCombineSendOnly = 1, kCombineReduceOnly = 2 };
 

@@ -7,8 +7,7 @@
 // glue of `DeepEP_Megatron/test_deepep_moe_dispatch_combine.py:276-388`.
 //
 // Structure of one launch:
-//   prologue (every CTA)  (a group of one in rank mode counts from the flags instead: count_own)
-//                         bounded wait for the peers' count vectors, then the prefix sums that
+//   prologue (every CTA)  bounded wait for the peers' count vectors, then the prefix sums that
 //                         give, per bucket, the first row at the destination (`send_base`) and
 //                         the first slot of this rank's combine region (`comb_base`), kept in
 //                         shared memory. One warp of the grid also writes the receive-side
@@ -100,43 +99,6 @@ __device__ bool dispatch_prologue(const EpGeom& g, const EpRegions& rg, char* se
   return true;
 }
 
-// A group of one in rank mode counts for itself: an item's place is the number of tokens before it that the flags name,
-// which every CTA finds from the flags alone (a byte a token). Fills s_bits[C] (flags of a chunk of 32 tokens)
-// and s_base[C] (flags before the chunk); returns the total. This takes the place of a count launch of its own, whose
-// tables the items then read back from global memory. On a device timeline of one B200 a count launch of 5.3 us goes
-// and the send kernel takes 27.7 us instead of 26.2 (4096 rows of 14 KiB; 7.2 us go, 9.6 instead of 9.4 with 96 rows of 2 KiB).
-__device__ __forceinline__ int count_own(const bool* __restrict__ in_rank, int T, unsigned int* s_bits, int* s_base) {
-  __shared__ int s_total;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const int C = (T + kChunkTokens - 1) / kChunkTokens;
-  constexpr int U = 8;                       // loads in flight
-  for (int c0 = warp; c0 < C; c0 += nwarps * U) {
-    bool in[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int t = (c0 + u * nwarps) * kChunkTokens + lane;
-      in[u] = t < T && in_rank[t];
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const unsigned m = __ballot_sync(0xffffffffu, in[u]);
-      if (lane == 0 && c0 + u * nwarps < C) s_bits[c0 + u * nwarps] = m;
-    }
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) s_base[c] = __popc(s_bits[c]);
-  __syncthreads();
-  if (warp == 0) {
-    const int last = s_base[C - 1];
-    __syncwarp();
-    warp_exclusive_scan(s_base, C, lane);
-    __syncwarp();
-    if (lane == 0) s_total = s_base[C - 1] + last;
-  }
-  __syncthreads();
-  return s_total;
-}
-
 // ONE warp of the grid: receive-side tables of the handle, host words, overflow checks. The other
 // warps of its CTA go on with their tokens meanwhile; the warp that owns the fewest items does it.
 // Lanes run over the experts and a shuffle scan makes the offsets: a single thread that walked
@@ -144,7 +106,7 @@ __device__ __forceinline__ int count_own(const bool* __restrict__ in_rank, int T
 __device__ void dispatch_publish_meta(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                                       char* self_base, const EpMeta& m, const int* s_send_base,
                                       const int* s_comb_base, volatile int* host_word, int* status,
-                                      bool ok, int lane, int own_total, const int* own_per_expert) {
+                                      bool ok, int lane) {
   const int R = g.R, E = g.E, El = g.El, V = g.R + g.E, me = g.rank, B = g.B;
   if (!ok) {
     if (lane == 0) {
@@ -159,11 +121,6 @@ __device__ void dispatch_publish_meta(const EpGeom& g, const EpRegions& rg, cons
     return;
   }
   const int* M = reinterpret_cast<const int*>(self_base + rg.counts);
-  // entry v of rank r's count vector [R rank counts | E expert counts]; own_total >= 0: a group of one that counted for itself
-  auto count = [&](int r, int v) {
-    if (own_total >= 0) return v < R ? own_total : own_per_expert != nullptr ? own_per_expert[v - R] : 0;
-    return __ldcg(&M[r * V + v]);
-  };
   for (int b = lane; b < B; b += 32) {
     m.send_base[b] = s_send_base[b];
     m.comb_base[b] = s_comb_base[b];
@@ -173,7 +130,7 @@ __device__ void dispatch_publish_meta(const EpGeom& g, const EpRegions& rg, cons
     const int q = q0 + lane;
     int cnt = 0;
     if (q < El)
-      for (int r = 0; r < R; ++r) cnt += count(r, R + me * El + q);
+      for (int r = 0; r < R; ++r) cnt += __ldcg(&M[r * V + R + me * El + q]);
     int incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -188,7 +145,7 @@ __device__ void dispatch_publish_meta(const EpGeom& g, const EpRegions& rg, cons
     acc += __shfl_sync(0xffffffffu, incl, 31);
   }
   // rows from every source rank (rank mode) and slots used on this rank
-  const int from = lane < R ? count(lane, me) : 0;
+  const int from = lane < R ? __ldcg(&M[lane * V + me]) : 0;
   int incl = from;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -199,9 +156,9 @@ __device__ void dispatch_publish_meta(const EpGeom& g, const EpRegions& rg, cons
   const int n_from = __shfl_sync(0xffffffffu, incl, 31);
   int stot = 0;
   if (g.mode == 1) {
-    for (int q = lane; q < E; q += 32) stot += count(me, R + q);
+    for (int q = lane; q < E; q += 32) stot += __ldcg(&M[me * V + R + q]);
   } else if (lane < R) {
-    stot = count(me, lane);
+    stot = __ldcg(&M[me * V + lane]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) stot += __shfl_xor_sync(0xffffffffu, stot, o);
@@ -238,11 +195,10 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
                      const long long* __restrict__ topk_idx, const float* __restrict__ topk_w,
                      const int* __restrict__ item_rank, const int* __restrict__ chunk_base,
                      int* send_row, int* send_slot, unsigned int* block_counter, int* host_word,
-                     int* status, const float* __restrict__ scales_in, const bool* __restrict__ own_flags,
-                     const int* __restrict__ own_per_expert) {
+                     int* status, const float* __restrict__ scales_in) {
   stream_order_wait();
   if (g.R == 1) stream_order_next();
-  extern __shared__ int dyn[];               // [B] send_base, [B] comb_base, [E] scratch; own_flags: [C] bits, [C] bases behind them
+  extern __shared__ int dyn[];               // [B] send_base, [B] comb_base, [E] scratch
   __shared__ char* s_dst[kSendWarps][kMaxItemsPerToken];
   __shared__ float* s_scl[kSendWarps][kMaxItemsPerToken];
   __shared__ int s_first[kMaxRanks];
@@ -255,9 +211,6 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
   char* self_base = peers.base[g.rank];
   int* s_send_base = dyn;
   int* s_comb_base = dyn + g.B;
-  const bool own = MODE == 0 && !CACHED && own_flags != nullptr;
-  unsigned int* s_bits = reinterpret_cast<unsigned int*>(dyn + 2 * g.B + g.E);
-  int* s_own_base = dyn + 2 * g.B + g.E + (g.T + kChunkTokens - 1) / kChunkTokens;
 
   if (CACHED && MODE == 1) {                 // where each rank's slots begin (from the handle)
     if ((int)threadIdx.x < g.R) s_first[threadIdx.x] = m.comb_base[threadIdx.x * El];
@@ -282,16 +235,9 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
   if (!CACHED) {
     // After a notify time-out the prefix tables are not valid: store nothing (the flags below are
     // still raised so that healthy peers are not kept waiting by this rank).
-    bool ok = true;
-    int total = -1;
-    if (own) {
-      if (threadIdx.x == 0) s_send_base[0] = s_comb_base[0] = 0;
-      total = count_own(own_flags, g.T, s_bits, s_own_base);
-    } else {
-      ok = dispatch_prologue(g, rg, self_base, s_send_base, s_comb_base, dyn + 2 * g.B, status);
-    }
+    const bool ok = dispatch_prologue(g, rg, self_base, s_send_base, s_comb_base, dyn + 2 * g.B, status);
     if (gw == nw - 1)
-      dispatch_publish_meta(g, rg, peers, self_base, m, s_send_base, s_comb_base, host_word, status, ok, lane, total, own_per_expert);
+      dispatch_publish_meta(g, rg, peers, self_base, m, s_send_base, s_comb_base, host_word, status, ok, lane);
     if (!ok) n_tokens = 0;
   }
 
@@ -311,17 +257,10 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
           slot = -1;
         }
       } else {
-        const int b = (MODE == 0) ? lane : (int)e;
-        int ir, pos = 0;
-        if (own) {
-          const unsigned bits = s_bits[t / kChunkTokens], at = 1u << (t % kChunkTokens);
-          ir = (bits & at) ? __popc(bits & (at - 1)) : -1;
-          if (ir >= 0) pos = s_own_base[t / kChunkTokens] + ir;
-        } else {
-          ir = item_rank[(size_t)t * J + lane];
-          if (ir >= 0) pos = chunk_base[(size_t)(t / kChunkTokens) * g.B + b] + ir;
-        }
+        const int ir = item_rank[(size_t)t * J + lane];
         if (ir >= 0) {
+          const int b = (MODE == 0) ? lane : (int)e;
+          const int pos = chunk_base[(size_t)(t / kChunkTokens) * g.B + b] + ir;
           row = s_send_base[b] + pos;
           slot = s_comb_base[b] + pos;
           if (row >= g.cap || slot >= g.slot_cap || row < 0 || slot < 0) {
@@ -447,14 +386,14 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
 #define B200EP_LAUNCH_DISPATCH(MODE, FP8, CACHED)                                              \
   launch_ordered(dispatch_send_kernel<MODE, FP8, CACHED>, blocks, warps * 32, smem, st, 1,     \
       g, rg, peers, m, x, row_bytes_in, parts, topk_idx, topk_w, item_rank, chunk_base,        \
-      send_row, send_slot, block_counter, host_word, status, scales_in, own_flags, own_per_expert)
+      send_row, send_slot, block_counter, host_word, status, scales_in)
 
 void launch_dispatch_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& peers,
                           const EpMeta& m, const char* x, int row_bytes_in, bool fp8, bool cached,
                           const long long* topk_idx, const float* topk_w, const int* item_rank,
                           const int* chunk_base, int* send_row, int* send_slot,
                           unsigned int* block_counter, int* host_word, int* status, int blocks,
-                          cudaStream_t st, const float* scales_in, const bool* own_flags, const int* own_per_expert) {
+                          cudaStream_t st, const float* scales_in) {
   if (blocks < 1) blocks = 1;
   // Few tokens: a row is cut into up to 8 parts of at least 2 KiB of input, one warp each (a warp that walks a
   // 14 KiB row alone pays seven memory round trips), and CTAs are no larger than the items need.
@@ -466,7 +405,7 @@ void launch_dispatch_send(const EpGeom& g, const EpRegions& rg, const PeerPtrs& 
   while (warps > 4 && (long long)blocks * (warps / 2) >= items) warps /= 2;
   const long long need = (items + warps - 1) / warps;
   if (need < blocks) blocks = need < 1 ? 1 : (int)need;
-  const size_t smem = sizeof(int) * (2 * (size_t)g.B + g.E + (own_flags ? 2 * ((g.T + kChunkTokens - 1) / kChunkTokens) : 0));
+  const size_t smem = sizeof(int) * (2 * (size_t)g.B + g.E);
   if (g.mode == 0) {
     if (fp8) { if (cached) B200EP_LAUNCH_DISPATCH(0, true, true); else B200EP_LAUNCH_DISPATCH(0, true, false); }
     else     { if (cached) B200EP_LAUNCH_DISPATCH(0, false, true); else B200EP_LAUNCH_DISPATCH(0, false, false); }

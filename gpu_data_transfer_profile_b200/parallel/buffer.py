@@ -476,7 +476,6 @@ class Buffer:
         per_expert = st.get("num_tokens_per_expert")
         if per_expert is not None and per_expert.dtype != torch.int32:
             per_expert = per_expert.to(torch.int32)
-        st["per_expert"] = per_expert
         st["meta"], st["send_row"], st["send_slot"] = self._ctx.notify(
             mode, T, st["epoch_n"], self._timeout_ns(), st.get("is_token_in_rank"), st["topk_idx"], per_expert)
         return st
@@ -496,7 +495,7 @@ class Buffer:
             own = min(max(items, st["handle"].n_recv if st["cached"] else 0), st["carve"].cap)
         st["own"] = self._ctx.send(st["mode"], st["epoch_d"], st.get("epoch_n", 0), self._single_launch, self._timeout_ns(), self._blocks(),
                        st["meta"], st["x"], st["fp8"], st["cached"], st["topk_idx"], st.get("topk_weights"), st["send_row"],
-                       st["send_slot"], st["scales_in"], own, st.get("is_token_in_rank"), st.get("per_expert"), own_probs)
+                       st["send_slot"], st["scales_in"], own, own_probs)
 
     def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1, own_probs: int = 0):
         R, E, K, H = self.group_size, st["E"], st["K"], st["H"]

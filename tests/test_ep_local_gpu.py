@@ -782,39 +782,3 @@ def test_owned_outputs_hold_no_more_memory_than_their_rows(masked, grouped):
         buf.check_status()
     finally:
         buf.destroy()
-
-
-@pytest.mark.parametrize("T", [1, 31, 32, 33, 255, 257, 1000, 16384, 16385])
-@pytest.mark.parametrize("masked", [False, True])
-def test_rank_mode_group_of_one_counts_for_itself(T, masked):
-    """The send kernel of a group of one finds every token's row from the flags (up to 16384 tokens; more are counted by
-    the count launch): edges of the chunks of 32, one CTA and many, tokens that go nowhere, with owned and with
-    region outputs, with and without the host's read of the count. Rows, routing, weights and counts are exact."""
-    from gpu_data_transfer_profile_b200.parallel.local import LocalGroup
-    H, E, K = 128, 16, 2
-    gen = torch.Generator().manual_seed(T)
-    idx = torch.stack([torch.randint(0, E // 2, (T,), generator=gen), torch.randint(E // 2, E, (T,), generator=gen)], 1)
-    if masked:
-        idx[torch.rand(T, generator=gen) < 0.4] = -1
-    x = torch.randn(T, H, generator=gen).to(torch.bfloat16).cuda()
-    w, idx = torch.rand(T, K, generator=gen).cuda(), idx.cuda()
-    keep = idx[:, 0] >= 0
-    n = int(keep.sum())
-    g = LocalGroup(1, 64 << 20, timeout_s=2.0)
-    try:
-        b = g.buffers[0]
-        per_rank, _, per_expert, in_rank, _ = b.get_dispatch_layout(idx, E)
-        for zero_copy in (False, True):
-            for worst in (0, T):
-                rx, ri, rw, counts, h, _ = b.dispatch(x, topk_idx=idx, topk_weights=w, num_tokens_per_rank=per_rank,
-                                                      is_token_in_rank=in_rank, num_tokens_per_expert=per_expert,
-                                                      zero_copy=zero_copy, num_worst_tokens=worst)
-                assert torch.equal(rx[:n], x[keep]) and torch.equal(ri[:n], idx[keep]) and torch.equal(rw[:n], w[keep])
-                if worst == 0:
-                    assert rx.shape[0] == n and counts == torch.bincount(idx[keep].flatten().cpu(), minlength=E).tolist()
-                assert int(h.n_recv_dev) == n
-                out, ow, _ = b.combine(rx, h, topk_weights=rw)
-                assert torch.equal(out, x * keep[:, None]) and torch.equal(ow, w * keep[:, None])
-        g.check_status()
-    finally:
-        g.destroy()
