@@ -5,7 +5,7 @@
 
 namespace b200ep {
 
-enum GemmEpilogue : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_COMBINE = 2 };
+enum GemmEpilogue : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_COMBINE = 2, EPI_DSWIGLU = 3, EPI_ACT = 4 };
 
 struct GemmParams {
   int El;                 // local experts
@@ -13,15 +13,17 @@ struct GemmParams {
   int K;                  // reduction length
   int N_out;              // columns of the stored result (== N)
   int w_rows;             // rows per expert in the weight tensor (N, or 2F for swiglu; K if b_mn)
-  int b_mn;               // 1: weights stored [El, K, N] (N contiguous), plain epilogue only
+  int b_mn;               // 1: weights stored [El, K, N] (N contiguous), plain and dswiglu epilogues only
   int n_tiles, max_rows;  // filled by the launcher
   int band_rows;          // activation rows per L2-resident band of the tile order (<= 0: 2048)
   const int* expert_off;  // device [El+1]: exclusive prefix of rows per local expert
-  void* out;              // bf16 [rows, out_ld]           (plain / swiglu)
+  void* out;              // bf16 [rows, out_ld]           (all but combine; dswiglu: gradient of the pre-activation, 2N columns)
   long long out_ld;
-  const float* row_prob;  // f32 [rows] or null            (swiglu)
+  const float* row_prob;  // f32 [rows] or null            (all but plain and combine)
   void* pre_out;          // bf16 [rows, pre_ld] or null   (swiglu: also store the pre-activation [gate | linear])
-  long long pre_ld;
+  long long pre_ld;       // (dswiglu: the same pre-activation, read; act: [rows, N])
+  int act_kind;           // act: 0 gelu (erf form), 1 silu, 2 relu
+  float* dp_part;         // f32 [N / 128, rows]: parts of the row sums that the probabilities' gradients are (dswiglu)
   const int2* recv_meta;  // {slot at source, source rank} (combine)
   long long comb_off;     // offset of the combine region in every rank's symmetric buffer
   int slot_cap, R, rank;
@@ -84,6 +86,8 @@ int launch_swiglu_bwd(const void* h, const float* p, const void* dact, void* dh,
 // Ungated activation x prob pair (h: bf16 [rows, F]); kind: 0 gelu (erf form), 1 silu, 2 relu.
 int launch_act_fwd(const void* h, const float* p, void* act, const int* n_rows_ptr, int max_rows, int F, int kind,
                    cudaStream_t st);
+// dp[row] = sum over the parts of a dswiglu GEMM, in ascending order.
+int launch_sum_parts(const float* part, int parts, int rows, float* dp, cudaStream_t st);
 int launch_act_bwd(const void* h, const float* p, const void* dact, void* dh, float* dp, const int* n_rows_ptr,
                    int max_rows, int F, int kind, cudaStream_t st);
 

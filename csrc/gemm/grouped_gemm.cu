@@ -9,6 +9,18 @@
 //   EPI_SWIGLU  : W holds [gate rows | linear rows]; a CTA multiplies 64 gate and the matching 64
 //                 linear rows, the epilogue writes silu(gate) * linear * prob[r] as bf16 and, for
 //                 training, the pre-activation too.
+//   EPI_ACT     : the same for gelu / silu / relu: f(result) * prob and, for training, the pre-activation. Three groups of
+//                 epilogue warps (8191 rows, 8 experts, 4096 x 4096: GEMM, activation kernel and fc2 with silu 441 us, in
+//                 the epilogue 415; forward and backward of 12001 rows, 16 experts, 2048 x 1408: 440 -> 428, with two
+//                 groups 437).
+//   EPI_DSWIGLU : (data gradient of fc2) the result is the gradient of silu(gate) * linear * prob; the epilogue
+//                 reads the kept pre-activation and writes its gradient, so the gradient of the activation never
+//                 goes to memory and no element-wise kernel follows. The sums for the probabilities' gradients
+//                 leave as one part per 128 columns (fixed order; sum_parts_kernel adds them). It has three groups
+//                 of epilogue warps: with two the element-wise work of a tile takes longer than its MMAs (12001 rows, 16 experts,
+//                 2048 x 1408: GEMM and element-wise kernel apart 68 + 34.4 us, in one with two groups 126, with three
+//                 75 + 4.0 for the sums). Not for gelu / silu / relu, whose element-wise backward moves 3 elements where
+//                 this moves 5: in one launch the same step with silu took 453 us, apart 433.
 //   EPI_COMBINE : the fc2 result rows are stored straight into the combine slot of each token's
 //                 SOURCE rank over NVLink (LSU stores), so no separate unpermute/combine-send
 //                 kernel runs; the source reduces its slots on arrival.
@@ -32,14 +44,15 @@
 //           into each CTA's TMEM. A token tile is thus fetched once per pair and the shared-memory
 //           traffic per flop halves for it; 6-stage ring of 32 KiB.
 // Epilogue: an accumulator lane is a weight row (an output column), so 16 token columns at a time go
-// through a f32 staging tile in shared memory and leave as 128-byte segments of output rows. Two
-// groups of four warps take alternate 16-column chunks.
+// through a f32 staging tile in shared memory and leave as 128-byte segments of output rows. Two or
+// three groups of four warps take 16-column chunks in turn.
 // The tile list is derived on the device from the per-expert row offsets (no host sync).
 // Every mbarrier wait is bounded; on a time-out all roles leave their loops, TMEM is freed.
 #include <cuda_bf16.h>
 #include "tc05.cuh"
 #include "tmap.h"
 #include "gemm_api.h"
+#include "act.cuh"
 
 namespace b200ep {
 
@@ -54,12 +67,14 @@ template <> struct Ring<2> { static constexpr int STAGES = 6, STAGE_BYTES = W_BY
 constexpr int MAX_STAGES = 6;
 constexpr int RING_BYTES = 4 * (W_BYTES + 2 * T_HALF_BYTES);
 static_assert(Ring<1>::STAGES * Ring<1>::STAGE_BYTES == RING_BYTES && Ring<2>::STAGES * Ring<2>::STAGE_BYTES == RING_BYTES, "");
-constexpr int EPI_GROUPS = 2, EPI_WARPS = 4 * EPI_GROUPS;
 constexpr int CHUNK = 16;                                     // token columns per staging pass
 constexpr int STG_LD = WM + 4;                                // f32 per staged token (pad: bank spread)
 constexpr int STG_BYTES = CHUNK * STG_LD * 4;
-constexpr int SMEM_BYTES = RING_BYTES + EPI_GROUPS * STG_BYTES + 1024 /*align slack*/;
-constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
+// groups of four epilogue warps
+template <int EPI> struct Epi {
+  static constexpr int GROUPS = EPI == EPI_DSWIGLU || EPI == EPI_ACT ? 3 : 2, WARPS = 4 * GROUPS;
+  static constexpr int THREADS = 64 + 32 * WARPS, SMEM_BYTES = RING_BYTES + GROUPS * STG_BYTES + 1024 /*align slack*/;
+};
 constexpr int kMaxLocalExperts = 256;
 constexpr int TOKEN_BOXES = 4;                                // token boxes of 16, 32, 64 and 128 rows
 
@@ -105,6 +120,35 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
+__device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+// Backward of silu(g) * l * prob for one element: d = gradient of the product; the gradients of g and l come back in
+// place of g and l, the element's share of the probability's gradient is returned.
+__device__ __forceinline__ float dswiglu(float d, float pr, float& g, float& l) {
+  const float sig = __fdividef(1.f, 1.f + __expf(-g));      // (within 2 ulp; what comes of it leaves as bf16)
+  const float s = g * sig, da = d * pr, share = d * s * l;
+  g = da * l * sig * (1.f + g * (1.f - sig));
+  l = da * s;
+  return share;
+}
+// four columns: d against bf16 pairs of gate and linear, both replaced by their gradients
+__device__ __forceinline__ float dswiglu4(const float4& d, float pr, uint2& hg, uint2& hl) {
+  float g[4] = {bf_lo(hg.x), bf_hi(hg.x), bf_lo(hg.y), bf_hi(hg.y)};
+  float l[4] = {bf_lo(hl.x), bf_hi(hl.x), bf_lo(hl.y), bf_hi(hl.y)};
+  const float dd[4] = {d.x, d.y, d.z, d.w};
+  float share = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) share += dswiglu(dd[i], pr, g[i], l[i]);
+  hg = make_uint2(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]));
+  hl = make_uint2(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]));
+  return share;
+}
+__device__ __forceinline__ float act_only(int kind, float x) {
+  if (kind == 1) return x * __fdividef(1.f, 1.f + __expf(-x));      // (within 2 ulp; what comes of it leaves as bf16)
+  float f, df;
+  act_eval(kind, x, &f, &df);
+  return f;
+}
 __device__ __forceinline__ void st_global_v2(void* p, uint32_t a, uint32_t b) {
   asm volatile("st.global.L1::no_allocate.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(b) : "memory");
 }
@@ -113,9 +157,10 @@ __device__ __forceinline__ void st_global_v2(void* p, uint32_t a, uint32_t b) {
 // then read as an M-major operand (64 x 64 boxes, one 128-byte row of 64 outputs per reduction
 // index), which is how the data gradients use the forward weights without a transposed copy.
 template <int EPI, int CG, bool WMN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(Epi<EPI>::THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ GemmParams p, const __grid_constant__ PeerPtrs peers) {
+  constexpr int EPI_GROUPS = Epi<EPI>::GROUPS, EPI_WARPS = Epi<EPI>::WARPS;
   constexpr int STAGES = Ring<CG>::STAGES, STAGE_BYTES = Ring<CG>::STAGE_BYTES, G = 16 * CG;
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_full[2], acc_empty[2];
@@ -295,11 +340,20 @@ grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_consta
       float prob[2] = {1.f, 1.f};
       // what the reader needs to know about its two tokens of chunk c, requested one chunk ahead
       int2 meta[2];
+      uint2 pre[2][4];                             // dswiglu: gate and linear of my columns, then of those 64 on
+      const bool ok_a = col0 < p.N, ok_b = col0 + 64 < p.N;      // (a last tile may hang over the expert's outputs)
       auto fetch = [&](int c) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int tok = c * CHUNK + tok_in + 8 * i;
-          if (EPI == EPI_SWIGLU && p.row_prob != nullptr && tok < tl.rows) prob[i] = p.row_prob[tl.row0 + tok];
+          if (EPI != EPI_PLAIN && EPI != EPI_COMBINE && p.row_prob != nullptr && tok < tl.rows) prob[i] = p.row_prob[tl.row0 + tok];
+          if (EPI == EPI_DSWIGLU && ok_a && tok < tl.rows) {
+            const char* h = reinterpret_cast<const char*>(p.pre_out) + ((size_t)(tl.row0 + tok) * p.pre_ld + col0) * 2;
+            pre[i][0] = __ldg(reinterpret_cast<const uint2*>(h));
+            pre[i][1] = __ldg(reinterpret_cast<const uint2*>(h + (size_t)p.N * 2));
+            pre[i][2] = __ldg(reinterpret_cast<const uint2*>(h + 128));
+            pre[i][3] = __ldg(reinterpret_cast<const uint2*>(h + (size_t)p.N * 2 + 128));
+          }
           if (EPI == EPI_COMBINE && tok < tl.rows) meta[i] = p.recv_meta[tl.row0 + tok];
         }
       };
@@ -316,6 +370,13 @@ grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_consta
         const float pr0 = prob[0], pr1 = prob[1];
         int2 mt[2];
         if (EPI == EPI_COMBINE) { mt[0] = meta[0]; mt[1] = meta[1]; }
+        uint2 hv[2][4];
+        if (EPI == EPI_DSWIGLU) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) hv[i][u] = pre[i][u];
+        }
         if (c + EPI_GROUPS < chunks) { fetch(c + EPI_GROUPS); tmem_ld16(t_addr + (c + EPI_GROUPS) * CHUNK, v); }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -324,7 +385,35 @@ grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_consta
           const float4 a = *reinterpret_cast<const float4*>(stg + tok * STG_LD + 4 * oct);
           const float4 b = *reinterpret_cast<const float4*>(stg + tok * STG_LD + 64 + 4 * oct);
           const size_t grow = (size_t)(tl.row0 + c * CHUNK + tok);
-          if (EPI == EPI_SWIGLU) {
+          if (EPI == EPI_DSWIGLU) {
+            // a and b are the gradient of the activation; it goes no further than these registers
+            const int block = tl.wt * CG + cta_rank;     // my CTA's 128 columns: all there or, behind an odd number, none
+            if (!ok_b) continue;
+            const float pr = i == 0 ? pr0 : pr1;
+            float share = dswiglu4(a, pr, hv[i][0], hv[i][1]) + dswiglu4(b, pr, hv[i][2], hv[i][3]);
+            char* o = reinterpret_cast<char*>(p.out) + (grow * p.out_ld + col0) * 2;
+            st_global_v2(o, hv[i][0].x, hv[i][0].y);
+            st_global_v2(o + 128, hv[i][2].x, hv[i][2].y);
+            o += (size_t)p.N * 2;
+            st_global_v2(o, hv[i][1].x, hv[i][1].y);
+            st_global_v2(o + 128, hv[i][3].x, hv[i][3].y);
+            // the 16 lanes of a token hold its 128 columns
+            const unsigned half_mask = 0xffffu << (lane & 16);
+#pragma unroll
+            for (int m = 8; m > 0; m >>= 1) share += __shfl_xor_sync(half_mask, share, m);
+            if (oct == 0) p.dp_part[(size_t)block * p.max_rows + grow] = share;
+          } else if (EPI == EPI_ACT) {
+            const float pr = i == 0 ? pr0 : pr1;
+            const int k = p.act_kind;
+            char* o = reinterpret_cast<char*>(p.out) + (grow * p.out_ld + col0) * 2;
+            if (ok_a) st_global_v2(o, pack_bf16(act_only(k, a.x) * pr, act_only(k, a.y) * pr), pack_bf16(act_only(k, a.z) * pr, act_only(k, a.w) * pr));
+            if (ok_b) st_global_v2(o + 128, pack_bf16(act_only(k, b.x) * pr, act_only(k, b.y) * pr), pack_bf16(act_only(k, b.z) * pr, act_only(k, b.w) * pr));
+            if (p.pre_out != nullptr) {
+              char* h = reinterpret_cast<char*>(p.pre_out) + (grow * p.pre_ld + col0) * 2;
+              if (ok_a) st_global_v2(h, pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
+              if (ok_b) st_global_v2(h + 128, pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+            }
+          } else if (EPI == EPI_SWIGLU) {
             const float pr = i == 0 ? pr0 : pr1;
             char* o = reinterpret_cast<char*>(p.out) + (grow * p.out_ld + col0) * 2;
             st_global_v2(o, pack_bf16(silu(a.x) * b.x * pr, silu(a.y) * b.y * pr),
@@ -386,8 +475,8 @@ static int max_resident_pairs() {
   if (cached < 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.blockDim = dim3(Epi<EPI>::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Epi<EPI>::SMEM_BYTES;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -406,12 +495,12 @@ template <int EPI, bool WMN>
 static int launch_one(const TokenMaps& ma, const CUtensorMap& mb, const GemmParams& p, const PeerPtrs& peers,
                       int ctas, bool pair, cudaStream_t st) {
   if (!pair) {
-    if (cudaFuncSetAttribute(grouped_gemm_kernel<EPI, 1, WMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(grouped_gemm_kernel<EPI, 1, WMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Epi<EPI>::SMEM_BYTES) != cudaSuccess)
       return 4;
-    grouped_gemm_kernel<EPI, 1, WMN><<<ctas, GEMM_THREADS, SMEM_BYTES, st>>>(ma, mb, p, peers);
+    grouped_gemm_kernel<EPI, 1, WMN><<<ctas, Epi<EPI>::THREADS, Epi<EPI>::SMEM_BYTES, st>>>(ma, mb, p, peers);
     return 0;
   }
-  if (cudaFuncSetAttribute(grouped_gemm_kernel<EPI, 2, WMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+  if (cudaFuncSetAttribute(grouped_gemm_kernel<EPI, 2, WMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Epi<EPI>::SMEM_BYTES) != cudaSuccess)
     return 4;
   int pairs = ctas / 2;
   const int resident = max_resident_pairs<EPI, WMN>();
@@ -420,8 +509,8 @@ static int launch_one(const TokenMaps& ma, const CUtensorMap& mb, const GemmPara
   if (pairs < 1) pairs = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.blockDim = dim3(Epi<EPI>::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = Epi<EPI>::SMEM_BYTES;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -437,7 +526,9 @@ int launch_grouped_gemm(const void* a, long long a_rows, const void* w, int epi,
                         const PeerPtrs& peers, int ctas, bool pair, cudaStream_t st) {
   if (p.El < 1 || p.El > kMaxLocalExperts || p.K <= 0 || p.K % 8 || p.N <= 0 || p.N_out % 8) return 1;
   if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(w) % 16) return 1;
-  if (epi == EPI_SWIGLU && (p.N % 128)) return 1;
+  if ((epi == EPI_SWIGLU || epi == EPI_DSWIGLU) && (p.N % 128)) return 1;
+  if (epi == EPI_ACT && (p.act_kind < 0 || p.act_kind > 2)) return 1;
+  if (epi == EPI_DSWIGLU && (!p.b_mn || p.pre_out == nullptr || p.dp_part == nullptr)) return 1;
   // 64-column boxes (one 128-byte swizzle row): the tokens in four heights, so that a small tile fetches no more
   // rows than it needs; the weights 128 rows high, 64 where a CTA's rows come from two places
   TokenMaps ma;
@@ -445,7 +536,7 @@ int launch_grouped_gemm(const void* a, long long a_rows, const void* w, int epi,
   for (int b = 0; b < TOKEN_BOXES; ++b)
     if (make_tmap_bf16(&ma.m[b], a, a_rows, p.K, BK, 16 << b)) return 3;
   if (p.b_mn) {
-    if (epi != EPI_PLAIN) return 1;
+    if (epi != EPI_PLAIN && epi != EPI_DSWIGLU) return 1;
     if (make_tmap_bf16(&mb, w, (long long)p.El * p.w_rows, p.N, 64, BK)) return 3;
   } else if (make_tmap_bf16(&mb, w, (long long)p.El * p.w_rows, p.K, BK, epi == EPI_SWIGLU ? 64 : WM)) return 3;
   const int tile_cols = (pair ? 2 : 1) * (epi == EPI_SWIGLU ? 64 : WM);       // output columns per tile
@@ -454,6 +545,8 @@ int launch_grouped_gemm(const void* a, long long a_rows, const void* w, int epi,
   if (p.band_rows <= 0) p.band_rows = 2048;
   if (ctas < 1) ctas = 1;
   if (epi == EPI_PLAIN && p.b_mn) return launch_one<EPI_PLAIN, true>(ma, mb, p, peers, ctas, pair, st);
+  if (epi == EPI_DSWIGLU) return launch_one<EPI_DSWIGLU, true>(ma, mb, p, peers, ctas, pair, st);
+  if (epi == EPI_ACT) return launch_one<EPI_ACT, false>(ma, mb, p, peers, ctas, pair, st);
   if (epi == EPI_PLAIN) return launch_one<EPI_PLAIN, false>(ma, mb, p, peers, ctas, pair, st);
   if (epi == EPI_SWIGLU) return launch_one<EPI_SWIGLU, false>(ma, mb, p, peers, ctas, pair, st);
   if (epi == EPI_COMBINE) return launch_one<EPI_COMBINE, false>(ma, mb, p, peers, ctas, pair, st);

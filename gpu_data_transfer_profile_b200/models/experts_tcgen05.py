@@ -4,10 +4,10 @@ Forward: fc1 with SwiGLU x probability fused into its epilogue (one kernel), fc2
 plain grouped GEMM or with the combine send fused into its epilogue (`forward_fused_combine`).
 Tile scheduling reads the per-expert row offsets on the device. Backward (SwiGLU path): the two
 data gradients run on the same grouped GEMM reading the forward weights in place as an M-major
-operand, the two weight gradients on the ragged-reduction kernel (`ops.gemm.grouped_wgrad`), the
-element-wise part on the fused SwiGLU backward kernel; no library GEMM and no host-side split.
+operand, the first with the SwiGLU backward in its epilogue, the two weight gradients on the
+ragged-reduction kernel (`ops.gemm.grouped_wgrad`); no library GEMM and no host-side split.
 gelu / silu / relu (`DeepEP_Megatron/test_deepep_moe_dispatch_combine.py:516-526`) take the same
-route with the ungated activation kernels of csrc/gemm/swiglu.cu.
+route, with the ungated backward kernel of csrc/gemm/swiglu.cu.
 """
 from __future__ import annotations
 
@@ -33,24 +33,21 @@ def _wgrad(dy, a, counts, out_shape, expert_off=None):
 
 
 class _GroupedMLP(torch.autograd.Function):
-    """Training path. SwiGLU: fc1 (tcgen05; the epilogue applies SwiGLU x prob AND stores the
-    pre-activation h for backward) -> fc2 (tcgen05). Backward: fused swiglu backward kernel, both dgrads on
-    the tcgen05 grouped GEMM (weights read in place, M-major), both wgrads on the tcgen05
-    ragged-reduction kernel."""
+    """Training path: fc1 (tcgen05; the epilogue applies activation x prob AND stores the
+    pre-activation h for backward) -> fc2 (tcgen05). Backward: both dgrads on the tcgen05 grouped GEMM
+    (weights read in place, M-major; the SwiGLU backward in the epilogue of the first), both wgrads on the
+    tcgen05 ragged-reduction kernel."""
 
     @staticmethod
     def forward(ctx, x, w1, w2, probs, expert_off, counts, activation):
         ctx.counts, ctx.activation = counts, activation
         ctx.off = expert_off
+        # one kernel: fc1, activation x prob in the epilogue, and the pre-activation kept for backward
+        h = torch.empty((x.shape[0], w1.shape[1]), dtype=x.dtype, device=x.device)
         if activation == "swiglu":
-            # one kernel: fc1, SwiGLU x prob in the epilogue, and the pre-activation kept for backward
-            h = torch.empty((x.shape[0], w1.shape[1]), dtype=x.dtype, device=x.device)
             act = G.grouped_gemm_swiglu(x, w1, expert_off, probs, pre_out=h)
-            y = G.grouped_gemm(act, w2, expert_off)
-            ctx.save_for_backward(x, w1, w2, probs, h, act)
-            return y
-        h = G.grouped_gemm(x, w1, expert_off)
-        act = G.act_fwd(h, probs, activation)
+        else:
+            act = G.grouped_gemm_act(x, w1, expert_off, probs, activation, pre_out=h)
         ctx.save_for_backward(x, w1, w2, probs, h, act)
         return G.grouped_gemm(act, w2, expert_off)
 
@@ -59,10 +56,10 @@ class _GroupedMLP(torch.autograd.Function):
         dy = dy.contiguous()
         x, w1, w2, probs, h, act = ctx.saved_tensors
         rows = sum(ctx.counts)
-        dact = G.grouped_gemm(dy, w2, ctx.off, w_kn=True)                             # [rows, F]
         if ctx.activation == "swiglu":
-            dh, dp = G.swiglu_bwd(h, probs, dact)
+            dh, dp = G.grouped_gemm_dswiglu(dy, w2, ctx.off, h, probs)                # [rows, 2F], [rows]
         else:
+            dact = G.grouped_gemm(dy, w2, ctx.off, w_kn=True)                         # [rows, F]
             dh, dp = G.act_bwd(h, probs, dact, ctx.activation)
         dx = G.grouped_gemm(dh, w1, ctx.off, w_kn=True)                               # [rows, H]
         dw2 = _wgrad(dy[:rows], act[:rows], ctx.counts, w2.shape, ctx.off)
@@ -90,8 +87,7 @@ class _GroupedMLPFusedCombine(torch.autograd.Function):
         x, w1, w2, probs, h, act = ctx.saved_tensors
         dy, *_ = ctx.buffer.dispatch(grad_out.contiguous(), handle=ctx.handle)
         rows = sum(ctx.counts)
-        dact = G.grouped_gemm(dy, w2, ctx.off, w_kn=True)
-        dh, dp = G.swiglu_bwd(h, probs, dact)
+        dh, dp = G.grouped_gemm_dswiglu(dy, w2, ctx.off, h, probs)
         dx = G.grouped_gemm(dh, w1, ctx.off, w_kn=True)
         dw2 = _wgrad(dy[:rows], act[:rows], ctx.counts, w2.shape, ctx.off)
         dw1 = _wgrad(dh[:rows], x[:rows], ctx.counts, w1.shape, ctx.off)
@@ -150,8 +146,8 @@ class Tcgen05GroupedExperts(GroupedExpertsBase):
         if isinstance(hidden_states, tuple):
             return self.forward_fp8(hidden_states, tokens_per_expert, routed_probs, expert_off)
         counts, off = self._offsets(tokens_per_expert, hidden_states.device, expert_off)
-        return _GroupedMLP.apply(hidden_states.contiguous(), self.weight1, self.weight2,
-                                 routed_probs.float().contiguous(), off, counts, self.activation)
+        x, probs = hidden_states.contiguous(), routed_probs.float().contiguous()
+        return _GroupedMLP.apply(x, self.weight1, self.weight2, probs, off, counts, self.activation)
 
     def forward_fused_combine_train(self, hidden_states, tokens_per_expert, routed_probs, buffer, handle):
         """Differentiable twin of `forward_fused_combine` (SwiGLU only)."""
@@ -173,5 +169,5 @@ class Tcgen05GroupedExperts(GroupedExpertsBase):
         if self.activation == "swiglu":
             act = G.grouped_gemm_swiglu(x, self.weight1, off, routed_probs.float().contiguous())
         else:
-            act = G.act_fwd(G.grouped_gemm(x, self.weight1, off), routed_probs.float().contiguous(), self.activation)
+            act = G.grouped_gemm_act(x, self.weight1, off, routed_probs.float().contiguous(), self.activation)
         return buffer.fused_fc2_combine(act, self.weight2, handle)

@@ -13,7 +13,7 @@ import torch
 
 from .. import _ext
 
-PLAIN, SWIGLU, COMBINE = 0, 1, 2
+PLAIN, SWIGLU, COMBINE, ACT = 0, 1, 2, 4
 
 # Default form of the kernel: True = a CTA pair (cluster of two SMs, `cta_group::2`) per tile of
 # 256 weight rows x up to 256 tokens, False = one CTA per 128 weight rows x up to 256 tokens. The
@@ -95,6 +95,26 @@ def grouped_wgrad(g: torch.Tensor, x: torch.Tensor, expert_off: torch.Tensor, *,
     use_pair = _pair(pair) and g.shape[1] % 256 == 0
     _ext.load().grouped_wgrad(g, x, expert_off, out, 0, ctas or _ctas(g.device), use_pair)
     return out
+
+
+def grouped_gemm_act(a: torch.Tensor, w: torch.Tensor, expert_off: torch.Tensor, row_prob: Optional[torch.Tensor], activation: str,
+                     *, ctas: int = 0, pair: Optional[bool] = None, band_bytes: Optional[int] = None,
+                     pre_out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """w bf16 [E, F, K]: out[r] = f(a[r] @ w[e(r)].T) * row_prob[r] -> bf16 [rows,F] for f in gelu (erf form) / silu / relu; f is
+    taken of the f32 sum. pre_out (bf16 [rows, F]): also stores a[r] @ w[e(r)].T there."""
+    out = torch.empty((a.shape[0], w.shape[1]), dtype=torch.bfloat16, device=a.device)
+    _ext.load().grouped_gemm(a, w, expert_off, ACT, out, row_prob, None, [], 0, 0, 0, -1, 0, None, 0, ctas or _ctas(a.device),
+                             _pair(pair), _band_rows(a.shape[1], band_bytes), False, pre_out, ACT_KIND[activation])
+    return out
+
+
+def grouped_gemm_dswiglu(dy: torch.Tensor, w2: torch.Tensor, expert_off: torch.Tensor, h: torch.Tensor,
+                         row_prob: Optional[torch.Tensor], *, ctas: int = 0, pair: Optional[bool] = None,
+                         band_bytes: Optional[int] = None):
+    """Data gradient of fc2 with the SwiGLU backward in its epilogue: dact = dy[r] @ w2[e(r)] (w2 bf16 [E,H,F]) stays
+    in f32 registers; -> (dh bf16 [rows,2F], dprob f32 [rows]) for act = silu(h[:, :F]) * h[:, F:] * row_prob."""
+    return _ext.load().grouped_gemm_dswiglu(dy, w2, expert_off, h, row_prob, ctas or _ctas(dy.device), _pair(pair),
+                                            _band_rows(dy.shape[1], band_bytes))
 
 
 def swiglu_fwd(h: torch.Tensor, row_prob: Optional[torch.Tensor]) -> torch.Tensor:

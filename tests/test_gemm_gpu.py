@@ -308,6 +308,55 @@ def test_grouped_wgrad_last_tile_columns(N, pair):
         r += c
 
 
+def _act_ref(h, activation):
+    f = torch.nn.functional
+    if activation == "swiglu":
+        g, l = h.chunk(2, -1)
+        return f.silu(g) * l
+    return {"gelu": f.gelu, "silu": f.silu, "relu": f.relu}[activation](h)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("activation", ["swiglu", "gelu", "silu", "relu"])
+@pytest.mark.parametrize("counts,F,H", [([1], 128, 64), ([255, 0, 257], 384, 264), ([16, 33, 0, 300, 7], 256, 512), ([700] + [3] * 39, 640, 128),
+                                        ([70, 9], 136, 72), ([40], 8, 64)])
+def test_grouped_gemm_activation_epilogues(counts, F, H, activation, pair):
+    """fc1 with an ungated activation, and the data gradient of fc2 with the SwiGLU backward, in the epilogue, against
+    f64: one row, tiles of 256 and one more, empty experts, an odd number of 128-column blocks (a pair's second CTA has
+    none), widths that end inside a block (ungated), more experts than a warp."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    if activation == "swiglu" and F % 128:
+        pytest.skip("swiglu takes multiples of 128")
+    torch.manual_seed(5)
+    rows, E = sum(counts), len(counts)
+    off = G.offsets_from_counts(counts, "cuda")
+    spans = [(int(o), int(o) + c) for o, c in zip(off.tolist(), counts)]
+    dy = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    w2 = (torch.randn(E, H, F, device="cuda") * H ** -0.5).to(torch.bfloat16)
+    h = torch.randn(rows, 2 * F if activation == "swiglu" else F, device="cuda").to(torch.bfloat16)
+    p = torch.rand(rows, device="cuda")
+    if activation == "swiglu":
+        dh, dp = G.grouped_gemm_dswiglu(dy, w2, off, h, p, pair=pair)
+        hf, pf = h.double().requires_grad_(True), p.double().requires_grad_(True)
+        dact = torch.cat([dy[a:b].double() @ w2[e].double() for e, (a, b) in enumerate(spans)])
+        gh, gp = torch.autograd.grad(_act_ref(hf, activation) * pf[:, None], [hf, pf], dact)
+        # one bf16 rounding (2^-9) of f32 results; f32 sums of F terms of order one for the probabilities
+        torch.testing.assert_close(dh.double(), gh, atol=1e-4, rtol=2 ** -8)
+        torch.testing.assert_close(dp.double(), gp, atol=1e-4 * F ** 0.5, rtol=1e-4)
+        dh1, dp1 = G.grouped_gemm_dswiglu(dy, w2, off, h, None, pair=pair)               # no probabilities: all ones
+        gh1, = torch.autograd.grad(_act_ref(hf, activation), hf, dact)
+        torch.testing.assert_close(dh1.double(), gh1, atol=1e-4, rtol=2 ** -8)
+        assert torch.equal(dp1, dp)
+    else:
+        w1 = (torch.randn(E, F, H, device="cuda") * H ** -0.5).to(torch.bfloat16)
+        pre = torch.full((rows, F), 7.0, dtype=torch.bfloat16, device="cuda")
+        act = G.grouped_gemm_act(dy, w1, off, p, activation, pair=pair, pre_out=pre)
+        ref = torch.cat([dy[a:b].double() @ w1[e].double().t() for e, (a, b) in enumerate(spans)])
+        torch.testing.assert_close(pre.double(), ref, atol=1e-4, rtol=2 ** -8)
+        torch.testing.assert_close(act.double(), _act_ref(ref, activation) * p.double()[:, None], atol=1e-4, rtol=2 ** -8)
+        assert torch.equal(G.grouped_gemm_act(dy, w1, off, p, activation, pair=pair), act)
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("counts,N,K", [([128], 256, 128), ([200, 0, 57], 384, 512), ([1, 300, 129, 0], 256, 1024),
                                         ([513], 128, 7168),
