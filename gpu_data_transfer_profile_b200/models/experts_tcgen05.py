@@ -39,16 +39,17 @@ class _GroupedMLP(torch.autograd.Function):
     tcgen05 ragged-reduction kernel."""
 
     @staticmethod
-    def forward(ctx, x, w1, w2, probs, expert_off, counts, activation):
+    def forward(ctx, x, w1, w2, probs, expert_off, counts, activation, keep):
         ctx.counts, ctx.activation = counts, activation
         ctx.off = expert_off
-        # one kernel: fc1, activation x prob in the epilogue, and the pre-activation kept for backward
-        h = torch.empty((x.shape[0], w1.shape[1]), dtype=x.dtype, device=x.device)
+        # one kernel: fc1, activation x prob in the epilogue, and the pre-activation where a backward may follow
+        h = torch.empty((x.shape[0], w1.shape[1]), dtype=x.dtype, device=x.device) if keep else None
         if activation == "swiglu":
             act = G.grouped_gemm_swiglu(x, w1, expert_off, probs, pre_out=h)
         else:
             act = G.grouped_gemm_act(x, w1, expert_off, probs, activation, pre_out=h)
-        ctx.save_for_backward(x, w1, w2, probs, h, act)
+        if keep:
+            ctx.save_for_backward(x, w1, w2, probs, h, act)
         return G.grouped_gemm(act, w2, expert_off)
 
     @staticmethod
@@ -64,7 +65,7 @@ class _GroupedMLP(torch.autograd.Function):
         dx = G.grouped_gemm(dh, w1, ctx.off, w_kn=True)                               # [rows, H]
         dw2 = _wgrad(dy[:rows], act[:rows], ctx.counts, w2.shape, ctx.off)
         dw1 = _wgrad(dh[:rows], x[:rows], ctx.counts, w1.shape, ctx.off)
-        return dx, dw1, dw2, dp, None, None, None
+        return dx, dw1, dw2, dp, None, None, None, None
 
 
 class _GroupedMLPFusedCombine(torch.autograd.Function):
@@ -147,7 +148,9 @@ class Tcgen05GroupedExperts(GroupedExpertsBase):
             return self.forward_fp8(hidden_states, tokens_per_expert, routed_probs, expert_off)
         counts, off = self._offsets(tokens_per_expert, hidden_states.device, expert_off)
         x, probs = hidden_states.contiguous(), routed_probs.float().contiguous()
-        return _GroupedMLP.apply(x, self.weight1, self.weight2, probs, off, counts, self.activation)
+        # without a backward to come the pre-activation (twice the size of the activation) is not written
+        keep = torch.is_grad_enabled() and any(t.requires_grad for t in (x, self.weight1, self.weight2, probs))
+        return _GroupedMLP.apply(x, self.weight1, self.weight2, probs, off, counts, self.activation, keep)
 
     def forward_fused_combine_train(self, hidden_states, tokens_per_expert, routed_probs, buffer, handle):
         """Differentiable twin of `forward_fused_combine` (SwiGLU only)."""
