@@ -31,7 +31,7 @@
 // 160 and 128. With tokens on M every expert was padded to a multiple of 128 or 256 rows: at 8 rows per
 // expert 31/32 of the MMA work and half of the operand traffic were padding, at 1000 rows 12 %.
 // Structure: persistent CTAs, one per SM; warp 0 = TMA producer (plain tile loads of this GPU's
-// memory; every CTA fetches its own tiles), warp 1 = MMA issuer and TMEM owner, warps 2-9 = epilogue.
+// memory; every CTA fetches its own tiles), warp 1 = MMA issuer and TMEM owner, the others = epilogue.
 // 2 TMEM accumulators (128 lanes x 256 f32 columns each) so the epilogue of tile i overlaps the MMAs
 // of tile i+1. Bound: few rows per expert: the weights, read once (32 experts x 8 rows, hidden 7168, FFN
 // 2048: fc1 + fc2 623-657 -> 437-450 us = 6.4 TB/s); many rows: the tensor pipe under the power cap

@@ -22,7 +22,9 @@
 // TFLOP/s); 1 x 16384 rows, K 4096, F 14336: 3321 -> 2225 us (1730 TFLOP/s); plain 331 -> 273 us and
 // 2509 -> 2183 us. Tried and slower: tokens on N as in the bf16 kernel (the scale then differs per
 // column: its shared-memory broadcasts cost 1024 cycles a block, 702 TFLOP/s); two MMAs of 128 columns with a
-// hand-over each (the A tile is read twice: 1593 against 1730).
+// hand-over each (the A tile is read twice: 1593 against 1730); CTA pairs, which halve a CTA's weight tile but hand over between
+// two SMs, a chain of 1700 cycles through two partials (8192 rows of the second shape 1079 us against 1004, ragged experts of 256
+// rows 404 against 338, as they pad to 256; four partials of 128 columns 1318); scales requested four blocks ahead (spills).
 // Structure per CTA (persistent, one per SM, 384 threads = three warpgroups):
 //   warp 0      TMA producer: per reduction block one 128 x 128-byte tile of A and one
 //               256 x 128-byte tile of W (128-byte swizzle), 4-stage ring; plain loads of this
