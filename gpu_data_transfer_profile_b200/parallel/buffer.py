@@ -229,6 +229,9 @@ class Buffer:
         self._carve: Optional[_Carve] = None
         self._ll = None
         self._ll_words = None
+        # The region has held rows or counters of some shape. Never False again: what is known of the present shape
+        # (`_carve`, `_ll`) says nothing about what earlier ones left behind.
+        self._region_used = False
         self.world.host_barrier()
 
     def destroy(self):
@@ -290,19 +293,20 @@ class Buffer:
     def _get_carve(self, E: int, K: int, H: int, row_bytes: int, comb_row_bytes: int) -> _Carve:
         key = (E, K, H, row_bytes, comb_row_bytes)
         if self._carve is None or self._carve.key != key:
-            if self._carve is not None or self._ll is not None:
+            c = _Carve(self.num_nvl_bytes, self.group_size, E, K, H, row_bytes, comb_row_bytes,
+                       self.num_max_recv_tokens, self.combine_slots)
+            if self._region_used:
                 self.barrier()           # region reuse with another shape: drain every rank first
-            self._ll = None
-            self._carve = _Carve(self.num_nvl_bytes, self.group_size, E, K, H, row_bytes, comb_row_bytes,
-                                 self.num_max_recv_tokens, self.combine_slots)
-            # paint the guard bands of MY region; peers store into it only after they have seen
-            # this rank's next count vector, which is stream-ordered after these fills
-            c = self._carve
-            for _, _, off, n in c.guards:
-                self.region.view(off, (n,), "uint8").fill_(CANARY)
             names = ("recv_x", "recv_scales", "recv_topk_idx", "recv_topk_w", "recv_meta", "recv_prob", "comb_x", "comb_w")
+            # (a shape is refused here or above, before anything that an earlier one left is given up)
             self._ctx.set_carve(self.peers, self.num_nvl_bytes, E, K, H, c.cap, c.slot_cap, c.flags, list(c.counts),
                                 [c.regions[0][k] for k in names], [c.regions[1][k] for k in names], c.pull_info)
+            self._region_used = True
+            self._carve, self._ll = c, None
+            # paint the guard bands of MY region; peers store into it only after they have seen
+            # this rank's next count vector, which is stream-ordered after these fills
+            for _, _, off, n in c.guards:
+                self.region.view(off, (n,), "uint8").fill_(CANARY)
         return self._carve
 
     def check_canaries(self) -> None:
@@ -773,27 +777,26 @@ class Buffer:
     def _ll_state(self, E: int, K: int, H: int, M: int):
         key = (E, K, H, M)
         if self._ll is None or self._ll["key"] != key:
-            reuse = self._ll is not None or self._carve is not None
-            carve = _LLCarve(self.num_nvl_bytes, self.group_size, E, M, H, K)
             dev = self.device
-            if reuse:
-                # the region held other data: every rank drains, clears its per-expert row counters
-                # (they must start at zero), and only then may anyone send again
-                self.barrier()
-                for off in carve.count:
-                    self.region.view(off, (E // self.group_size,), "int32").zero_()
-                self.barrier()
-            self._ll_dispatch_pending = False
             if self._ll_words is None:
                 # device-resident op state (epochs and arrival targets); lives as long as the buffer
                 # because the peers' arrival counters are cumulative
                 self._ll_words = torch.zeros(18, dtype=torch.int32, device=dev)
-            ll = dict(key=key, carve=carve, words=self._ll_words,
+            ll = dict(key=key, carve=_LLCarve(self.num_nvl_bytes, self.group_size, E, M, H, K), words=self._ll_words,
                       send_slot=torch.full((M * K,), -1, dtype=torch.int32, device=dev))
-            self._ll = self._carve = None          # (whatever lay in the region is gone, also if the shape is refused)
+            # (a shape is refused here, before anything that an earlier one left is given up)
             ll["ctx"] = self.C.LLContext(self._ll_params(ll, 0, False), self.peers, self._ll_words, ll["send_slot"],
                                          self.status_ptr)
-            self._ll = ll
+            if self._region_used:
+                # the region held other data: every rank drains, clears its per-expert row counters
+                # (they must start at zero), and only then may anyone send again
+                self.barrier()
+                for off in ll["carve"].count:
+                    self.region.view(off, (E // self.group_size,), "int32").zero_()
+                self.barrier()
+            self._region_used = True
+            self._ll_dispatch_pending = False
+            self._carve, self._ll = None, ll
         return self._ll
 
     def _ll_params(self, st, T: int, fp8: bool):

@@ -304,3 +304,64 @@ def test_low_latency_counts_of_a_group_of_one(E, M):
         g.check_status()
     finally:
         g.destroy()
+
+
+@pytest.mark.parametrize("first", ["low latency", "exchange", "both"])
+def test_low_latency_shape_after_a_refused_one(first):
+    """A shape that is refused (top-k, hidden size, a region too small, too many experts) leaves the buffer as it
+    was: what an earlier shape left in the row counters is cleared before another one counts there. Counts, sources
+    and combined rows are exact."""
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.local import LocalGroup
+    M, H, K, E = 64, 256, 4, 256
+    g = LocalGroup(1, Buffer.get_low_latency_nvl_size_hint(M, H, 1, 512, K), timeout_s=2.0)
+    gen = torch.Generator().manual_seed(3)
+
+    def inputs(T, experts, k=K, h=H):
+        return (torch.randn(T, h, generator=gen).to(torch.bfloat16).cuda(),
+                torch.stack([torch.randperm(experts, generator=gen)[:k] for _ in range(T)]).cuda())
+
+    def exchange(b):
+        x, idx = inputs(M, 8)
+        recv, _, _, _, handle, _ = b.dispatch(x, topk_idx=idx, group_by_expert=True, num_experts=8)
+        assert torch.equal(b.combine(recv, handle)[0], 4 * x)
+
+    def low_latency(b, experts):
+        x, idx = inputs(M, experts)
+        recv, count, handle, _, _ = b.low_latency_dispatch(x, idx, M, experts, use_fp8=False)
+        assert torch.equal(count.cpu().long(), torch.bincount(idx.flatten().cpu(), minlength=experts))
+        for e in idx.unique().tolist():
+            n = int(count[e])
+            _, t, k = _unpack(handle[0][e, :n].long())
+            assert n == len(set(t.tolist())) and torch.equal(idx[t, k], torch.full_like(t, e)) and torch.equal(recv[e, :n], x[t])
+        out, _, _ = b.low_latency_combine(recv, idx, torch.ones(M, K, device="cuda"), handle)
+        assert torch.equal(out, 4 * x)
+
+    try:
+        b = g.buffers[0]
+        if first != "low latency":
+            exchange(b)
+        for _ in range(2 * (first != "exchange")):
+            low_latency(b, 512)
+        for _ in range(2):
+            x, idx = inputs(2, 64, 33)
+            with pytest.raises(RuntimeError):
+                b.low_latency_dispatch(x, idx, M, 64, use_fp8=False)
+            x, idx = inputs(2, 64, 33)
+            with pytest.raises(RuntimeError):
+                b.dispatch(x, topk_idx=idx, group_by_expert=True, num_experts=64)
+            x, idx = inputs(2, E, K, 100)
+            with pytest.raises(RuntimeError):
+                b.low_latency_dispatch(x, idx, M, E, use_fp8=False)
+            x, idx = inputs(2, E)
+            with pytest.raises(ValueError):
+                b.low_latency_dispatch(x, idx, 100 * M, E, use_fp8=False)
+            with pytest.raises(ValueError):
+                b.dispatch(x, topk_idx=idx, group_by_expert=True, num_experts=1 << 20)
+        for _ in range(3):
+            low_latency(b, E)
+        exchange(b)
+        low_latency(b, 512)
+        b.check_status()
+    finally:
+        g.destroy()
