@@ -528,15 +528,22 @@ int launch_grouped_gemm(const void* a, long long a_rows, const void* w, int epi,
   if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(w) % 16) return 1;
   if ((epi == EPI_SWIGLU || epi == EPI_DSWIGLU) && (p.N % 128)) return 1;
   if (epi == EPI_ACT && (p.act_kind < 0 || p.act_kind > 2)) return 1;
+  if (p.b_mn && epi != EPI_PLAIN && epi != EPI_DSWIGLU) return 1;
+  // No rows (no tokens, or a rank that none was sent to): nothing to compute, and a tensor map may not be empty. The combine
+  // epilogue has its flag to raise all the same: its map names one row of the weights, which no tile reads.
+  const long long map_rows = a_rows > 0 ? a_rows : 1;
+  if (a_rows == 0) {
+    if (epi != EPI_COMBINE || p.signal_flag_off < 0) return 0;
+    a = w;
+  }
   if (epi == EPI_DSWIGLU && (!p.b_mn || p.pre_out == nullptr || p.dp_part == nullptr)) return 1;
   // 64-column boxes (one 128-byte swizzle row): the tokens in four heights, so that a small tile fetches no more
   // rows than it needs; the weights 128 rows high, 64 where a CTA's rows come from two places
   TokenMaps ma;
   CUtensorMap mb;
   for (int b = 0; b < TOKEN_BOXES; ++b)
-    if (make_tmap_bf16(&ma.m[b], a, a_rows, p.K, BK, 16 << b)) return 3;
+    if (make_tmap_bf16(&ma.m[b], a, map_rows, p.K, BK, 16 << b)) return 3;
   if (p.b_mn) {
-    if (epi != EPI_PLAIN && epi != EPI_DSWIGLU) return 1;
     if (make_tmap_bf16(&mb, w, (long long)p.El * p.w_rows, p.N, 64, BK)) return 3;
   } else if (make_tmap_bf16(&mb, w, (long long)p.El * p.w_rows, p.K, BK, epi == EPI_SWIGLU ? 64 : WM)) return 3;
   const int tile_cols = (pair ? 2 : 1) * (epi == EPI_SWIGLU ? 64 : WM);       // output columns per tile

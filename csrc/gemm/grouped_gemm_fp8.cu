@@ -378,9 +378,10 @@ int launch_grouped_gemm_fp8(const void* a, long long a_rows, const void* w, int 
   using namespace f8;
   if (p.El < 1 || p.El > kMaxLocalExperts || p.K <= 0 || p.K % BKB || p.N <= 0 || p.N % 128 || p.N_out % 8) return 1;
   if ((long long)p.El * (p.w_rows / 128) * (p.K / BKB) > 0x7fffffff) return 1;
-  if (p.w_rows % 128 || p.sa == nullptr || p.sw == nullptr || p.sa_ld < p.K / BKB) return 1;
+  if (p.w_rows % 128 || (epi != EPI_PLAIN && epi != EPI_SWIGLU)) return 1;
+  if (a_rows == 0) return 0;                          // nothing to compute (a tensor map may not be empty)
+  if (p.sa == nullptr || p.sw == nullptr || p.sa_ld < p.K / BKB) return 1;
   if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(w) % 16) return 1;
-  if (epi != EPI_PLAIN && epi != EPI_SWIGLU) return 1;
   CUtensorMap ma, mb;
   if (make_map_u8(&ma, a, a_rows, p.K, BM)) return 3;
   if (make_map_u8(&mb, w, (long long)p.El * p.w_rows, p.K, 128)) return 3;

@@ -444,3 +444,29 @@ def test_grouped_gemms_work_from_a_fresh_thread():
             torch.testing.assert_close(out[r:r + c].float(), a[r:r + c].float() @ w[e].float().t(), atol=3e-2, rtol=3e-2)
             torch.testing.assert_close(dx[r:r + c].float(), g[r:r + c].float() @ w[e].float(), atol=3e-2, rtol=3e-2)
         r += c
+
+
+@pytest.mark.parametrize("activation", ["swiglu", "gelu"])
+def test_experts_without_rows(activation):
+    """No rows at all (no tokens, or a rank that none was sent to): empty outputs and zero weight gradients."""
+    from gpu_data_transfer_profile_b200.models.experts_tcgen05 import Tcgen05GroupedExperts
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    E, H, F = 3, 256, 128
+    m = Tcgen05GroupedExperts(E, H, F, activation=activation, use_fp8=True)
+    x = torch.empty(0, H, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    p = torch.empty(0, device="cuda", requires_grad=True)
+    for pair in (False, True):
+        off = G.offsets_from_counts([0] * E, "cuda")
+        assert G.grouped_gemm(x.detach(), m.weight1, off, pair=pair).shape == (0, m.weight1.shape[1])
+        assert G.grouped_gemm(x.detach(), m.weight2, off, pair=pair, w_kn=True).shape == (0, F)
+        dh, dp = G.grouped_gemm_dswiglu(x.detach(), m.weight2, off, torch.empty(0, 2 * F, device="cuda", dtype=torch.bfloat16), None, pair=pair)
+        assert dh.shape == (0, 2 * F) and dp.shape == (0,)
+    y = m(x, [0] * E, p)
+    assert y.shape == (0, H)
+    y.float().sum().backward()
+    assert x.grad.shape == x.shape and p.grad.shape == p.shape
+    for w in (m.weight1, m.weight2):
+        assert w.grad.shape == w.shape and not w.grad.any()
+    q = torch.empty(0, H, device="cuda").to(torch.float8_e4m3fn)
+    assert m((q, torch.empty(0, H // 128, device="cuda")), [0] * E, p.detach()).shape == (0, H)
+    torch.cuda.synchronize()

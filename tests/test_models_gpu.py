@@ -390,3 +390,36 @@ def test_training_router_matches_the_torch_form(T, E, K):
     lt = l.detach().clone().requires_grad_(True)
     (gt,) = torch.autograd.grad(topk_softmax_router(lt, K)[1], lt, gw)
     assert bool(g[-1].isnan().all()) and bool(gt[-1].isnan().all()) and not bool(g[:-1].isnan().any())
+
+
+@pytest.mark.parametrize("use_fp8,fuse", [(False, True), (True, True), (False, False)])
+@pytest.mark.parametrize("activation", ["swiglu", "silu"])
+def test_moe_layer_without_tokens(use_fp8, fuse, activation):
+    """A batch of no tokens between ordinary ones: empty outputs, zero gradients, and calls before and after it agree."""
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A
+    from gpu_data_transfer_profile_b200.models.moe_layer import MoELayer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    torch.manual_seed(0)
+    world = LocalWorld.make(1)[0]
+    A.configure_buffer(num_max_tokens_per_rank=128, num_topk=2, num_experts=4, group_by_expert=True)
+    try:
+        layer = MoELayer(256, 128, 4, 2, None, activation=activation, expert_backend="tcgen05", world=world,
+                         use_fp8=use_fp8, fuse_combine=fuse)
+        x = torch.randn(65, 256, device="cuda").to(torch.bfloat16)
+        none = x[:0].detach()
+        with torch.no_grad():
+            want = layer(x)
+            assert layer(none).shape == (0, 256)
+            assert torch.equal(layer(x), want)
+        leaf = none.clone().requires_grad_(True)
+        out = layer(leaf)
+        assert out.shape == (0, 256)
+        out.float().sum().backward()
+        assert leaf.grad.shape == (0, 256)
+        for w in (layer.router.weight, layer.experts.weight1, layer.experts.weight2):
+            assert w.grad.shape == w.shape and not w.grad.any()
+        with torch.no_grad():
+            assert torch.equal(layer(x), want)
+        A._BUFFERS[(id(None), id(world))].check_status()
+    finally:
+        A.release_buffers()
