@@ -470,3 +470,16 @@ def test_experts_without_rows(activation):
     q = torch.empty(0, H, device="cuda").to(torch.float8_e4m3fn)
     assert m((q, torch.empty(0, H // 128, device="cuda")), [0] * E, p.detach()).shape == (0, H)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("H,E", [(12, 2), (64, 257)])
+def test_grouped_gemm_dswiglu_refuses_bad_shapes(H, E):
+    """A width that tensor maps do not take, more experts than the kernel's tables hold: an error that a program can catch."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    F, rows = 128, 4
+    dy = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    w2 = torch.randn(E, H, F, device="cuda").to(torch.bfloat16)
+    h = torch.randn(rows, 2 * F, device="cuda").to(torch.bfloat16)
+    off = G.offsets_from_counts([rows] + [0] * (E - 1), "cuda")
+    with pytest.raises(RuntimeError, match="invalid arguments"):
+        G.grouped_gemm_dswiglu(dy, w2, off, h, None)
