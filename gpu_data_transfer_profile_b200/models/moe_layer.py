@@ -39,13 +39,15 @@ class _TopkSoftmax(torch.autograd.Function):
     @staticmethod
     def backward(ctx, _grad_idx, grad_w):
         idx, w = ctx.saved_tensors
-        if torch.is_grad_enabled():          # a graph of the backward is asked for
+        if torch.is_grad_enabled() or _carries_more(grad_w):          # a graph, a tangent or a batch of gradients is asked for
             d = w * (grad_w - (w * grad_w).sum(-1, keepdim=True))
             return torch.zeros((w.shape[0], ctx.num_experts), dtype=w.dtype, device=w.device).scatter(1, idx, d), None
         return _ext.load().topk_softmax_bwd(idx, w, grad_w.float().contiguous(), ctx.num_experts), None
 
 
 _LINEAR_FORWARD = torch.nn.Linear.forward
+# a program that puts a router of its own in its place has it called
+_OWN_ROUTER = topk_softmax_router
 
 
 def _plain_linear(m: torch.nn.Module) -> bool:
@@ -70,9 +72,11 @@ def _unchanged(obj, methods) -> bool:
 
 
 def _carries_more(t: Optional[torch.Tensor]) -> bool:
-    """A tensor with a forward-mode tangent or inside a function transform: the inference path, which knows nothing of
-    either, would drop what it carries without a word; the autograd functions of the general path refuse it."""
-    return t is not None and (torch._C._functorch.is_functorch_wrapped_tensor(t) or unpack_dual(t).tangent is not None)
+    """A tensor with a forward-mode tangent or inside a function transform (a batch of gradients is one, in a form of its
+    own): kernels, which know nothing of either, would drop what it carries without a word or fail on it; the autograd
+    functions of the general path refuse it."""
+    F = torch._C._functorch
+    return t is not None and (F.is_functorch_wrapped_tensor(t) or F.is_legacy_batchedtensor(t) or unpack_dual(t).tangent is not None)
 
 
 class MoELayer(torch.nn.Module):
@@ -105,7 +109,7 @@ class MoELayer(torch.nn.Module):
             if router_logits is None:
                 router_logits = self.router(hidden_states.float())
             l = router_logits
-            if (not inference and type(l) is torch.Tensor and l.is_cuda and l.dim() == 2 and 1 <= K <= min(32, l.shape[1])
+            if (not inference and topk_softmax_router is _OWN_ROUTER and type(l) is torch.Tensor and l.is_cuda and l.dim() == 2 and 1 <= K <= min(32, l.shape[1])
                     and l.get_device() == torch.cuda.current_device() and l.shape[1] <= _ext.load().ROUTER_MAX_EXPERTS and not _carries_more(l)
                     and not torch.compiler.is_compiling() and not torch.jit.is_tracing()):
                 return _TopkSoftmax.apply(l.float().contiguous(), K)
@@ -123,8 +127,8 @@ class MoELayer(torch.nn.Module):
 
     def forward(self, hidden_states: torch.Tensor, router_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
         """hidden_states [T,H]; router_logits [T,E] override the learnable router when given."""
-        inference = not (torch.is_grad_enabled() or _carries_more(hidden_states) or _carries_more(router_logits)
-                         or _carries_more(getattr(self.router, "weight", None)))
+        inference = not (torch.is_grad_enabled() or topk_softmax_router is not _OWN_ROUTER or _carries_more(hidden_states)
+                         or _carries_more(router_logits) or _carries_more(getattr(self.router, "weight", None)))
         idx, probs = self._route(hidden_states, router_logits, inference)
         if (inference and self.dispatcher.mode == "fused" and hidden_states.dtype == torch.bfloat16
                 and (self.use_fp8 or self.fuse_combine)

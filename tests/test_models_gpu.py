@@ -423,3 +423,62 @@ def test_moe_layer_without_tokens(use_fp8, fuse, activation):
         A._BUFFERS[(id(None), id(world))].check_status()
     finally:
         A.release_buffers()
+
+
+def test_training_router_gradient_of_batches_and_tangents():
+    """A batch of incoming gradients (both forms of it) and one with a tangent, as the torch form takes them."""
+    from torch.autograd import forward_ad
+    from gpu_data_transfer_profile_b200.models.moe_layer import _TopkSoftmax, topk_softmax_router
+    T, E, K, B = 9, 8, 3, 4
+    gen = torch.Generator().manual_seed(7)
+    logits = torch.randn(T, E, generator=gen).cuda()
+    gw = torch.randn(B, T, K, generator=gen).cuda()
+
+    def grads(router):
+        l = logits.clone().requires_grad_(True)
+        w = router(l, K)[1]
+        one = lambda g: torch.autograd.grad(w, l, g, retain_graph=True)[0]
+        batch = torch.autograd.grad(w, l, gw, retain_graph=True, is_grads_batched=True)[0]
+        mapped = torch.func.vmap(one)(gw)
+        with forward_ad.dual_level():
+            dual = forward_ad.unpack_dual(one(forward_ad.make_dual(gw[0], gw[1])))
+            return torch.stack([one(g) for g in gw]), batch, mapped, dual.primal.clone(), dual.tangent.clone()
+
+    want = grads(topk_softmax_router)
+    for got, ref in zip(grads(_TopkSoftmax.apply), want):
+        # f32 softmax and its gradient: a few units of 2^-24 relative to the incoming gradient
+        torch.testing.assert_close(got, ref, atol=2 ** -18 * float(gw.abs().max()), rtol=0)
+
+
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("given", [False, True])
+def test_moe_layer_calls_a_router_put_in_place_of_its_own(train, given, monkeypatch):
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A, moe_layer as M
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    torch.manual_seed(0)
+    A.configure_buffer(num_max_tokens_per_rank=128, num_topk=2, num_experts=4, group_by_expert=True)
+    seen = []
+
+    def fixed(logits, topk):                                  # the same two experts for every token, one choice masked
+        seen.append(tuple(logits.shape))
+        idx = torch.arange(topk, device=logits.device).repeat(logits.shape[0], 1)
+        idx[0, 1] = -1
+        return idx, torch.ones(idx.shape, device=logits.device)
+
+    try:
+        layer = M.MoELayer(256, 128, 4, 2, None, expert_backend="tcgen05", world=LocalWorld.make(1)[0])
+        x = torch.randn(65, 256, device="cuda").to(torch.bfloat16)
+        logits = torch.randn(65, 4, device="cuda") if given else None
+        monkeypatch.setattr(M, "topk_softmax_router", fixed)
+        with torch.set_grad_enabled(train):
+            y = layer(x, logits).detach()
+        assert seen == [(65, 4)]
+        counts = [65, 64, 0, 0]
+        rows = torch.cat([x, x[1:]])
+        with torch.no_grad():
+            z = layer.experts(rows, counts, torch.ones(129, device="cuda")).float()
+        want = z[:65]
+        want[1:] += z[65:]
+        torch.testing.assert_close(y.float(), want, rtol=2.0 ** -6, atol=2.0 ** -8 * float(want.abs().max()))
+    finally:
+        A.release_buffers()
