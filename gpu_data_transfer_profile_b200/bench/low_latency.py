@@ -31,8 +31,9 @@ def main() -> int:
     ap.add_argument("--warmup-iters", type=int, default=10)
     ap.add_argument("--benchmark-iters", type=int, default=100)
     ap.add_argument("--num-sms", type=int, default=32)
-    ap.add_argument("--overlap-launches", action="store_true",
-                    help="launch the kernels with programmatic stream serialisation (launch latencies overlap)")
+    ap.add_argument("--overlap-launches", action=argparse.BooleanOptionalAction, default=None,
+                    help="launch the kernels with programmatic stream serialisation (launch latencies overlap); "
+                         "default: by group size")
     ap.add_argument("--signal-mode", type=int, choices=(0, 1), default=None,
                     help="0: every send CTA signals every peer; 1: the last CTA does; default: by group size")
     ap.add_argument("--combine", choices=("pull", "push"), default="pull",

@@ -769,10 +769,10 @@ class Buffer:
     # are placed while its predecessor still runs and wait in their first instruction until it has
     # completed, so launch latencies overlap (also inside a captured CUDA graph). On one GPU a replay of
     # 128 fp8 tokens takes 12.3 us either way, of 128 bf16 tokens 14.3 -> 13.9, of one token 11.5 -> 10.3, an eager
-    # round 27.2 -> 26.3 us (one set of inputs, back to back). A group of one always does so. Off by default for others
+    # round 27.2 -> 26.3 us (one set of inputs, back to back). None = by group size: on in a group of one, off for others
     # because of the last measurement with 2 ranks, taken while the receive half was a launch of its own: eager
     # dispatch got slower there (45 -> 54 us).
-    ll_overlap_launches: bool = False
+    ll_overlap_launches: Optional[bool] = None
 
     def _ll_state(self, E: int, K: int, H: int, M: int):
         key = (E, K, H, M)
@@ -812,7 +812,7 @@ class Buffer:
         return (1 if self.group_size >= 8 else 0) if Buffer.ll_signal_mode is None else int(Buffer.ll_signal_mode)
 
     def _ll_overlap(self) -> bool:
-        return bool(Buffer.ll_overlap_launches) or self.group_size == 1
+        return self.group_size == 1 if Buffer.ll_overlap_launches is None else bool(Buffer.ll_overlap_launches)
 
     def _ll_dispatch_send(self, x, topk_idx, M, E, use_fp8, fused=False):
         """fused: the same launch also does the receive half (its last CTA waits for the peers)."""

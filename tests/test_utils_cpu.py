@@ -312,3 +312,16 @@ def test_fused_router_stands_in_for_an_untouched_linear_only(monkeypatch):
     forward = torch.nn.Linear.forward
     monkeypatch.setattr(torch.nn.Linear, "forward", lambda self, x: forward(self, x) + 1)
     assert not _plain_linear(plain)
+
+
+def test_low_latency_launch_overlap_can_be_switched_either_way(monkeypatch):
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    assert Buffer.ll_overlap_launches is None
+    for size in (1, 2, 8):
+        b = object.__new__(Buffer)
+        b.group_size = size
+        assert b._ll_overlap() is (size == 1)                 # the default goes by group size
+        for on in (False, True):
+            with monkeypatch.context() as m:
+                m.setattr(Buffer, "ll_overlap_launches", on)
+                assert b._ll_overlap() is on
