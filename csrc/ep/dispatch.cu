@@ -281,8 +281,11 @@ dispatch_send_kernel(EpGeom g, EpRegions rg, const __grid_constant__ PeerPtrs pe
         char* pb = peers.base[d];
         if (part == 0) {
           reinterpret_cast<int2*>(pb + rg.recv_meta)[row] = make_int2(slot, g.rank);
-          if (MODE == 1)
-            reinterpret_cast<float*>(pb + rg.recv_prob)[row] = topk_w ? topk_w[(size_t)t * K + lane] : 1.f;
+          if (MODE == 1) {
+            const float w = topk_w ? topk_w[(size_t)t * K + lane] : 1.f;
+            reinterpret_cast<float*>(pb + rg.recv_prob)[row] = w;
+            if (!CACHED && rg.own_prob != 0) reinterpret_cast<float*>(pb + rg.own_prob)[row] = w;
+          }
         }
         s_dst[warp][lane] = pb + rg.recv_x + (size_t)row * row_bytes_out;
         s_scl[warp][lane] = reinterpret_cast<float*>(pb + rg.recv_scales) + (size_t)row * scale_cols;

@@ -43,6 +43,7 @@ struct EpRegions {
   long long recv_topk_w;   // float [cap][K]
   long long recv_meta;     // int2  [cap]  {slot at source, source rank}
   long long recv_prob;     // float [cap]
+  long long own_prob;      // float [cap] or 0: a second place for the probabilities (a group of one)
   long long comb_x;        // bytes [slot_cap][comb_row_bytes]
   long long comb_w;        // float [slot_cap][K]
   long long pull_info;     // int64 [kMaxRanks][4]: where rank d keeps the rows that a pulling combine reads

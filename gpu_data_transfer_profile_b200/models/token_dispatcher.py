@@ -143,8 +143,8 @@ class B200TokenDispatcher:
         weights = token_probs.contiguous().float()
         # (what callers may look at later is their own; the rows' view is for the computation)
         if worst and getattr(type(buf), "dispatch", None) is _BUFFER_DISPATCH and "dispatch" not in vars(buf):
-            rows, handle = buf._dispatch_own_probs(x, idx, weights, self.num_experts, use_fp8, worst)
-            self.handle, self.dispatched_probs = handle, handle.recv_prob
+            rows, handle, self.dispatched_probs = buf._dispatch_own_probs(x, idx, weights, self.num_experts, use_fp8, worst)
+            self.handle = handle
         else:
             rows, _, _, _, handle, _ = buf.dispatch(
                 x, topk_idx=idx, topk_weights=weights, group_by_expert=True,

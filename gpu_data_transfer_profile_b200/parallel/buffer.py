@@ -501,7 +501,7 @@ class Buffer:
                        st["meta"], st["x"], st["fp8"], st["cached"], st["topk_idx"], st.get("topk_weights"), st["send_row"],
                        st["send_slot"], st["scales_in"], own, own_probs)
 
-    def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1, own_probs: int = 0):
+    def _dispatch_p3(self, st, zero_copy: bool, num_worst_tokens: int = 0, expert_alignment: int = 1):
         R, E, K, H = self.group_size, st["E"], st["K"], st["H"]
         El = E // R
         carve = st["carve"]
@@ -534,10 +534,7 @@ class Buffer:
             self._poll_status()       # the host already waited for the kernel's prologue: cheap to look
         side = st["mode"] == 0 and st["topk_idx"] is not None
         n_x = 2 if st["fp8_out"] else 1
-        if own_probs:
-            views = self._region_outputs(st, carve, n_recv, side)
-            views[n_x] = st["own"][0]
-        elif st["own"]:
+        if st["own"] and not zero_copy:
             views = st["own"]
             if views[0].shape[0] != n_recv:
                 # masked choices: tensors of the exact size, so that the rows nobody sent keep no memory (nor come
@@ -615,14 +612,14 @@ class Buffer:
 
     @_nvtx("b200ep.dispatch")
     def _dispatch_own_probs(self, x, topk_idx, topk_weights, num_experts: int, use_fp8: bool, rows: int):
-        """A group of one, expert mode: `rows` rows (the number of choices) in the region, their probabilities in a tensor
-        of the caller's own. -> (recv_x | (recv_x_fp8, scales), handle)"""
+        """A group of one, expert mode, zero copy: `rows` rows (the number of choices), their probabilities in the region
+        and in a tensor of the caller's own. -> (recv_x | (recv_x_fp8, scales), handle, probabilities)"""
         self._enter(None, False, False)
         with self._on_stream():
             st = self._dispatch_p1(x, None, None, None, topk_idx, topk_weights, use_fp8, True, num_experts)
             self._dispatch_p2(st, True, rows, rows)
-            recv_x, _, _, _, handle = self._dispatch_p3(st, True, rows, 1, rows)
-        return recv_x, handle
+            recv_x, _, _, _, handle = self._dispatch_p3(st, True, rows)
+        return recv_x, handle, st["own"][0]
 
     # ---- combine ---------------------------------------------------------------------
     def _combine_prepare(self, x, handle: DispatchHandle, topk_weights):

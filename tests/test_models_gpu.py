@@ -482,3 +482,38 @@ def test_moe_layer_calls_a_router_put_in_place_of_its_own(train, given, monkeypa
         torch.testing.assert_close(y.float(), want, rtol=2.0 ** -6, atol=2.0 ** -8 * float(want.abs().max()))
     finally:
         A.release_buffers()
+
+
+@pytest.mark.parametrize("slots", [True, False])
+@pytest.mark.parametrize("T,K", [(1, 1), (65, 3)])
+def test_dispatch_in_place_keeps_what_a_pulling_combine_reads_in_the_region(slots, T, K):
+    """Rows and probabilities of a dispatch in place go back to their tokens without a copy (all that a buffer without
+    combine slots can do); the dispatcher's record of the probabilities is a tensor of its own."""
+    from gpu_data_transfer_profile_b200.models import fused_a2a as A
+    from gpu_data_transfer_profile_b200.models.token_dispatcher import B200TokenDispatcher
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.symm import LocalWorld
+    H, E = 256, 8
+    world = LocalWorld.make(1)[0]
+    A.configure_buffer(num_max_tokens_per_rank=T, num_topk=K, num_experts=E, group_by_expert=True)
+    try:
+        buf = Buffer(None, 64 << 20, world=world, timeout_s=2.0, combine_slots=slots)
+        A.set_buffer(None, buf, world)
+        d = B200TokenDispatcher(None, E, E, 0, world=world)
+        g = torch.Generator().manual_seed(T)
+        for _ in range(3):
+            x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+            idx, w = torch.rand(T, E, generator=g).topk(K, dim=-1).indices.cuda(), torch.rand(T, K, generator=g).cuda()
+            rows, probs, handle = d.dispatch_in_place(x, idx, w)
+            own = d.dispatched_probs
+            order = torch.sort(idx.flatten(), stable=True).indices
+            assert torch.equal(rows, x[order // K]) and torch.equal(probs, w.flatten()[order]) and torch.equal(own, probs)
+            out, back, _ = buf.combine(rows, handle, topk_weights=probs)
+            assert torch.equal(back, w)
+            torch.testing.assert_close(out.float(), K * x.float(), rtol=2.0 ** -8, atol=0)
+            probs.zero_()
+            assert torch.equal(own, w.flatten()[order])
+        buf.check_status()
+        buf.check_canaries()
+    finally:
+        A.release_buffers()
