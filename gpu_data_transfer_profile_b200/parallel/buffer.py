@@ -295,6 +295,8 @@ class Buffer:
         if self._carve is None or self._carve.key != key:
             c = _Carve(self.num_nvl_bytes, self.group_size, E, K, H, row_bytes, comb_row_bytes,
                        self.num_max_recv_tokens, self.combine_slots)
+            if c.cap <= 0:               # (not even the guard bands have to fit then)
+                raise ValueError("num_nvl_bytes too small for this hidden size")
             if self._region_used:
                 self.barrier()           # region reuse with another shape: drain every rank first
             names = ("recv_x", "recv_scales", "recv_topk_idx", "recv_topk_w", "recv_meta", "recv_prob", "comb_x", "comb_w")
@@ -461,8 +463,6 @@ class Buffer:
         elem = 2 if st["fp8_out"] else x.element_size()
         carve = self._get_carve(E, K, H, H * elem, H * elem)
         st["carve"] = carve
-        if carve.cap <= 0:
-            raise ValueError("num_nvl_bytes too small for this hidden size")
         J, B = (R, R) if mode == 0 else (K, E)
         st.update(J=J, B=B, row_bytes_out=row_bytes_out)
         if st["cached"]:

@@ -325,3 +325,36 @@ def test_low_latency_launch_overlap_can_be_switched_either_way(monkeypatch):
             with monkeypatch.context() as m:
                 m.setattr(Buffer, "ll_overlap_launches", on)
                 assert b._ll_overlap() is on
+
+
+def test_a_shape_without_room_for_a_row_leaves_region_and_layout_alone():
+    """Refused before a byte of the region is painted (in the smallest regions its guard bands would lie behind the end)
+    and before the layout of an earlier shape is given up."""
+    import types
+    import pytest
+    from gpu_data_transfer_profile_b200.parallel.buffer import Buffer
+    from gpu_data_transfer_profile_b200.parallel.config import FIXED_BYTES, REGION_ALIGN
+    for extra, kept in ((REGION_ALIGN, False), (64 * REGION_ALIGN, True)):
+        nbytes = FIXED_BYTES + extra
+        painted = []
+
+        def view(off, shape, dtype):
+            assert dtype == "uint8" and 0 <= off and off + shape[0] <= nbytes
+            painted.append(off)
+            return types.SimpleNamespace(fill_=lambda v: None)
+
+        b = object.__new__(Buffer)
+        b.num_nvl_bytes, b.group_size, b.num_max_recv_tokens, b.combine_slots = nbytes, 1, 0, True
+        b._carve = b._ll = None
+        b._region_used = False
+        b.barrier = lambda: painted.append("barrier")
+        b.region = types.SimpleNamespace(view=view, peer_ptrs=[1])
+        b._ctx = types.SimpleNamespace(set_carve=lambda *a: painted.append("layout"))
+        if kept:
+            first = b._get_carve(8, 2, 256, 512, 512)
+            assert first.cap > 0 and "layout" in painted
+            painted.clear()
+        for _ in range(2):
+            with pytest.raises(ValueError, match="too small"):
+                b._get_carve(8, 2, 1 << 20, 1 << 21, 1 << 21)
+        assert not painted and b._region_used is kept and (b._carve is first if kept else b._carve is None)
