@@ -3,6 +3,18 @@
 
 namespace b200ep {
 
+// 1 / (1 + exp(-x)): the hardware's approximate reciprocal (within 1 ulp, subnormal results included) and one step of
+// Newton's iteration r + r (1 - y r) in fused multiply-adds, which leaves an error of half an ulp and a little, as a
+// rounded division does; where exp overflows the approximation, 0, is the result. The division itself takes a branch for
+// its rare cases, and the epilogues that use it then take longer than their tiles' MMAs: data gradient of 12001 rows, 16
+// experts, 2048 x 1408 101 us with it, 79 so; fc1 of the same with silu 76 and 66.
+__device__ __forceinline__ float sigmoid(float x) {
+  const float y = 1.f + __expf(-x);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return y < __int_as_float(0x7f800000) ? fmaf(r, fmaf(-y, r, 1.f), r) : r;
+}
+
 // kind: 0 gelu (erf form, as torch.nn.functional.gelu), 1 silu, 2 relu.
 __device__ __forceinline__ void act_eval(int kind, float x, float* f, float* df) {
   if (kind == 0) {
@@ -11,7 +23,7 @@ __device__ __forceinline__ void act_eval(int kind, float x, float* f, float* df)
     *f = x * cdf;
     *df = cdf + x * pdf;
   } else if (kind == 1) {
-    const float sig = 1.f / (1.f + __expf(-x));
+    const float sig = sigmoid(x);
     *f = x * sig;
     *df = sig * (1.f + x * (1.f - sig));
   } else {

@@ -125,7 +125,7 @@ __device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 
 // Backward of silu(g) * l * prob for one element: d = gradient of the product; the gradients of g and l come back in
 // place of g and l, the element's share of the probability's gradient is returned.
 __device__ __forceinline__ float dswiglu(float d, float pr, float& g, float& l) {
-  const float sig = __fdividef(1.f, 1.f + __expf(-g));      // (within 2 ulp; what comes of it leaves as bf16)
+  const float sig = sigmoid(g);
   const float s = g * sig, da = d * pr, share = d * s * l;
   g = da * l * sig * (1.f + g * (1.f - sig));
   l = da * s;
@@ -144,7 +144,6 @@ __device__ __forceinline__ float dswiglu4(const float4& d, float pr, uint2& hg, 
   return share;
 }
 __device__ __forceinline__ float act_only(int kind, float x) {
-  if (kind == 1) return x * __fdividef(1.f, 1.f + __expf(-x));      // (within 2 ulp; what comes of it leaves as bf16)
   float f, df;
   act_eval(kind, x, &f, &df);
   return f;

@@ -483,3 +483,54 @@ def test_grouped_gemm_dswiglu_refuses_bad_shapes(H, E):
     off = G.offsets_from_counts([rows] + [0] * (E - 1), "cuda")
     with pytest.raises(RuntimeError, match="invalid arguments"):
         G.grouped_gemm_dswiglu(dy, w2, off, h, None)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_activation_epilogues_divide_where_the_sigmoid_is_subnormal(pair):
+    """Gates between -88.7 and -87.4: 1 + exp(-x) lies above 2^126, the sigmoid is a subnormal f32, silu and its
+    gradients are ordinary bf16 numbers of about 1e-37. Identity weights bring the values to the epilogues as they are."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    F, rows = 128, 5
+    off = G.offsets_from_counts([rows], "cuda")
+    eye = torch.eye(F, device="cuda").to(torch.bfloat16)[None]
+    g = torch.tensor([-87.5, -88.0, -88.5, -3.0, 2.0], device="cuda").to(torch.bfloat16)[:, None].expand(rows, F).contiguous()
+    one = torch.ones(rows, F, device="cuda", dtype=torch.bfloat16)
+    x = g.double()
+    silu, sig = x / (1 + (-x).exp()), 1 / (1 + (-x).exp())
+    assert bool((silu[:3].abs() > 2.0 ** -126).all()) and bool((sig[:3] < 2.0 ** -126).all())
+    # one bf16 rounding, and exp of an argument of 88 from the fast exponential (88 x 2^-22 relative)
+    bound = dict(rtol=2.0 ** -8, atol=0)
+    torch.testing.assert_close(G.grouped_gemm_act(g, eye, off, None, "silu", pair=pair).double(), silu, **bound)
+    dh, dp = G.grouped_gemm_dswiglu(one, eye, off, torch.cat([g, one], 1), None, pair=pair)
+    torch.testing.assert_close(dh[:, F:].double(), silu, **bound)
+    torch.testing.assert_close(dh[:, :F].double(), sig * (1 + x * (1 - sig)), **bound)
+    torch.testing.assert_close(dp.double(), silu.sum(1), rtol=2.0 ** -12, atol=0)
+
+
+def test_epilogue_sigmoid_is_as_near_as_a_rounded_division():
+    """silu of every finite bf16 gate as an f32 number (a row's sum for the gradient of its probability, one term not
+    zero), from the epilogue and from the element-wise kernel, which divides."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    F = 128
+    g = torch.arange(1 << 16, device="cuda").to(torch.int32).to(torch.int16).view(torch.bfloat16)
+    g = g[g.isfinite()]
+    rows = g.numel()
+    at = (torch.arange(rows, device="cuda"), torch.arange(rows, device="cuda") % F)
+    dy = torch.zeros(rows, F, device="cuda", dtype=torch.bfloat16)
+    gate = torch.zeros_like(dy)
+    dy[at], gate[at] = 1, g
+    h = torch.cat([gate, dy], 1)
+    eye = torch.eye(F, device="cuda").to(torch.bfloat16)[None]
+    dh, dp = G.grouped_gemm_dswiglu(dy, eye, G.offsets_from_counts([rows], "cuda"), h, None)
+    dh1, dp1 = G.swiglu_bwd(h, None, dy)
+    # sigmoids within an ulp of each other and a product rounded in both: two ulps, or two of the smallest subnormal times
+    # the gate; the gradient of the gate is a bf16 number, 1 + g (1 - sigmoid) cancels near -1.28
+    bound = 2.0 ** -22 * dp1.double().abs() + 2.0 ** -148 * g.double().abs()
+    assert bool(((dp.double() - dp1.double()).abs() <= bound).all())
+    torch.testing.assert_close(dh.float(), dh1.float(), rtol=2.0 ** -7, atol=2.0 ** -20)
+    # no further from 64 bits than the division's, down to where exp overflows
+    x = g.double()
+    silu = x / (1 + (-x).exp())
+    normal = (silu.abs() > 2.0 ** -126) & (x > -88.7)
+    err = [((d.double() - silu).abs() / silu.abs())[normal] for d in (dp, dp1)]
+    assert float(err[0].mean()) <= float(err[1].mean()) * (1 + 2.0 ** -6) and float(err[0].max()) <= float(err[1].max()) + 2.0 ** -23
