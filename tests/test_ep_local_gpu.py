@@ -782,3 +782,40 @@ def test_owned_outputs_hold_no_more_memory_than_their_rows(masked, grouped):
         buf.check_status()
     finally:
         buf.destroy()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("R,pull", [(1, True), (1, False), (2, True), (2, False)])
+@pytest.mark.parametrize("K", [1, 2, 3, 5, 9, 17, 32])
+def test_combine_sums_in_order_whatever_the_number_of_contributors(K, R, pull, dtype):
+    """Bit by bit the f32 sum over the choices in ascending order, rounded once: every form of the reduction, with rows
+    read where they lie and from slots, some choices masked, a token without any, a row that ends inside a step."""
+    T, H, E = 37, 264, 32
+    g = torch.Generator().manual_seed(K)
+    idxs = [torch.rand(T, E, generator=g).topk(K, dim=-1).indices for _ in range(R)]
+    for i in idxs:
+        i[torch.rand(T, K, generator=g) < 0.25] = -1
+        i[3] = -1
+    ws = [torch.rand(T, K, generator=g) for _ in range(R)]
+    grp = _group(R, 64 << 20)
+    try:
+        outs = grp.dispatch([torch.randn(T, H, generator=g).to(dtype).cuda() for _ in range(R)], topk_idx=[i.cuda() for i in idxs],
+                            topk_weights=[w.cuda() for w in ws], group_by_expert=True, num_experts=E, zero_copy=pull)
+        handles = [o[4] for o in outs]
+        values = [torch.randn(o[0].shape, generator=g).to(dtype) for o in outs]
+        ys = [o[0].copy_(v) if pull else v.cuda() for o, v in zip(outs, values)]
+        comb = grp.combine(ys, handles, topk_weights=[h.recv_prob for h in handles])
+        got = [(c[0].cpu(), c[1].cpu()) for c in comb]
+        rows = [h.send_row[:T].cpu() for h in handles]
+        grp.check_status()
+        grp.check_canaries()
+    finally:
+        grp.destroy()
+    for r in range(R):
+        acc = torch.zeros(T, H)
+        for k in range(K):
+            for d in range(R):
+                t = (idxs[r][:, k] >= 0) & (idxs[r][:, k] // (E // R) == d)
+                acc[t] += values[d][rows[r][t, k].long()].float()
+        assert torch.equal(got[r][0], acc.to(dtype))
+        assert torch.equal(got[r][1], torch.where(idxs[r] >= 0, ws[r], torch.zeros(())))

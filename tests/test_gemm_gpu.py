@@ -534,3 +534,28 @@ def test_epilogue_sigmoid_is_as_near_as_a_rounded_division():
     normal = (silu.abs() > 2.0 ** -126) & (x > -88.7)
     err = [((d.double() - silu).abs() / silu.abs())[normal] for d in (dp, dp1)]
     assert float(err[0].mean()) <= float(err[1].mean()) * (1 + 2.0 ** -6) and float(err[0].max()) <= float(err[1].max()) + 2.0 ** -23
+
+
+@pytest.mark.parametrize("activation", ["swiglu", "gelu", "silu", "relu"])
+@pytest.mark.parametrize("counts", [[1], [40, 0, 257]])
+def test_experts_without_gradients_give_what_those_with_them_give(activation, counts):
+    """The pre-activation that a backward needs is written or not: the outputs are the same bits."""
+    from gpu_data_transfer_profile_b200.models.experts_tcgen05 import Tcgen05GroupedExperts
+    torch.manual_seed(2)
+    H, F, rows = 256, 384, sum(counts)
+    m = Tcgen05GroupedExperts(len(counts), H, F, activation=activation)
+    x, p = torch.randn(rows, H, device="cuda").to(torch.bfloat16), torch.rand(rows, device="cuda")
+    want = m(x, counts, p)
+    assert want.requires_grad
+    for forward in (torch.no_grad, torch.inference_mode):
+        with forward():
+            assert torch.equal(m(x, counts, p), want)
+    for t in m.parameters():
+        t.requires_grad_(False)
+    got = m(x, counts, p)                                          # nothing that asks for a gradient
+    assert torch.equal(got, want) and not got.requires_grad
+    probs = p.clone().requires_grad_(True)                         # the probabilities alone ask for one
+    y = m(x, counts, probs)
+    assert torch.equal(y, want)
+    (g,) = torch.autograd.grad(y.float().sum(), probs)
+    assert bool(g.isfinite().all()) and bool(g.any())
