@@ -559,3 +559,47 @@ def test_experts_without_gradients_give_what_those_with_them_give(activation, co
     assert torch.equal(y, want)
     (g,) = torch.autograd.grad(y.float().sum(), probs)
     assert bool(g.isfinite().all()) and bool(g.any())
+
+
+def test_grouped_gemms_refuse_outputs_and_values_that_their_kernels_cannot_address():
+    """Rows that 8-byte stores (16 in fp8 and the weight gradients) would meet unaligned, probabilities on the host or
+    with strides, offsets with strides: an error before a launch. What is aligned is taken, with gaps between the rows."""
+    from gpu_data_transfer_profile_b200.ops import gemm as G
+    E, rows, H, F = 2, 37, 128, 256
+    off = G.offsets_from_counts([17, 20], "cuda")
+    a = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, F, H, device="cuda") * 0.1).to(torch.bfloat16)
+    p = torch.rand(rows, device="cuda")
+    new = lambda cols, gap, first: torch.zeros(rows, cols + gap, device="cuda", dtype=torch.bfloat16)[:, first:first + cols]
+    q, qs = torch.randn(rows, H, device="cuda").to(torch.float8_e4m3fn), torch.ones(rows, 1, device="cuda")
+    wq, ws = torch.randn(E, F, H, device="cuda").to(torch.float8_e4m3fn), torch.ones(E, F // 128, 1, device="cuda")
+    calls = {
+        "plain": lambda o, p=None, off=off: G.grouped_gemm(a, w, off, out=o),
+        "swiglu pre": lambda o, p=p, off=off: G.grouped_gemm_swiglu(a, w, off, p, pre_out=o),
+        "act pre": lambda o, p=p, off=off: G.grouped_gemm_act(a, w, off, p, "gelu", pre_out=o),
+        "fp8": lambda o, p=None, off=off: G.grouped_gemm_fp8(q, qs, wq, ws, off, out=o),
+    }
+    for name, call in calls.items():
+        vec = 8 if name == "fp8" else 4                              # elements of a store
+        want = new(F, 0, 0)
+        call(want)
+        for gap, first in ((vec, 0), (vec, vec), (2 * vec, vec)):
+            got = new(F, gap, first)
+            call(got)
+            assert torch.equal(got, want) and bool(got.any())
+        for gap, first in ((1, 0), (vec, 1), (vec, vec // 2), (2, 0)):
+            with pytest.raises(RuntimeError, match="aligned rows"):
+                call(new(F, gap, first))
+        with pytest.raises(RuntimeError, match="aligned rows"):
+            call(torch.zeros(rows, F, dtype=torch.bfloat16))
+        with pytest.raises(RuntimeError, match="expert_off"):
+            call(want, off=torch.stack([off, off], 1)[:, 0])
+        if "pre" in name:
+            for bad in (p.cpu(), p[:1].expand(rows), torch.stack([p, p], 1)[:, 0], p[:-1]):
+                with pytest.raises(RuntimeError, match="row_prob"):
+                    call(want, p=bad)
+    flat = torch.zeros(E * H * F + 8, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(rows, F, device="cuda").to(torch.bfloat16)
+    assert torch.equal(G.grouped_wgrad(a, x, off, out=flat[8:].view(E, H, F)), G.grouped_wgrad(a, x, off))
+    with pytest.raises(RuntimeError, match="aligned"):
+        G.grouped_wgrad(a, x, off, out=flat[4:-4].view(E, H, F))
