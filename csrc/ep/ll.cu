@@ -22,7 +22,7 @@
 // another rank (a token's row, its routing, the slots of a combine) is therefore requested before
 // the first wait, a group of one neither signals nor waits, and rows of the rank's own tokens are
 // combined where they lie. Measured on one B200, inputs rotated from pass to pass: a CUDA-graph replay
-// (128 tokens x 7168, top-8 of 32, fp8, pull combine) 22.5 -> 13.1 us, then 10.3 us with the rows counted by a CTA of
+// (128 tokens x 7168, top-8 of 32, fp8, pull combine) 22.5 -> 13.1 us, then 10.9 us with the rows counted by a CTA of
 // its own, epochs committed as soon as they are read and overlapping launches in a group of one (send kernel
 // 6.3 -> 4.2 us on a device timeline); an eager bf16 round trip of 7 tokens with the experts' output elsewhere 42 -> 28 us, host
 // time for the most part.
@@ -38,7 +38,8 @@ constexpr int kLLHistExperts = 1024;   // experts that the counting CTA of a gro
 
 // Per-op device state (6 ints): [0] committed epoch, [1] committed arrival target,
 // [2] epoch published by the send half, [3] target published by the send half,
-// [4] CTAs of the running send launch that have finished (0 between launches), [5] unused.
+// [4] CTAs of the running launch that have finished or, where they count themselves early, have read the pair (0 between
+// launches), [5] unused.
 // Send half: works with epoch = [0]+1, target = [1]+grid; CTA 0 publishes them in [2],[3].
 // Receive half: the CTA of the send launch that finishes last (every CTA has read [0],[1] by then)
 // commits the pair to [0],[1]; as a launch of its own it reads [2],[3] and CTA 0 commits them. Where nothing but
@@ -459,7 +460,7 @@ ll_combine_pull_kernel(LLParams P, const __grid_constant__ PeerPtrs peers, int p
   int it = blockIdx.x * nwarps + warp;
   fetch(it);
   // state: [0] committed epoch, [1] committed arrival target, [2],[3] the pair published by an
-  // announce-only launch, [4] CTAs of this launch that have finished
+  // announce-only launch, [4] CTAs of this launch that have read them
   if (threadIdx.x == 0) {
     if (phase == 2) {
       s_epoch = *reinterpret_cast<volatile int*>(state + 2);

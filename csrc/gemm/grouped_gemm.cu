@@ -318,7 +318,7 @@ grouped_gemm_kernel(const __grid_constant__ TokenMaps map_t, const __grid_consta
       }
     }
   } else {
-    // ---------------- epilogue: two groups of 4 warps, one TMEM lane quarter per warp ----------------
+    // ---------------- epilogue: two or three groups of 4 warps, one TMEM lane quarter per warp ----------------
     const int q = warp & 3;                        // TMEM lanes [32q, 32q+32)
     const int grp = (warp - 2) >> 2;
     const int bar_id = 1 + grp;                    // the group's barrier (128 threads)

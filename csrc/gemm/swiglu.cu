@@ -1,5 +1,5 @@
-// SwiGLU x routing-probability, forward and backward, for the training path of the expert MLP
-// (the inference path fuses the forward into the fc1 GEMM epilogue instead).
+// SwiGLU x routing-probability, forward and backward, as operations of their own (the expert MLP has both in epilogues
+// of its GEMMs, which these are compared with), and the ungated activations, whose backward the expert MLP takes from here.
 //   h = [gate | linear]  (bf16 [rows, 2F]),  act = silu(gate) * linear * p[row]
 // Backward, given dact:  dp[row] = sum_f dact * silu(gate) * linear
 //                         dlinear = dact * p * silu(gate)

@@ -148,7 +148,7 @@ class Tcgen05GroupedExperts(GroupedExpertsBase):
             return self.forward_fp8(hidden_states, tokens_per_expert, routed_probs, expert_off)
         counts, off = self._offsets(tokens_per_expert, hidden_states.device, expert_off)
         x, probs = hidden_states.contiguous(), routed_probs.float().contiguous()
-        # without a backward to come the pre-activation (twice the size of the activation) is not written
+        # without a backward to come the pre-activation (with swiglu twice the size of the activation) is not written
         keep = torch.is_grad_enabled() and any(t.requires_grad for t in (x, self.weight1, self.weight2, probs))
         return _GroupedMLP.apply(x, self.weight1, self.weight2, probs, off, counts, self.activation, keep)
 

@@ -125,7 +125,8 @@ def swiglu_fwd(h: torch.Tensor, row_prob: Optional[torch.Tensor]) -> torch.Tenso
 
 
 def swiglu_bwd(h: torch.Tensor, row_prob: Optional[torch.Tensor], dact: torch.Tensor):
-    """-> (dh bf16 [rows, 2F], dprob f32 [rows]) for act = swiglu(h) * prob."""
+    """-> (dh bf16 [rows, 2F], dprob f32 [rows]) for act = swiglu(h) * prob. For callers that have dact in memory; the
+    expert MLP's own backward is `grouped_gemm_dswiglu`, which this is compared with."""
     dh = torch.empty_like(h)
     dp = torch.empty(h.shape[0], dtype=torch.float32, device=h.device)
     _ext.load().swiglu_bwd(h, row_prob, dact.contiguous(), dh, dp)
