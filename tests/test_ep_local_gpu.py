@@ -819,3 +819,30 @@ def test_combine_sums_in_order_whatever_the_number_of_contributors(K, R, pull, d
                 acc[t] += values[d][rows[r][t, k].long()].float()
         assert torch.equal(got[r][0], acc.to(dtype))
         assert torch.equal(got[r][1], torch.where(idxs[r] >= 0, ws[r], torch.zeros(())))
+
+
+@pytest.mark.parametrize("zero_copy", [False, True])
+@pytest.mark.parametrize("R", [2, 4])
+def test_fc2_epilogue_combine_where_a_rank_receives_nothing(R, zero_copy):
+    """All tokens go to experts of rank 0: the others' GEMMs have no rows and still tell their peers that they are done."""
+    T, H, E, K = 70, 256, 8, 1
+    El = E // R
+    xs, idxs, ws = _mk(R, T, H, E, K, seed=4)
+    idxs = [i % El for i in idxs]
+    torch.manual_seed(1)
+    g = _group(R, 64 << 20)
+    try:
+        w2s = [(torch.randn(El, H, H) * 0.05).to(torch.bfloat16) for _ in range(R)]
+        for _ in range(3):                                    # both parities of the combine region, and one again
+            outs = g.dispatch([x.cuda() for x in xs], topk_idx=[i.cuda() for i in idxs], topk_weights=[w.cuda() for w in ws],
+                              group_by_expert=True, num_experts=E, zero_copy=zero_copy)
+            assert [o[0].shape[0] for o in outs] == [R * T] + [0] * (R - 1)
+            comb = g.fused_fc2_combine([o[0] for o in outs], [w.cuda() for w in w2s], [o[4] for o in outs])
+            got = [c.cpu().float() for c in comb]
+            g.check_status()
+            for r in range(R):
+                want = torch.einsum("th,tfh->tf", xs[r].float(), w2s[0][idxs[r][:, 0]].float())
+                torch.testing.assert_close(got[r], want, atol=2e-3, rtol=2.0 ** -7)
+        g.check_canaries()
+    finally:
+        g.destroy()
